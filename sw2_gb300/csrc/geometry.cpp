@@ -3,7 +3,9 @@
 // -ffp-contract=off, so the tables are bit-identical to the values the
 // reference computes per cell.
 #include <cmath>
+#include <cstring>
 
+#include "sigmath.cuh"
 #include "sw2g_internal.h"
 
 namespace sw2g {
@@ -41,7 +43,30 @@ double fcor(const Planet& p, double lat) { return 2.0 * p.Omega * std::sin(lat);
 // init.c:56-58 does), or already converted (SW2G_FLAG_RADIANS).
 double angle(const sw2g_case& c, double a) { return (c.flags & SW2G_FLAG_RADIANS) ? a : deg2rad(a); }
 
+// The divisors of the integer-pipe quotients and where their reciprocals go.
+struct SigDivisor {
+  int row, recip;
+};
+constexpr SigDivisor kSigDivisors[] = {{R_DXE, R_YDXE}, {R_DXC, R_YDXC},   {R_DXV, R_YDXV},   {R_DYN, R_YDYN},
+                                       {R_DYC, R_YDYC}, {R_DYV, R_YDYV},   {R_DXE2, R_YDXE2}, {R_DYNS, R_YDYNS},
+                                       {R_RZC, R_YRZC}, {R_RZN, R_YRZN}};
+uint64_t bits_of(double x) {
+  uint64_t b;
+  std::memcpy(&b, &x, sizeof b);
+  return b;
+}
+bool positive_in_window(uint64_t b) { return !(b >> 63) && in_window((uint32_t)(b >> 32)); }
+
 }  // namespace
+
+bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows) {
+  const int H = c.ny + 4;
+  if (!positive_in_window(bits_of(c.Dt))) return false;
+  for (const auto& d : kSigDivisors)
+    for (int j = 0; j <= c.ny + 1; j++)  // the rows a step divides by
+      if (!positive_in_window(bits_of(rows[(size_t)d.row * H + (j + 1)]))) return false;
+  return true;
+}
 
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my) {
   const int ny = c.ny, H = c.ny + 4;
@@ -106,6 +131,11 @@ void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, 
     R(R_IRZC, j) = 1.0 / R(R_RZC, j);
     R(R_IRZN, j) = 1.0 / R(R_RZN, j);
   }
+  for (int j = -1; j <= ny + 2; j++)
+    for (const auto& d : kSigDivisors) {
+      const uint64_t b = bits_of(R(d.row, j)), y = positive_in_window(b) ? sig_recip(b) : 0;
+      std::memcpy(&R(d.recip, j), &y, sizeof y);
+    }
   // compute_Dt fallback for a flow at rest (calc.c:715-725): depends on geometry only
   double mx = 0, my = 0;
   for (int j = 1; j <= ny; j++) {

@@ -13,6 +13,7 @@
 // IEEE sums).
 #include <cuda_runtime.h>
 
+#include "sigmath.cuh"
 #include "sw2g_internal.h"
 
 namespace sw2g {
@@ -284,11 +285,10 @@ __global__ void k_mass(DevState s, F7 f, double* out) {
   out[IX(W, i, j)] = mass_cell<SCH>(s, f, i, j);
 }
 
-// BODYTRACER (calc.c:117-163)
+// BODYTRACER (calc.c:117-163), one cell
 template <int SCH>
-__global__ void k_tracer(DevState s, F7 f, double* out) {
-  SW2G_PDL_ENTRY();
-  INTERIOR_IJ
+__device__ __forceinline__ double tracer_cell(const DevState& s, const F7& f, int i, int j) {
+  const int W = s.W;
   const double Dt = s.Dt, dxe = RW(s, R_DXE, j), dyn = RW(s, R_DYN, j);
   double qx[5], qy[5];
 #pragma unroll
@@ -302,7 +302,14 @@ __global__ void k_tracer(DevState s, F7 f, double* out) {
   double acc = pv1 + pv2;
   const double sigma = s.polar ? PF(s, P_STR, IX(W, i, j)) : s.sigma_tr;  // calc.c:152-161
   acc -= 2.0 * Dt * (sigma) * t;
-  out[IX(W, i, j)] = acc;
+  return acc;
+}
+
+template <int SCH>
+__global__ void k_tracer(DevState s, F7 f, double* out) {
+  SW2G_PDL_ENTRY();
+  INTERIOR_IJ
+  out[IX(W, i, j)] = tracer_cell<SCH>(s, f, i, j);
 }
 
 // BODYU (calc.c:168-200), one cell
@@ -359,6 +366,10 @@ __device__ __noinline__ double mass_cell_ool(const DevState& s, const F7& f, int
   return mass_cell<SCH>(s, f, i, j);
 }
 template <int SCH>
+__device__ __noinline__ double tracer_cell_ool(const DevState& s, const F7& f, int i, int j) {
+  return tracer_cell<SCH>(s, f, i, j);
+}
+template <int SCH>
 __device__ __noinline__ double advu_cell_ool(const DevState& s, const F7& f, int i, int j) {
   return advu_cell<SCH>(s, f, i, j);
 }
@@ -368,11 +379,11 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 }
 
 // ------------------------------------------------------------ fast TVD bodies
-// The same values as k_mass, k_adv_u and k_adv_v, bit for bit, with about a
-// third of their FP64 operations. Three properties of the reference formulas
-// (calc.c:41-49, 70-237) make that possible:
-//  (1) x faces. With polar 0 the metric factors DXE, DXC, DXV depend on j
-//      only, so the Courant numbers, limiter ratios and limited values of the
+// The same values as k_mass, k_tracer, k_adv_u and k_adv_v, bit for bit, with
+// about a tenth of their FP64 instructions. Four properties of the reference
+// formulas (calc.c:41-49, 70-237) and of the unit make that possible:
+//  (1) x faces. The metric factors DXE, DXC, DXV depend on j only, so the
+//      Courant numbers, limiter ratios and limited values of the
 //      face between columns i-1 and i are the same operations on the same
 //      operands for cell i (its west face) and cell i-1 (its east face). Each
 //      lane of a warp computes the face west of its column; a warp covers 31
@@ -380,23 +391,40 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 //  (2) y faces. The ratios and limiter values of the face between rows j and
 //      j+1 are shared by both cells; only the Courant numbers differ, since
 //      each cell divides by its own DYN, DYV or DYC. A warp marches up its
-//      rows and carries the face's shared part from one row to the next.
+//      rows and carries the face's shared part from one row to the next, and
+//      the differences q(j+1)-q(j), which serve three faces.
 //  (3) Upwind split. C+ = 0.5(U+|U|)*Dt/DX is +0 when U <= 0, and C- is a
 //      zero when U >= 0 (for the two-velocity averages, when both are), so
 //      the term C*B of an unused side is a zero whenever B is finite, and
 //      0.5(U+|U|) = U exactly when U > 0 (0.5(U-|U|) = U when U < 0). Leaving
 //      zero terms out of a sum of otherwise identical terms, in the same
-//      order, can change only the sign of a zero result. So the unused side
-//      is skipped, and a cell is recomputed literally when its sum is zero,
-//      when an input is not finite, or when the skipped side's limiter ratio
-//      could exceed 2^498 (the bound under which every limiter gives a finite
-//      value, squares included).
+//      order, can change only the sign of a zero result (see below). When
+//      both velocities of an average have one sign, the sum of their used
+//      halves is the sum of the velocities, which the second term of the
+//      body needs as well.
+//  (4) The integer pipe. The quotients (limiter ratios, Courant numbers, the
+//      second term's divisions) and the products that enter them are taken
+//      from the operands' bits (sigmath.cuh: IEEE results); the FP64 unit
+//      keeps the additions and the products around them.
+// Ranges: each value that a warp reads is zero or of magnitude 2^-300 ..
+// 2^100 (in_range); otherwise the warp's cells are recomputed literally for
+// the rest of its strip. Differences and sums of such values are zero or at
+// least 2^-352 (they are multiples of the smallest unit among them), so no
+// quotient or product leaves the normal range, and no slope ratio, of the
+// side in use or not, exceeds 2^453, for which every limiter (squares
+// included) is finite.
+// Zero sums. A sum that is zero because nonzero terms cancel is +0, as the
+// reference's is (x - x = +0, and +0 plus or minus a zero is +0). When every
+// term is zero the reference's sum is +0 if its first term is +0, which holds
+// when the + side's velocity at the west face is not positive and that
+// side's face value is not negative (west_plus_zero): a flow at rest.
+// Otherwise the cell is recomputed literally.
 // The Van Leer limiter in its reference form (0/0 at r = -1) keeps the
-// literal kernels.
+// literal kernels, and so do cases whose Dt or metric factors lie outside
+// [2^-127, 2^129) (DevState::sig_ok).
 constexpr int FW = 31;      // cells per strip along x (32 faces)
 constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the launch's queue
-// Resident blocks per SM the register allocation must allow: 5 blocks (20
-// warps) at 96 registers hide the FP64 unit's latency better than 4 at ~120.
+// Resident blocks per SM the register allocation must allow.
 #define FAST_MIN_BLOCKS 5
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -429,83 +457,175 @@ __device__ __forceinline__ double limiter_fast(double r) {
   else return limiter<SCH>(r);
 }
 
-
-// n/d for d nonzero, with a zero n answered on the integer pipe: the IEEE
-// quotient of +-0 by d is the zero whose sign is sign(n) xor sign(d).
-__device__ __forceinline__ double div_nz(double n, double d) {
-  const long long nb = dbits(n);
-  if ((nb & 0x7fffffffffffffffLL) == 0)
-    return __longlong_as_double((nb ^ dbits(d)) & (long long)0x8000000000000000ULL);
-  return n / d;
+// Operands of the integer-pipe quotients and products.
+__device__ __forceinline__ unsigned long long mag(double x) {
+  return (unsigned long long)dbits(x) & 0x7fffffffffffffffULL;
+}
+__device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)((unsigned long long)dbits(x) >> 32); }
+__device__ __forceinline__ bool usable(double x) { return in_window(hi_word(x)); }
+// zero, or 2^-300 <= |x| < 2^100
+__device__ __forceinline__ bool in_range(double x) {
+  return ((hi_word(x) & 0x7fffffffu) - (723u << 20)) < (400u << 20) || !nz(x);
+}
+__device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
+// p ? a : b, opaque: one operation on the selected value stays one FP64
+// instruction (the compiler would evaluate it for both and select after).
+__device__ __forceinline__ double pick(bool p, double a, double b) {
+  long long r;
+  asm("mov.b64 %0, %1;" : "=l"(r) : "l"(p ? __double_as_longlong(a) : __double_as_longlong(b)));
+  return __longlong_as_double(r);
+}
+// x with its sign bit changed by `neg` (0 or the sign bit), on the integer
+// pipe: the compiler's negation of a double is an FP64 addition.
+__device__ __forceinline__ double flip(double x, unsigned long long neg) {
+  return __longlong_as_double(dbits(x) ^ (long long)neg);
+}
+__device__ __forceinline__ unsigned long long sign_of(double x) {
+  return (unsigned long long)dbits(x) & 0x8000000000000000ULL;
 }
 
+// A row metric as a divisor: its bits and its reciprocal (sig_recip).
+struct Metric {
+  unsigned long long b, y;
+};
+__device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j) {
+  return Metric{(unsigned long long)dbits(RW(s, t, j)), (unsigned long long)dbits(RW(s, ty, j))};
+}
+#define METRIC(NAME, j) metric(s, R_##NAME, R_Y##NAME, j)
+
+// RN(RN(a*b)*2^k / x) of zero or in-range a and b (k20 = k << 20).
+__device__ __forceinline__ double product_over(double a, double b, unsigned k20, const Metric& x) {
+  const unsigned long long p = sig_mul(mag(a), mag(b), k20);
+  const unsigned long long q = sig_div_known(p, x.b, x.y);
+  return (nz(a) && nz(b)) ? from_bits(q | (sign_of(a) ^ sign_of(b))) : 0.0;
+}
+
+// a/b on the integer pipe where both are usable (the quotient is then normal),
+// a zero numerator from the bits; otherwise on the FP64 unit, out of line.
+__device__ __noinline__ double quotient_fp64(double a, double b) { return zdiv(a, b); }
+__device__ __forceinline__ double quotient(double a, double b) {
+  if (usable(a) && usable(b)) return from_bits(sig_div(mag(a), mag(b)) | (sign_of(a) ^ sign_of(b)));
+  return quotient_fp64(a, b);
+}
+
+// Half the limited slope factor: 0.5*limiter(n/d), n/d read as 0 for d = 0
+// (calc.c:42-47), of zero or in-range differences. The limiters whose formula
+// divides take that quotient on the integer pipe too.
 template <int SCH>
 __device__ __forceinline__ double half_psi(double n, double d) {
-  const double r = nz(d) ? div_nz(n, d) : 0.0;  // r2rP / r2rM (calc.c:42-43)
-  return HALF(limiter_fast<SCH>(r));
+  const bool zero = !nz(d) || !nz(n);
+  const unsigned long long q = sig_div(mag(n), mag(d)) | (sign_of(n) ^ sign_of(d));
+  if constexpr (SCH == 2) {  // min(r, 1): a negative r has a negative image
+    const long long m = (long long)q < dbits(1.0) ? (long long)q : dbits(1.0);
+    return zero ? 0.0 : __longlong_as_double(m - (1LL << 52));
+  }
+  const double r = zero ? 0.0 : from_bits(q);
+  if constexpr (SCH == 4) {
+    const double r2 = TWICE(r);
+    return HALF(mx(0.0, mn(r2, mn(quotient(1 + r2, 3.0), 2.0))));
+  } else if constexpr (SCH == 5) {
+    return HALF(quotient(1.5 * (r * r + r), r * r + r + 1.0));
+  } else if constexpr (SCH == 6) {
+    return HALF(quotient(r * r + r, r * r + 1.0));
+  } else if constexpr (SCH == kVanLeerSafe) {
+    return (dbits(r) == dbits(-1.0)) ? 0.0 : HALF(quotient(r + fabs(r), 1.0 + r));
+  } else {
+    return HALF(limiter_fast<SCH>(r));
+  }
 }
 
-// c*B of one side: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or B2BM =
-// q1 - psi*0.5*(1+c)*(q1-q0); 1 + c = 1 - (-c) and q1 - X = q1 + (-X) exactly.
-// SB: the last sum on the integer pipe (measured faster in the mass body only).
-template <bool SB>
-__device__ __forceinline__ double side_term(bool pos, double c, double hpsi, double q0, double q1, double d) {
-  const double g = 1.0 - (pos ? c : -c);
-  const double X = (hpsi * g) * d;
-  if constexpr (SB) return c * sadd(pos ? q0 : q1, pos ? X : -X);
-  else return c * ((pos ? q0 : q1) + (pos ? X : -X));
-}
-
-// Shared part of a face q0|q1 (outer neighbours qm, q2), with the Courant
-// numerators pn = 0.5(...+|...|) >= 0 and mn <= 0 before "*Dt/dx".
-struct Face {
-  double d, q0, q1, pn, mn, hp1, hp2;
-  bool pos1, act, both, ok;
+// The velocity of a face: one (calc.c:72-79) or the sum of two to be averaged
+// (calc.c:170-177), w; the side in use is + (pos) or -, none when !act; `both`
+// if the two have opposite signs, each then using one side.
+struct Vel {
+  double w, a, b;
+  bool pos, act, both;
 };
-
-template <int SCH>
-__device__ __forceinline__ Face make_face(double qm, double q0, double q1, double q2, double pn, double mn,
-                                          bool cfin) {
+__device__ __forceinline__ Vel vel_one(double a) { return Vel{a, 0.0, 0.0, dbits(a) >= 0 || !nz(a), nz(a), false}; }
+__device__ __forceinline__ Vel vel_pair(double a, double b, double sum) {
+  Vel v;
+  v.w = sum;
+  v.a = a;
+  v.b = b;
+  v.both = (dbits(a) ^ dbits(b)) < 0 && nz(a) && nz(b);
+  v.act = nz(sum) || v.both;
+  v.pos = v.both || dbits(sum) >= 0 || !nz(sum);
+  return v;
+}
+// Shared part of a face q0|q1. p: magnitude bits of the used side's numerator
+// 0.5(...+-|...|)*Dt; hp: half its limited slope factor; p2, hp2: those of
+// the - side when both are in use.
+struct Face {
+  double d, q0, q1, hp, hp2;
+  unsigned long long p, p2;
+  bool pos, act, both;
+};
+// PAIR: w is a sum of two velocities, to be halved. n1: q0 - qm when v.pos,
+// q2 - q1 otherwise; q2 is read when both sides are in use.
+template <int SCH, bool PAIR>
+__device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, double q0, double q1, double q2,
+                                          unsigned long long dt) {
+  constexpr unsigned K = PAIR ? 0xfff00000u : 0u;  // exponent of the halving
   Face F;
-  F.d = q1 - q0;
+  F.d = d;
   F.q0 = q0;
   F.q1 = q1;
-  F.pn = pn;
-  F.mn = mn;
-  const bool aP = nz(pn), aM = nz(mn);
-  F.pos1 = aP;  // the side computed first: + if in use, else -
-  F.act = aP || aM;
-  F.both = aP && aM;
-  F.hp1 = half_psi<SCH>(aP ? (q0 - qm) : (q2 - q1), F.d);
+  F.pos = v.pos;
+  F.act = v.act;
+  F.both = v.both;
+  F.hp = half_psi<SCH>(n1, d);
+  F.p = sig_mul(mag(v.w), dt, K);
   F.hp2 = 0.0;
-  if (__any_sync(FULL, F.both)) {
-    if (F.both) F.hp2 = half_psi<SCH>(q2 - q1, F.d);
+  F.p2 = 0;
+  if constexpr (PAIR) {
+    if (__any_sync(FULL, v.both)) {
+      if (v.both) {
+        const bool apos = dbits(v.a) > 0;
+        F.p = sig_mul(mag(apos ? v.a : v.b), dt, K);
+        F.p2 = sig_mul(mag(apos ? v.b : v.a), dt, K);
+        F.hp2 = half_psi<SCH>(q2 - q1, d);
+      }
+    }
   }
-  const int E = max(max(dexp(qm), dexp(q0)), max(dexp(q1), dexp(q2)));
-  F.ok = cfin && (E < 0x7ff) && (!nz(F.d) || dexp(F.d) + 498 > E);
   return F;
 }
 
-// The face's two terms for a cell whose metric divisor is dx (idx = 1.0/dx).
-template <bool SB>
-__device__ __forceinline__ void face_terms(const Face& F, double Dt, double dx, double idx, double& tP,
-                                           double& tM) {
-  const double c1 = div_rcp((F.pos1 ? F.pn : F.mn) * Dt, dx, idx);
-  const double t1 = F.act ? side_term<SB>(F.pos1, c1, F.hp1, F.q0, F.q1, F.d) : 0.0;
-  tP = F.pos1 ? t1 : 0.0;
-  tM = F.pos1 ? 0.0 : t1;
-  if (__any_sync(FULL, F.both)) {
-    if (F.both) tM = side_term<SB>(false, div_rcp(F.mn * Dt, dx, idx), F.hp2, F.q0, F.q1, F.d);
-  }
+// C*B of one side with c = |C|: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or
+// B2BM = q1 - psi*0.5*(1-c)*(q1-q0) (C- = -c; q1 - X = q1 + (-X) exactly).
+__device__ __forceinline__ double side_term(bool pos, unsigned long long p, const Metric& dx, double hp, double q0,
+                                            double q1, double d) {
+  const double c = from_bits(sig_div_known(p, dx.b, dx.y));
+  const double X = (hp * (1.0 - c)) * d;
+  const unsigned long long neg = pos ? 0 : 0x8000000000000000ULL;
+  return flip(c * (pick(pos, q0, q1) + flip(X, neg)), neg);
 }
-#define ROW2(t, it, j) RW(s, t, j), RW(s, it, j)
 
-// calc.c:100 over the four faces: +wP +wM -eP -eM +sP +sM -nP -nM. The term
-// of an unused side is a +0 placeholder; leaving it out changes only the sign
-// of a zero sum, which the literal path recomputes. Unless a face of the
-// warp's cells uses both sides, each face has one term (the side in use) and
-// the sum takes three additions; otherwise all eight terms are summed, out of
-// line so that the common case does not carry the extra FP64 operations.
+// A face's terms as seen by one cell: that of the side in use (0 when none
+// is), and the - side's when both are.
+struct Side {
+  double t, m;
+  bool pos, both;
+};
+template <bool PAIR>
+__device__ __forceinline__ Side side_of(const Face& F, const Metric& dx) {
+  Side r;
+  const double t = side_term(F.pos, F.p, dx, F.hp, F.q0, F.q1, F.d);
+  r.t = F.act ? t : 0.0;
+  r.m = 0.0;
+  r.pos = F.pos;
+  r.both = F.both;
+  if constexpr (PAIR) {
+    if (__any_sync(FULL, F.both)) {
+      if (F.both) r.m = side_term(false, F.p2, dx, F.hp2, F.q0, F.q1, F.d);
+    }
+  }
+  return r;
+}
+
+// calc.c:100 over the four faces: +wP +wM -eP -eM +sP +sM -nP -nM. Unless a
+// face of the warp's cells uses both sides, each face has one term and the sum
+// takes three additions; otherwise all eight are summed, out of line so that
+// the common case does not carry the extra FP64 operations.
 __device__ __noinline__ double sum_faces8(double wP, double wM, double eP, double eM, double sP, double sM,
                                           double nP, double nM) {
   double S = wP + wM;
@@ -517,38 +637,40 @@ __device__ __noinline__ double sum_faces8(double wP, double wM, double eP, doubl
   S = S - nM;
   return S;
 }
-struct Side {  // a face's terms as seen by one cell, and which side is in use
-  double P, M;
-  bool pos, both;
-};
-__device__ __forceinline__ double sum_faces(const Side& w, const Side& e, const Side& so, const Side& n) {
-  if (__any_sync(FULL, w.both || e.both || so.both || n.both))
-    return sum_faces8(w.P, w.M, e.P, e.M, so.P, so.M, n.P, n.M);
-  const double tw = w.pos ? w.P : w.M, te = e.pos ? e.P : e.M;
-  const double ts = so.pos ? so.P : so.M, tn = n.pos ? n.P : n.M;
-  return ssub(sadd(ssub(tw, te), ts), tn);
-}
-__device__ __forceinline__ Side east_of(const Side& w, int lane) {
-  Side e;
-  e.P = __shfl_sync(FULL, w.P, (lane + 1) & 31);
-  e.M = __shfl_sync(FULL, w.M, (lane + 1) & 31);
-  e.pos = __shfl_sync(FULL, (int)w.pos, (lane + 1) & 31) != 0;
-  e.both = __shfl_sync(FULL, (int)w.both, (lane + 1) & 31) != 0;
-  return e;
-}
-template <bool SB = false>
-__device__ __forceinline__ Side side_of(const Face& F, double Dt, double dx, double idx) {
-  Side t;
-  face_terms<SB>(F, Dt, dx, idx, t.P, t.M);
-  t.pos = F.pos1;
-  t.both = F.both;
-  return t;
+// Whether the reference's first term at a west face qm | q0 | q1 whose + side
+// has no positive velocity is +0: its face value q0 + X must not be negative.
+// With the Courant number 0, X is a zero where q1 = q0, and otherwise
+// |X| <= |q1-q0| + |q0-qm| for every limiter (|psi(r)| <= 2 + |r|).
+__device__ __forceinline__ bool west_plus_zero(bool act, double qm, double q0, double q1) {
+  if (act || dbits(q0) < 0) return false;
+  const double d = q1 - q0, n = q0 - qm;
+  if (!nz(d)) return true;
+  return max(hi_word(d) & 0x7fffffffu, hi_word(n) & 0x7fffffffu) + (3u << 20) <= hi_word(q0);
 }
 
-// Upwind halves of one velocity: 0.5(a+|a|) and 0.5(a-|a|) up to the sign of a zero.
-__device__ __forceinline__ double up_p(double a) { return gt0(a) ? a : 0.0; }
-__device__ __forceinline__ double up_m(double a) { return lt0(a) ? a : 0.0; }
-__device__ __forceinline__ bool fin(double a) { return dexp(a) != 0x7ff; }
+// The sum for the lane's cell: w its west face (whose east neighbour's is taken
+// from the next lane), so and n its south and north faces; slow: a zero sum
+// whose sign only the literal expression tells. act, qm, q0, q1: the west
+// face's, for that question.
+template <bool PAIR>
+__device__ __forceinline__ double sum_faces(const Side& w, const Side& so, const Side& n, int lane, bool act,
+                                            double qm, double q0, double q1, bool& slow) {
+  const double te = __shfl_sync(FULL, w.t, (lane + 1) & 31);
+  if constexpr (PAIR) {
+    if (__any_sync(FULL, w.both || so.both || n.both)) {
+      const double me = __shfl_sync(FULL, w.m, (lane + 1) & 31);
+      const bool epos = __shfl_sync(FULL, (int)w.pos, (lane + 1) & 31) != 0;
+      const double S = sum_faces8(w.pos ? w.t : 0.0, w.pos ? w.m : w.t, epos ? te : 0.0, epos ? me : te,
+                                  so.pos ? so.t : 0.0, so.pos ? so.m : so.t, n.pos ? n.t : 0.0, n.pos ? n.m : n.t);
+      slow = !nz(S);
+      return S;
+    }
+  }
+  const double S = ((w.t - te) + so.t) - n.t;
+  slow = false;
+  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !west_plus_zero(act, qm, q0, q1);
+  return S;
+}
 
 // Values of the lane's x neighbours at one row: own value v of column i,
 // aux = the value of column base-2 (lane 0), base-1 (lane 1) or base+32 (lane 31).
@@ -565,6 +687,12 @@ __device__ __forceinline__ XN x_neighbours(double v, double aux, int lane) {
   if (lane == 0) n.m1 = a1;
   if (lane == 31) n.p1 = aux;
   return n;
+}
+// The face west of the lane's column from its x neighbours: q0 = m1, q1 = v.
+template <int SCH, bool PAIR>
+__device__ __forceinline__ Face x_face(const Vel& vel, const XN& n, double v, unsigned long long dt) {
+  const double n1 = pick(vel.pos, n.m1, n.p1) - pick(vel.pos, n.m2, v);
+  return make_face<SCH, PAIR>(vel, v - n.m1, n1, n.m1, v, n.p1, dt);
 }
 
 // A strip is 31 columns x s.fk rows (chosen per launch, see fast_launch).
@@ -590,6 +718,7 @@ __device__ __forceinline__ void strips_done(unsigned* q, int lane) {
   const int FK = s.fk;                                                                      \
   const int nsx = (nx + FW - 1) / FW, nstrips = nsx * ((ny + FK - 1) / FK);                  \
   const double Dt = s.Dt;                                                                   \
+  const unsigned long long dt = (unsigned long long)dbits(Dt);                              \
   for (int strip = next_strip(s.strips, lane); strip < nstrips; strip = next_strip(s.strips, lane)) { \
     const int j0 = (strip / nsx) * FK + 1;                                                  \
     const int jn = min(j0 + FK - 1, ny);                                                    \
@@ -615,34 +744,43 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
   FAST_SETUP
   const int iu = min(i - 1, nx + 2);
   const double damp = 2.0 * Dt * (s.sigma);  // calc.c:112: (2.0*Dt*sigma)*ETA
-  // H at this lane's column, rows j-1 .. j+1 (window), and the face south of j0
-  double h1 = HF(ic, j0 - 1), h2 = HF(ic, j0), h3 = HF(ic, j0 + 1);
+  // H at this lane's column, rows j and j+1, the differences of rows j-1 .. j+1,
+  // and the face south of j0
+  double h2 = HF(ic, j0), h3 = HF(ic, j0 + 1), dm, d0;
+  bool bad = !in_range(h2) || !in_range(h3);  // any value of the strip so far out of range
   // UD (no damping: sigma = 0, a band): the product damp*eta is a zero (eta is
   // finite on the fast path), and a nonzero S minus a zero is S
   Side ts;
-  bool oks;
   {
-    const double b = VF(ic, j0 - 1);
-    const Face F = make_face<SCH>(HF(ic, j0 - 2), h1, h2, h3, up_p(b), up_m(b), fin(b));
-    ts = side_of<true>(F, Dt, ROW2(R_DYN, R_IDYN, j0));
-    oks = F.ok;
+    const double h0 = HF(ic, j0 - 2), h1 = HF(ic, j0 - 1);
+    bad = bad || !in_range(h0) || !in_range(h1);
+    const double vs = VF(ic, j0 - 1);
+    bad = bad || !in_range(vs);
+    const Vel b = vel_one(vs);
+    dm = h2 - h1;
+    d0 = h3 - h2;
+    const Face F = make_face<SCH, false>(b, dm, b.pos ? h1 - h0 : d0, h1, h2, h3, dt);
+    ts = side_of<false>(F, METRIC(DYN, j0));
   }
   for (int j = j0; j <= jn; j++) {
-    const double h4 = HF(ic, j + 2);
+    const double h4 = HF(ic, j + 2), ha = HF(ia, j);
+    const double d1 = h4 - h3;
+    bad = bad || !in_range(h4) || !in_range(ha);
     // x face west of column i, row j
-    const XN xn = x_neighbours(h2, HF(ia, j), lane);
     const double a = UF(iu, j);
-    const Face FX = make_face<SCH>(xn.m2, xn.m1, h2, xn.p1, up_p(a), up_m(a), fin(a));
-    const Side tw = side_of<true>(FX, Dt, ROW2(R_DXE, R_IDXE, j));
-    const Side te = east_of(tw, lane);
-    const bool oke = __shfl_sync(FULL, (int)FX.ok, (lane + 1) & 31) != 0;
+    const XN xn = x_neighbours(h2, ha, lane);
+    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt);
+    const Side tw = side_of<false>(FX, METRIC(DXE, j));
     // y face north of row j: shared by this cell and the cell above
-    const double b = VF(ic, j);
-    const Face FY = make_face<SCH>(h1, h2, h3, h4, up_p(b), up_m(b), fin(b));
-    const Side tn = side_of<true>(FY, Dt, ROW2(R_DYN, R_IDYN, j));
-    const Side ns = side_of<true>(FY, Dt, ROW2(R_DYN, R_IDYN, j + 1));
-    const double S = sum_faces(tw, te, ts, tn);  // calc.c:100 in its order: +w -e +s -n
-    const bool slow = !(FX.ok && oke && oks && FY.ok) || !nz(S);
+    const double vn = VF(ic, j);
+    bad = bad || !in_range(a) || !in_range(vn);
+    const Vel b = vel_one(vn);
+    const Face FY = make_face<SCH, false>(b, d0, b.pos ? dm : d1, h2, h3, h4, dt);
+    const Side tn = side_of<false>(FY, METRIC(DYN, j));
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
+    bool slow;
+    const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);  // calc.c:100 in its order: +w -e +s -n
+    slow = __any_sync(FULL, bad) || slow;
     if (own) {
       double r;
       if (slow) r = mass_cell_ool<SCH>(s, f, i, j);
@@ -651,10 +789,67 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
       out[IX(W, i, j)] = r;
     }
     ts = ns;
-    oks = FY.ok;
-    h1 = h2;
     h2 = h3;
     h3 = h4;
+    dm = d0;
+    d0 = d1;
+  }
+  FAST_END
+}
+
+// BODYTRACER, fast form (calc.c:117-163).
+template <int SCH, bool PL>
+__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(DevState s, F7 f, double* out) {
+  SW2G_PDL_ENTRY();
+  FAST_SETUP
+  const int iu = min(i - 1, nx + 2);
+  const double damp = 2.0 * Dt * (s.sigma_tr);  // calc.c:161
+  double h2 = f.tr[IX(W, ic, j0)], h3 = f.tr[IX(W, ic, j0 + 1)], dm, d0;
+  bool bad = !in_range(h2) || !in_range(h3);
+  double vs = VF(ic, j0 - 1);
+  Side ts;
+  {
+    const double h0 = f.tr[IX(W, ic, j0 - 2)], h1 = f.tr[IX(W, ic, j0 - 1)];
+    bad = bad || !in_range(h0) || !in_range(h1) || !in_range(vs);
+    const Vel b = vel_one(vs);
+    dm = h2 - h1;
+    d0 = h3 - h2;
+    const Face F = make_face<SCH, false>(b, dm, b.pos ? h1 - h0 : d0, h1, h2, h3, dt);
+    ts = side_of<false>(F, METRIC(DYN, j0));
+  }
+  for (int j = j0; j <= jn; j++) {
+    const double h4 = f.tr[IX(W, ic, j + 2)], ha = f.tr[IX(W, ia, j)];
+    const double d1 = h4 - h3;
+    bad = bad || !in_range(h4) || !in_range(ha);
+    const double a = UF(iu, j);
+    const Metric mx = METRIC(DXE, j), my = METRIC(DYN, j);
+    const XN xn = x_neighbours(h2, ha, lane);
+    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt);
+    const Side tw = side_of<false>(FX, mx);
+    const double vn = VF(ic, j);
+    bad = bad || !in_range(a) || !in_range(vn);
+    const Vel b = vel_one(vn);
+    const Face FY = make_face<SCH, false>(b, d0, b.pos ? dm : d1, h2, h3, h4, dt);
+    const Side tn = side_of<false>(FY, my);
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
+    bool slow;
+    const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);
+    slow = __any_sync(FULL, bad) || slow;
+    // Dt*TRACER*(UW(E)-UW(W))/DXE + Dt*TRACER*(VW(N)-VW(S))/DYN (calc.c:146-149)
+    const double du = __shfl_sync(FULL, a, (lane + 1) & 31) - a, dv = vn - vs, tt = Dt * h2;
+    const double p2 = product_over(tt, du, 0, mx) + product_over(tt, dv, 0, my);
+    if (own) {
+      double r;
+      if (slow) r = tracer_cell_ool<SCH>(s, f, i, j);
+      else r = (S + p2) - (s.polar ? 2.0 * Dt * PF(s, P_STR, IX(W, i, j)) : damp) * h2;
+      out[IX(W, i, j)] = r;
+    }
+    ts = ns;
+    vs = vn;
+    h2 = h3;
+    h3 = h4;
+    dm = d0;
+    d0 = d1;
   }
   FAST_END
 }
@@ -665,54 +860,56 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
   SW2G_PDL_ENTRY();
   FAST_SETUP
   const int ic1 = min(i + 1, nx + 2);
-  // U at this lane's column, rows j-1 .. j+1, and V at columns i, i+1 of row j-1
-  double u1 = UF(ic, j0 - 1), u2 = UF(ic, j0), u3 = UF(ic, j0 + 1);
-  double vs0 = VF(ic, j0 - 1), vs1 = VF(ic1, j0 - 1);
+  // U at this lane's column, rows j and j+1, the differences of rows j-1 .. j+1,
+  // and the sum of V at columns i, i+1 of row j-1
+  double u2 = UF(ic, j0), u3 = UF(ic, j0 + 1), dm, d0, vs;
+  bool bad = !in_range(u2) || !in_range(u3);
   Side ts;
-  bool oks;
   {
-    const Face F = make_face<SCH>(UF(ic, j0 - 2), u1, u2, u3, HALF(up_p(vs0) + up_p(vs1)),
-                                  HALF(up_m(vs0) + up_m(vs1)), fin(vs0) && fin(vs1));
-    ts = side_of(F, Dt, ROW2(R_DYV, R_IDYV, j0));
-    oks = F.ok;
+    const double u0 = UF(ic, j0 - 2), u1 = UF(ic, j0 - 1), a = VF(ic, j0 - 1), b = VF(ic1, j0 - 1);
+    bad = bad || !in_range(u0) || !in_range(u1) || !in_range(a);
+    vs = a + b;
+    const Vel v = vel_pair(a, b, vs);
+    dm = u2 - u1;
+    d0 = u3 - u2;
+    const Face F = make_face<SCH, true>(v, dm, v.pos ? u1 - u0 : d0, u1, u2, u3, dt);
+    ts = side_of<true>(F, METRIC(DYV, j0));
   }
-  double vsh = HALF(vs0 + vs1);  // (vs0 + vs1) / 2., calc.c:198, carried from the row below
   for (int j = j0; j <= jn; j++) {
-    const double u4 = UF(ic, j + 2);
+    const double u4 = UF(ic, j + 2), ua = UF(ia, j);
+    const double d1 = u4 - u3;
+    bad = bad || !in_range(u4) || !in_range(ua);
     // x face west of column i, row j: velocities u(i-1), u(i)
-    const XN xn = x_neighbours(u2, UF(ia, j), lane);
-    const Face FX = make_face<SCH>(xn.m2, xn.m1, u2, xn.p1, HALF(up_p(xn.m1) + up_p(u2)),
-                                   HALF(up_m(xn.m1) + up_m(u2)), true);
-    const Side tw = side_of(FX, Dt, ROW2(R_DXC, R_IDXC, j));
-    const Side te = east_of(tw, lane);
-    const bool oke = __shfl_sync(FULL, (int)FX.ok, (lane + 1) & 31) != 0;
+    const XN xn = x_neighbours(u2, ua, lane);
+    const Face FX = x_face<SCH, true>(vel_pair(xn.m1, u2, xn.m1 + u2), xn, u2, dt);
+    const Side tw = side_of<true>(FX, METRIC(DXC, j));
     // y face north of row j: velocities v(i, j), v(i+1, j)
-    const double vn0 = VF(ic, j), vn1 = VF(ic1, j);
-    const Face FY = make_face<SCH>(u1, u2, u3, u4, HALF(up_p(vn0) + up_p(vn1)), HALF(up_m(vn0) + up_m(vn1)),
-                                   fin(vn0) && fin(vn1));
-    const Side tn = side_of(FY, Dt, ROW2(R_DYV, R_IDYV, j));
-    const Side ns = side_of(FY, Dt, ROW2(R_DYV, R_IDYV, j + 1));
-    const double S = sum_faces(tw, te, ts, tn);
-    const bool slow = !(FX.ok && oke && oks && FY.ok) || !nz(S);
-    const double vnh = HALF(vn0 + vn1);
+    const double va = VF(ic, j), vb = VF(ic1, j), vn = va + vb;
+    bad = bad || !in_range(va);  // vb is the next lane's
+    const Metric my = METRIC(DYV, j);
+    const Vel v = vel_pair(va, vb, vn);
+    const Face FY = make_face<SCH, true>(v, d0, v.pos ? dm : d1, u2, u3, u4, dt);
+    const Side tn = side_of<true>(FY, my);
+    const Side ns = side_of<true>(FY, METRIC(DYV, j + 1));
+    bool slow;
+    const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, u2, slow);
+    slow = __any_sync(FULL, bad) || slow;
+    // calc.c:198: u0*(uep-uwm)/(2 DXE) + u0*((vn0+vn1)/2 - (vs0+vs1)/2)/DYV; the
+    // halving commutes with the difference (its operands are zero or at least 2^-352)
+    const double ux = xn.p1 - xn.m1, vy = vn - vs;
+    const double p2 = Dt * (product_over(u2, ux, 0, METRIC(DXE2, j)) + product_over(u2, vy, 0xfff00000u, my));
     if (own) {
       double r;
-      if (slow) {
-        r = advu_cell_ool<SCH>(s, f, i, j);
-      } else {
-        const double uwm = xn.m1, u0 = u2, uep = xn.p1;  // calc.c:198
-        const double p2 = Dt * (div_rcp(u0 * (uep - uwm), ROW2(R_DXE2, R_IDXE2, j)) +
-                                div_rcp(u0 * (vnh - vsh), ROW2(R_DYV, R_IDYV, j)));
-        r = S + p2;
-      }
+      if (slow) r = advu_cell_ool<SCH>(s, f, i, j);
+      else r = S + p2;
       out[IX(W, i, j)] = r;
     }
     ts = ns;
-    oks = FY.ok;
-    vsh = vnh;
-    u1 = u2;
+    vs = vn;
     u2 = u3;
     u3 = u4;
+    dm = d0;
+    d0 = d1;
   }
   FAST_END
 }
@@ -723,54 +920,58 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
   SW2G_PDL_ENTRY();
   FAST_SETUP
   const int iu = min(i - 1, nx + 2);
-  // V at this lane's column, rows j-1 .. j+1; U at column i-1, row j
-  double v1 = VF(ic, j0 - 1), v2 = VF(ic, j0), v3 = VF(ic, j0 + 1);
+  // V at this lane's column, rows j-1 .. j+1, the differences of rows j-1 ..
+  // j+1; U at column i-1, row j
+  double v1 = VF(ic, j0 - 1), v2 = VF(ic, j0), v3 = VF(ic, j0 + 1), dm, d0;
   double uw0 = UF(iu, j0);
+  bool bad = !in_range(v1) || !in_range(v2) || !in_range(v3) || !in_range(uw0);
   Side ts;
-  bool oks;
   {
-    const Face F = make_face<SCH>(VF(ic, j0 - 2), v1, v2, v3, HALF(up_p(v1) + up_p(v2)),
-                                  HALF(up_m(v1) + up_m(v2)), true);
-    ts = side_of(F, Dt, ROW2(R_DYC, R_IDYC, j0));
-    oks = F.ok;
+    const double v0 = VF(ic, j0 - 2);
+    bad = bad || !in_range(v0);
+    const Vel v = vel_pair(v1, v2, v1 + v2);
+    dm = v2 - v1;
+    d0 = v3 - v2;
+    const Face F = make_face<SCH, true>(v, dm, v.pos ? v1 - v0 : d0, v1, v2, v3, dt);
+    ts = side_of<true>(F, METRIC(DYC, j0));
   }
   for (int j = j0; j <= jn; j++) {
-    const double v4 = VF(ic, j + 2);
-    const double uw1 = UF(iu, j + 1);
+    const double v4 = VF(ic, j + 2), va = VF(ia, j);
+    const double d1 = v4 - v3;
+    bad = bad || !in_range(v4) || !in_range(va);
+    const double uw1 = UF(iu, j + 1), uw = uw1 + uw0;
+    bad = bad || !in_range(uw1);
+    const Metric mx = METRIC(DXV, j);
     // x face west of column i, row j: velocities u(i-1, j+1), u(i-1, j)
-    const XN xn = x_neighbours(v2, VF(ia, j), lane);
-    const Face FX = make_face<SCH>(xn.m2, xn.m1, v2, xn.p1, HALF(up_p(uw1) + up_p(uw0)),
-                                   HALF(up_m(uw1) + up_m(uw0)), fin(uw1) && fin(uw0));
-    const Side tw = side_of(FX, Dt, ROW2(R_DXV, R_IDXV, j));
-    const Side te = east_of(tw, lane);
-    const bool oke = __shfl_sync(FULL, (int)FX.ok, (lane + 1) & 31) != 0;
-    // (u(i-1, j) + u(i-1, j+1))/2 and, from the next lane, (u(i, j) + u(i, j+1))/2 (calc.c:235)
-    const double uwh = HALF(uw0 + uw1);
-    const double ueh = __shfl_sync(FULL, uwh, (lane + 1) & 31);
+    const XN xn = x_neighbours(v2, va, lane);
+    const Face FX = x_face<SCH, true>(vel_pair(uw1, uw0, uw), xn, v2, dt);
+    const Side tw = side_of<true>(FX, mx);
     // y face north of row j: velocities v(i, j), v(i, j+1)
-    const Face FY = make_face<SCH>(v1, v2, v3, v4, HALF(up_p(v2) + up_p(v3)), HALF(up_m(v2) + up_m(v3)), true);
-    const Side tn = side_of(FY, Dt, ROW2(R_DYC, R_IDYC, j));
-    const Side ns = side_of(FY, Dt, ROW2(R_DYC, R_IDYC, j + 1));
-    const double S = sum_faces(tw, te, ts, tn);
-    const bool slow = !(FX.ok && oke && oks && FY.ok) || !nz(S);
+    const Vel v = vel_pair(v2, v3, v2 + v3);
+    const Face FY = make_face<SCH, true>(v, d0, v.pos ? dm : d1, v2, v3, v4, dt);
+    const Side tn = side_of<true>(FY, METRIC(DYC, j));
+    const Side ns = side_of<true>(FY, METRIC(DYC, j + 1));
+    bool slow;
+    const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, v2, slow);
+    slow = __any_sync(FULL, bad) || slow;
+    // calc.c:235: v0*((ue0+ue1)/2 - (uw0+uw1)/2)/DXV + v0*(vnp-vsm)/(DYN+DYN), the
+    // sums of u symmetric in their operands
+    const double ue = __shfl_sync(FULL, uw, (lane + 1) & 31);
+    const double ux = ue - uw, vy = v3 - v1;
+    const double p2 = Dt * (product_over(v2, ux, 0xfff00000u, mx) + product_over(v2, vy, 0, METRIC(DYNS, j)));
     if (own) {
       double r;
-      if (slow) {
-        r = advv_cell_ool<SCH>(s, f, i, j);
-      } else {
-        const double vsm = v1, v0 = v2, vnp = v3;  // calc.c:235
-        const double p2 = Dt * (div_rcp(v0 * (ueh - uwh), ROW2(R_DXV, R_IDXV, j)) +
-                                div_rcp(v0 * (vnp - vsm), ROW2(R_DYNS, R_IDYNS, j)));
-        r = S + p2;
-      }
+      if (slow) r = advv_cell_ool<SCH>(s, f, i, j);
+      else r = S + p2;
       out[IX(W, i, j)] = r;
     }
     ts = ns;
-    oks = FY.ok;
     uw0 = uw1;
     v1 = v2;
     v2 = v3;
     v3 = v4;
+    dm = d0;
+    d0 = d1;
   }
   FAST_END
 }
@@ -779,7 +980,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
 #undef UF
 #undef VF
 #undef HF
-#undef ROW2
+#undef METRIC
 
 // Self-check of div_rcp: for each divisor b, `samples` numerators a drawn
 // from a SplitMix64 stream (random significands over exponents 2^-950..2^60,
@@ -1463,15 +1664,17 @@ template <int SCH>
 void launch_bodies(int which, dim3 g, cudaStream_t st, const DevState& s, const F7& f, double* out) {
   if constexpr (SCH != 3) {
     const bool ud = !s.polar && s.sigma == 0.0;
-    if (s.plain && ud) {
-      if (which == 0) { fast_launch(k_mass_fast<SCH, true, true>, st, s, f, out); return; }
-    }
-    if (s.plain) {
+    if (!s.sig_ok) {
+      // Dt or a metric factor outside the range of the integer-pipe quotients
+    } else if (s.plain) {
+      if (which == 0 && ud) { fast_launch(k_mass_fast<SCH, true, true>, st, s, f, out); return; }
       if (which == 0) { fast_launch(k_mass_fast<SCH, true, false>, st, s, f, out); return; }
+      if (which == 1) { fast_launch(k_tracer_fast<SCH, true>, st, s, f, out); return; }
       if (which == 2) { fast_launch(k_adv_u_fast<SCH, true>, st, s, f, out); return; }
       if (which == 3) { fast_launch(k_adv_v_fast<SCH, true>, st, s, f, out); return; }
     } else {
       if (which == 0) { fast_launch(k_mass_fast<SCH, false, false>, st, s, f, out); return; }
+      if (which == 1) { fast_launch(k_tracer_fast<SCH, false>, st, s, f, out); return; }
       if (which == 2) { fast_launch(k_adv_u_fast<SCH, false>, st, s, f, out); return; }
       if (which == 3) { fast_launch(k_adv_v_fast<SCH, false>, st, s, f, out); return; }
     }

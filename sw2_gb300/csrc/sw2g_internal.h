@@ -33,6 +33,8 @@ enum Row {
   R_DYNS,  // DYN(j)+DYN(j+1)              calc.c:234
   R_SURF,  // DXC*DYC                      energy.c:40
   R_IDYV, R_IDXE2, R_IDYNS, R_IRZC, R_IRZN,  // 1.0/x of DYV, DXE2, DYNS, rZ(latc), rZ(latn): divisors of div_rcp
+  // 64-bit reciprocals (sig_recip, the integer's bits) of the divisors on the integer pipe
+  R_YDXE, R_YDXC, R_YDXV, R_YDYN, R_YDYC, R_YDYV, R_YDXE2, R_YDYNS, R_YRZC, R_YRZN,
   R_NUM
 };
 
@@ -52,6 +54,7 @@ struct DevState {
   double nu2dt, nu4dt, nu6dt;  // (nu)*(Dt) as the reference forms it (calc.c:346-348)
   int plain;           // windx, windy and hB are +0.0 in every padded cell
   int lape_eta;        // laplacian_eta of eta instead of u (SW2G_FLAG_LAPE_ETA)
+  int sig_ok;          // Dt and the metric factors lie in the range of the integer-pipe quotients
   int fk;              // rows per strip of the fast TVD bodies (set per launch)
   unsigned* strips;    // the fast bodies' strip queue: next strip, warps done (zero between launches)
   int polar;           // 0: band; +-1: polar cap, with the fields below
@@ -68,6 +71,8 @@ bool grid_ok(const sw2g_case* c);
 // Host geometry (geometry.cpp): fills rows[R_NUM*H]; returns the at-rest CFL
 // maxima used by compute_Dt when the flow is at rest (calc.c:715-725).
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my);
+// Whether Dt and every metric divisor of the rows lie in [2^-127, 2^129) (sigmath.cuh: in_window).
+bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows);
 // The fields of a polar cap (P_NUM x (nx+4)(ny+4)) and the at-rest CFL maxima
 // computed with them.
 void polar_fields(const sw2g_case& c, std::vector<double>& f, double* rest_mx, double* rest_my);
