@@ -424,8 +424,11 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 // [2^-127, 2^129) (DevState::sig_ok).
 constexpr int FW = 31;      // cells per strip along x (32 faces)
 constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the launch's queue
-// Resident blocks per SM the register allocation must allow.
-#define FAST_MIN_BLOCKS 5
+// Resident blocks per SM the register allocation must allow: 7 blocks (28
+// warps) at 72 registers hide the FP64 unit's latency best. k_adv_u at
+// 2048x1024 with 4, 5, 6, 7, 8 and 10 blocks: 0.138, 0.133, 0.128, 0.122,
+// 0.124 and 0.125 ms.
+#define FAST_MIN_BLOCKS 7
 constexpr unsigned FULL = 0xffffffffu;
 
 
@@ -439,8 +442,6 @@ __device__ __forceinline__ long long key(double x) {  // order-preserving intege
   return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
 __device__ __forceinline__ bool nz(double x) { return (dbits(x) & 0x7fffffffffffffffLL) != 0; }
-__device__ __forceinline__ bool gt0(double x) { return dbits(x) > 0; }
-__device__ __forceinline__ bool lt0(double x) { return key(x) < -1; }
 __device__ __forceinline__ double mn(double a, double b) { return key(a) < key(b) ? a : b; }  // sw.h MIN
 __device__ __forceinline__ double mx(double a, double b) { return key(a) > key(b) ? a : b; }  // sw.h MAX
 
@@ -458,6 +459,7 @@ __device__ __forceinline__ double limiter_fast(double r) {
 }
 
 // Operands of the integer-pipe quotients and products.
+constexpr unsigned long long kSign = 0x8000000000000000ULL;
 __device__ __forceinline__ unsigned long long mag(double x) {
   return (unsigned long long)dbits(x) & 0x7fffffffffffffffULL;
 }
@@ -481,7 +483,7 @@ __device__ __forceinline__ double flip(double x, unsigned long long neg) {
   return __longlong_as_double(dbits(x) ^ (long long)neg);
 }
 __device__ __forceinline__ unsigned long long sign_of(double x) {
-  return (unsigned long long)dbits(x) & 0x8000000000000000ULL;
+  return (unsigned long long)dbits(x) & kSign;
 }
 
 // A row metric as a divisor: its bits and its reciprocal (sig_recip).
@@ -492,6 +494,30 @@ __device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j
   return Metric{(unsigned long long)dbits(RW(s, t, j)), (unsigned long long)dbits(RW(s, ty, j))};
 }
 #define METRIC(NAME, j) metric(s, R_##NAME, R_Y##NAME, j)
+
+// Products and quotients of any operands, on the integer pipe when the
+// operands are of magnitude 2^-255 .. 2^257 (the result is then normal), on
+// the FP64 unit, out of line, otherwise. c: a factor that is finite and not
+// zero (a row constant or a coefficient): a zero times it is that zero.
+__device__ __forceinline__ bool mid(double x) { return ((hi_word(x) - 0x30000000u) & 0x60000000u) == 0; }
+__device__ __noinline__ double mul_fp64(double a, double b) { return a * b; }
+__device__ __forceinline__ double smul(double a, double b) {
+  if (mid(a) && mid(b)) return from_bits(sig_mul(mag(a), mag(b)) | ((unsigned long long)(dbits(a) ^ dbits(b)) & kSign));
+  return mul_fp64(a, b);
+}
+__device__ __forceinline__ double cmul(double c, double a) {
+  const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(c)) & kSign;
+  if (mid(a) && mid(c)) return from_bits(sig_mul(mag(a), mag(c)) | sg);
+  if (!nz(a)) return from_bits(sg);
+  return mul_fp64(c, a);
+}
+__device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
+// a / x.b (x.b > 0; s.sig_ok): a zero gives itself.
+__device__ __forceinline__ double mdiv(double a, const Metric& x) {
+  if (mid(a) && x.y) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
+  if (!nz(a)) return a;
+  return div_fp64(a, from_bits(x.b));
+}
 
 // RN(RN(a*b)*2^k / x) of zero or in-range a and b (k20 = k << 20).
 __device__ __forceinline__ double product_over(double a, double b, unsigned k20, const Metric& x) {
@@ -590,13 +616,21 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, dou
   return F;
 }
 
+// (hp*g)*d of zero or in-range factors, rounded twice as written. On the
+// integer pipe: k_adv_u at 2048x1024 0.146 ms with both products on the FP64
+// unit, 0.136 with one of them, 0.133 with none (the mass body 0.118, 0.109,
+// 0.101); c*B, whose B may be anything, stays there.
+__device__ __forceinline__ double slope_term(double hp, double g, double d) {
+  const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
+  return (nz(hp) && nz(g) && nz(d)) ? from_bits(sig_mul(sig_mul(mag(hp), mag(g)), mag(d)) | sg) : 0.0;
+}
 // C*B of one side with c = |C|: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or
 // B2BM = q1 - psi*0.5*(1-c)*(q1-q0) (C- = -c; q1 - X = q1 + (-X) exactly).
 __device__ __forceinline__ double side_term(bool pos, unsigned long long p, const Metric& dx, double hp, double q0,
                                             double q1, double d) {
   const double c = from_bits(sig_div_known(p, dx.b, dx.y));
-  const double X = (hp * (1.0 - c)) * d;
-  const unsigned long long neg = pos ? 0 : 0x8000000000000000ULL;
+  const double X = slope_term(hp, 1.0 - c, d);
+  const unsigned long long neg = pos ? 0 : kSign;
   return flip(c * (pick(pos, q0, q1) + flip(X, neg)), neg);
 }
 
@@ -980,8 +1014,6 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
 #undef UF
 #undef VF
 #undef HF
-#undef METRIC
-
 // Self-check of div_rcp: for each divisor b, `samples` numerators a drawn
 // from a SplitMix64 stream (random significands over exponents 2^-950..2^60,
 // both signs, and numerators whose quotient lies within a few ulps of a
@@ -1191,8 +1223,8 @@ __global__ void k_lape_pass1(DevState s, const double* e, double* psi, double* x
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  psi[q] = div_rcp(RW(s, R_KX, j) * (e[IX(W, i + 1, j)] - e[q]), RW(s, R_DXC, j), RW(s, R_IDXC, j));
-  xi[q] = div_rcp(RW(s, R_KY, j) * (e[IX(W, i, j + 1)] - e[q]), RW(s, R_DYC, j), RW(s, R_IDYC, j));
+  psi[q] = mdiv(cmul(RW(s, R_KX, j), e[IX(W, i + 1, j)] - e[q]), METRIC(DXC, j));
+  xi[q] = mdiv(cmul(RW(s, R_KY, j), e[IX(W, i, j + 1)] - e[q]), METRIC(DYC, j));
 }
 
 // laplacian_eta second pass (laplacian.c:125-127)
@@ -1202,8 +1234,8 @@ __global__ void k_lape_pass2(DevState s, const double* psi, const double* xi, do
   INTERIOR_IJ
   const int q = IX(W, i, j);
   const double v =
-      RW(s, R_KC, j) * sadd(div_rcp(psi[q] - psi[IX(W, i - 1, j)], RW(s, R_DXE, j), RW(s, R_IDXE, j)),
-                        div_rcp(xi[q] - xi[IX(W, i, j - 1)], RW(s, R_DYN, j), RW(s, R_IDYN, j)));
+      cmul(RW(s, R_KC, j), mdiv(psi[q] - psi[IX(W, i - 1, j)], METRIC(DXE, j)) +
+                              mdiv(xi[q] - xi[IX(W, i, j - 1)], METRIC(DYN, j)));
   put_images<HK_LE>(s, eo, i, j, v);
 }
 
@@ -1235,7 +1267,7 @@ __device__ __forceinline__ double hyper_terms(const DevState& s, double x, const
 #pragma unroll
     for (int t = 0; t < 3; t++) {
       const double v = V[t];
-      if ((NZ >> t) & 1) x = sadd(x, nd[t] * v);
+      if ((NZ >> t) & 1) x = x + cmul(nd[t], v);
       else if (!zero_term_is_exact(x, v)) x = add_product(x, nd[t], v);
     }
     return x;
@@ -1293,18 +1325,18 @@ __global__ void k_pres_sum(DevState s, F7 f, const double* duadv, const double* 
   const double* e = f.eta;
   const double mge = s.polar ? -PF(s, P_GE, q) * s.Dt : RW(s, R_MGEDT, j);  // -GE*Dt, calc.c:517
   const double mgn = s.polar ? -PF(s, P_GN, q) * s.Dt : RW(s, R_MGNDT, j);
-  const double dup = div_rcp(mge * (e[IX(W, i + 1, j)] - e[q]), RW(s, R_DXC, j), RW(s, R_IDXC, j));
-  const double dvp = div_rcp(mgn * (e[IX(W, i, j + 1)] - e[q]), RW(s, R_DYC, j + 1), RW(s, R_IDYC, j + 1));
-  double a = sadd(duadv[q], dup);
-  double b = sadd(dvadv[q], dvp);
+  const double dup = mdiv(cmul(mge, e[IX(W, i + 1, j)] - e[q]), METRIC(DXC, j));
+  const double dvp = mdiv(cmul(mgn, e[IX(W, i, j + 1)] - e[q]), METRIC(DYC, j + 1));
+  double a = duadv[q] + dup;
+  double b = dvadv[q] + dvp;
   if constexpr (UD) {
     const double U = f.u[q], V = f.v[q];
     if (!zero_term_is_exact(a, U)) a = minus_damping(a, U, s.sigma, s.Dt);
     if (!zero_term_is_exact(b, V)) b = minus_damping(b, V, s.sigma, s.Dt);
   } else {
     const double su = s.polar ? PF(s, P_SU, q) : s.sigma, sv = s.polar ? PF(s, P_SV, q) : s.sigma;  // calc.c:374-394
-    a = ssub(a, f.u[q] * su * s.Dt);
-    b = ssub(b, f.v[q] * sv * s.Dt);
+    a = a - f.u[q] * su * s.Dt;
+    b = b - f.v[q] * sv * s.Dt;
   }
   dun[q] = a;
   dvn[q] = b;
@@ -1325,17 +1357,15 @@ __global__ void k_lapv_pass1(DevState s, const double* uu, const double* vv, dou
   const int j0 = blockIdx.y * LV_ROWS + 1;
   if (i > s.nx) return;
   const int j1 = min(j0 + LV_ROWS - 1, s.ny);
-  double pu = RW(s, R_DXC, j0) * uu[IX(W, i, j0)];
-  double qv = RW(s, R_DXV, j0 - 1) * vv[IX(W, i, j0 - 1)];
+  double pu = cmul(RW(s, R_DXC, j0), uu[IX(W, i, j0)]);
+  double qv = cmul(RW(s, R_DXV, j0 - 1), vv[IX(W, i, j0 - 1)]);
   for (int j = j0; j <= j1; j++) {
     const int q = IX(W, i, j);
-    const double pu1 = RW(s, R_DXC, j + 1) * uu[IX(W, i, j + 1)];
-    const double qv1 = RW(s, R_DXV, j) * vv[q];
-    double a = RW(s, R_IDXV, j), b = -RW(s, R_IDYC, j + 1);
-    const double z = a * sadd((vv[IX(W, i + 1, j)] - vv[q]), b * (pu1 - pu));
-    a = RW(s, R_IDXE, j);
-    b = RW(s, R_IDYN, j);
-    const double d = a * sadd((uu[q] - uu[IX(W, i - 1, j)]), b * (qv1 - qv));
+    const double pu1 = cmul(RW(s, R_DXC, j + 1), uu[IX(W, i, j + 1)]);
+    const double qv1 = cmul(RW(s, R_DXV, j), vv[q]);
+    // x + (-b)*y is x - b*y
+    const double z = cmul(RW(s, R_IDXV, j), (vv[IX(W, i + 1, j)] - vv[q]) - cmul(RW(s, R_IDYC, j + 1), pu1 - pu));
+    const double d = cmul(RW(s, R_IDXE, j), (uu[q] - uu[IX(W, i - 1, j)]) + cmul(RW(s, R_IDYN, j), qv1 - qv));
     put_images<HK_ZE>(s, ze, i, j, z);
     put_images<HK_DI>(s, di, i, j, d);
     if (j == s.ny && s.polar == 0)  // laplacian.c:73
@@ -1351,11 +1381,10 @@ __global__ void k_lapv_pass2(DevState s, const double* ze, const double* di, dou
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  double a = -RW(s, R_IDYN, j), b = RW(s, R_IDXC, j);
-  const double vu = sadd(a * ssub(ze[q], ze[IX(W, i, j - 1)]), b * ssub(di[IX(W, i + 1, j)], di[q]));
-  a = RW(s, R_IDXV, j);
-  b = RW(s, R_IDYC, j + 1);
-  const double vl = sadd(a * ssub(ze[q], ze[IX(W, i - 1, j)]), b * ssub(di[IX(W, i, j + 1)], di[q]));
+  const double z = ze[q], d = di[q];
+  // (-a)*x + b*y = b*y - a*x
+  const double vu = cmul(RW(s, R_IDXC, j), di[IX(W, i + 1, j)] - d) - cmul(RW(s, R_IDYN, j), z - ze[IX(W, i, j - 1)]);
+  const double vl = cmul(RW(s, R_IDXV, j), z - ze[IX(W, i - 1, j)]) + cmul(RW(s, R_IDYC, j + 1), di[IX(W, i, j + 1)] - d);
   put_images<HK_LU>(s, lu, i, j, vu);
   put_images<HK_LV>(s, lv, i, j, vl);
 }
@@ -1401,8 +1430,8 @@ __device__ __forceinline__ bool range_bad(double x, bool first) {
 //   eta: the geofactor (calc.c:403-422) and eta += D (core.c:203-205);
 //   u, v: the Coriolis update (calc.c:542-598).
 __device__ __forceinline__ double ab3(double dn, double dm1, double dm2) {
-  const double t = sadd(-(4.0 / 3.0) * dm1, +(5.0 / 12.0) * dm2);
-  return sadd((23.0 / 12.0) * dn, t);  // 1.0 * t is t
+  const double t = cmul(5.0 / 12.0, dm2) - cmul(4.0 / 3.0, dm1);  // -(4/3)*dm1 + (5/12)*dm2
+  return cmul(23.0 / 12.0, dn) + t;  // 1.0 * t is t
 }
 // v + (+0): v, except that -0 becomes +0 (the plain form's zero winds).
 __device__ __forceinline__ double plus_pos_zero(double v) {
@@ -1427,9 +1456,9 @@ __global__ void k_eta_ab3(DevState s, F7 f, double* eta, double* dn, const doubl
   const double e = f.eta[q];
   if constexpr (PL) {
     const double h = e + s.depth;  // - hB with hB = +0 is exact
-    ab -= (HALF(RW(s, R_GEO, j) * h) * (plus_pos_zero(f.v[q]) + plus_pos_zero(f.v[IX(W, i, j - 1)])));
+    ab -= smul(HALF(cmul(RW(s, R_GEO, j), h)), plus_pos_zero(f.v[q]) + plus_pos_zero(f.v[IX(W, i, j - 1)]));
   } else {
-    ab -= (HALF(RW(s, R_GEO, j) * HH(i, j)) * (VW(i, j) + VW(i, j - 1)));
+    ab -= smul(HALF(cmul(RW(s, R_GEO, j), HH(i, j))), VW(i, j) + VW(i, j - 1));
   }
   const double en = e + ab;
   put_images<HK_WRAP>(s, eta, i, j, en);  // with eta's halo update (core.c:206-210)
@@ -1446,12 +1475,12 @@ __global__ void k_coriolis_u_ab3(DevState s, double* u, const double* v, double*
   const double x = hyper_terms<NZ>(s, dn[q], l2, l4, l6, q);
   if constexpr (NZ != kNoHyper) dn[q] = x;
   const double duab = ab3(x, dm1[q], dm2[q]);
-  const double semi =
-      QUARTER(sadd(sadd(sadd(v[IX(W, i, j)], v[IX(W, i + 1, j)]), v[IX(W, i, j - 1)]), v[IX(W, i + 1, j - 1)]));
+  const double u0 = u[q];
+  const double semi = QUARTER(v[IX(W, i, j)] + v[IX(W, i + 1, j)] + v[IX(W, i, j - 1)] + v[IX(W, i + 1, j - 1)]);
   const double dtf = s.polar ? s.Dt * PF(s, P_FE, q) : RW(s, R_DTFE, j);
-  const double al = sadd(dtf, div_rcp(s.Dt * u[q] * RW(s, R_SINC, j), RW(s, R_RZC, j), RW(s, R_IRZC, j)));
-  const double be = QUARTER(al) * al;
-  const double un = sadd(ssub(sadd(u[q], duab), be * u[q]), al * semi) / sadd(1.0, be);
+  const double al = dtf + mdiv(cmul(s.Dt, u0) * RW(s, R_SINC, j), METRIC(RZC, j));
+  const double be = smul(QUARTER(al), al);
+  const double un = quotient(((u0 + duab) - smul(be, u0)) + smul(al, semi), 1.0 + be);
   u[q] = un;
   check_range(bad, un, i, j);
 }
@@ -1466,12 +1495,12 @@ __global__ void k_coriolis_v_ab3(DevState s, const double* u, double* v, double*
   const double x = hyper_terms<NZ>(s, dn[q], l2, l4, l6, q);
   if constexpr (NZ != kNoHyper) dn[q] = x;
   const double dvab = ab3(x, dm1[q], dm2[q]);
-  const double semi =
-      QUARTER(sadd(sadd(sadd(u[IX(W, i - 1, j + 1)], u[IX(W, i, j + 1)]), u[IX(W, i, j)]), u[IX(W, i - 1, j)]));
+  const double v0 = v[q];
+  const double semi = QUARTER(u[IX(W, i - 1, j + 1)] + u[IX(W, i, j + 1)] + u[IX(W, i, j)] + u[IX(W, i - 1, j)]);
   const double dtf = s.polar ? s.Dt * PF(s, P_FN, q) : RW(s, R_DTFN, j);
-  const double al = sadd(dtf, div_rcp(s.Dt * semi * RW(s, R_SINN, j), RW(s, R_RZN, j), RW(s, R_IRZN, j)));
-  const double be = QUARTER(al) * al;
-  const double vn = ssub(ssub(sadd(v[q], dvab), be * v[q]), al * semi) / sadd(1.0, be);
+  const double al = dtf + mdiv(cmul(s.Dt, semi) * RW(s, R_SINN, j), METRIC(RZN, j));
+  const double be = smul(QUARTER(al), al);
+  const double vn = quotient(((v0 + dvab) - smul(be, v0)) - smul(al, semi), 1.0 + be);
   v[q] = vn;
   // a band's row ny is a wall: do_channel zeroes it before the range check
   // (core.c:303-312), so the check sees +0 there
