@@ -21,6 +21,7 @@ namespace {
 
 constexpr int TX = 128;
 
+
 __device__ __forceinline__ int IX(int W, int i, int j) { return (i + 1) + (j + 1) * W; }
 __device__ __forceinline__ double RW(const DevState& s, int t, int j) { return s.rows[t * s.H + j + 1]; }
 // A field of a polar cap at padded index q.
@@ -1658,21 +1659,28 @@ __global__ void k_range(DevState s, RangeFields r, int* bad) {
 
 // Launch of a fast body. Its warps take strips of 31 columns x fk rows from
 // a queue (next_strip), and the grid is the blocks resident on the device at
-// once (or fewer when there are fewer strips). Measured on the 2048x1024 and
-// 4096x2048 workloads with strips dealt in turn (bodies' CUDA-event times for
-// 8, 12, 16 and 24 rows): 12 rows is the best or within 0.2 % of it on both,
-// 16 loses 10 % at 2048x1024, where its 1.4 rounds of strips leave most warps
-// idle in the second. The queue instead of the fixed turns: the same time at
-// 2048x1024, 1 % less at 4096x2048. With the queue, 8 rows beat 12 by 0.6 %
-// at 2048x1024 (1.9 rounds of 12-row strips, 2.8 of 8-row ones) and lose
-// 0.6 % at 4096x2048 (7.5 rounds of 12-row strips): the tallest strip that
-// gives every resident warp at least 2.5 strips, down to 4 rows.
+// once (or fewer when there are fewer strips). A strip costs its rows and
+// about one row more (the face south of its first row); the queue evens out
+// the warps' different speeds, and the last strips run with part of the warps
+// idle, about 0.3 of a strip's time on average. So the height is the one with
+// the least (fk + 1) * max(1, strips per resident warp + 0.3). Measured
+// (k_adv_u, 4256 resident warps): at 2048x1024 9 rows 0.123 ms and 17 rows,
+// one strip for each warp, 0.140; at 4096x2048 16 rows 0.480, 8 rows 0.492
+// and 32 rows 0.486; at 256x128, where every strip finds a warp, 1 row 0.014
+// and 4 rows 0.022 (with the timers' events).
 int choose_strip_rows(int nx, int ny, long long warps) {
-  for (int fk : {12, 8, 6}) {
+  int best = 1;
+  double least = 0;
+  for (int fk = 1; fk <= 24; fk++) {
     const long long strips = (long long)((nx + FW - 1) / FW) * ((ny + fk - 1) / fk);
-    if (2 * strips >= 5 * warps) return fk;
+    const double rounds = (double)strips / (double)warps + 0.3;
+    const double cost = (fk + 1) * (rounds > 1.0 ? rounds : 1.0);
+    if (fk == 1 || cost < least) {
+      least = cost;
+      best = fk;
+    }
   }
-  return 4;
+  return best;
 }
 
 template <typename K>
