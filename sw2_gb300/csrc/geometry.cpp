@@ -55,7 +55,10 @@ uint64_t bits_of(double x) {
   std::memcpy(&b, &x, sizeof b);
   return b;
 }
-bool positive_in_window(uint64_t b) { return !(b >> 63) && in_window((uint32_t)(b >> 32)); }
+bool positive_in_window(uint64_t b) {  // 2^-20 <= x < 2^60
+  const uint32_t hi = (uint32_t)(b >> 32);
+  return hi >= (1003u << 20) && hi < (1083u << 20);
+}
 
 }  // namespace
 

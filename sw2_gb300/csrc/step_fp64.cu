@@ -55,6 +55,19 @@ __device__ __forceinline__ double zdiv(double a, double b) {
   return a / b;
 }
 
+// The literal cells' division: on the integer pipe where both operands and
+// the quotient are normal numbers (sigmath.cuh), else as zdiv. Out of line: a
+// cell has up to eighteen of them.
+__device__ __noinline__ double ldiv(double a, double b) {
+  const unsigned ea = (unsigned)(((unsigned long long)dbits(a) >> 52) & 0x7ff);
+  const unsigned eb = (unsigned)(((unsigned long long)dbits(b) >> 52) & 0x7ff);
+  if (ea - 1 < 2046u && eb - 1 < 2046u && ea - eb + 1021u < 2043u) {
+    const unsigned long long m = 0x7fffffffffffffffULL, A = (unsigned long long)dbits(a), B = (unsigned long long)dbits(b);
+    return __longlong_as_double((long long)(sig_div(A & m, B & m) | ((A ^ B) & ~m)));
+  }
+  return zdiv(a, b);
+}
+
 // x * 2^k for k in -2..1 (p = 2^k), the same value as the FP64 product: when
 // x and the product are normal numbers, the product only changes the exponent
 // field, done here on the integer pipe; zeros are their own product; other
@@ -195,8 +208,8 @@ template <int SCH>
 __device__ __forceinline__ void tvd_face(double qm, double q0, double q1, double q2, double cP, double cM,
                                          double& BP, double& BM) {
   const double d = q1 - q0;
-  const double rP = (d != 0) ? zdiv(q0 - qm, d) : 0.0;
-  const double rM = (d != 0) ? zdiv(q2 - q1, d) : 0.0;
+  const double rP = (d != 0) ? ldiv(q0 - qm, d) : 0.0;
+  const double rM = (d != 0) ? ldiv(q2 - q1, d) : 0.0;
   BP = q0 + limiter<SCH>(rP) * 0.5 * (1 - cP) * d;
   BM = q1 - limiter<SCH>(rM) * 0.5 * (1 + cM) * d;
 }
@@ -213,13 +226,13 @@ __device__ __forceinline__ double tvd_sum(const double* qx, const double* qy, do
   return cwP * wP + cwM * wM - ceP * eP - ceM * eM + csP * sP + csM * sM - cnP * nP - cnM * nM;
 }
 
-__device__ __forceinline__ double cpos(double a, double dt, double dx) { return zdiv(0.5 * (a + fabs(a)) * dt, dx); }
-__device__ __forceinline__ double cneg(double a, double dt, double dx) { return zdiv(0.5 * (a - fabs(a)) * dt, dx); }
+__device__ __forceinline__ double cpos(double a, double dt, double dx) { return ldiv(0.5 * (a + fabs(a)) * dt, dx); }
+__device__ __forceinline__ double cneg(double a, double dt, double dx) { return ldiv(0.5 * (a - fabs(a)) * dt, dx); }
 __device__ __forceinline__ double cpos2(double a, double b, double dt, double dx) {
-  return zdiv(0.5 * (0.5 * (a + fabs(a)) + 0.5 * (b + fabs(b))) * dt, dx);
+  return ldiv(0.5 * (0.5 * (a + fabs(a)) + 0.5 * (b + fabs(b))) * dt, dx);
 }
 __device__ __forceinline__ double cneg2(double a, double b, double dt, double dx) {
-  return zdiv(0.5 * (0.5 * (a - fabs(a)) + 0.5 * (b - fabs(b))) * dt, dx);
+  return ldiv(0.5 * (0.5 * (a - fabs(a)) + 0.5 * (b - fabs(b))) * dt, dx);
 }
 
 struct F7 {
@@ -298,8 +311,8 @@ __device__ __forceinline__ double tracer_cell(const DevState& s, const F7& f, in
   const double pv1 = tvd_sum<SCH>(qx, qy, cpos(a, Dt, dxe), cneg(a, Dt, dxe), cpos(b, Dt, dxe), cneg(b, Dt, dxe),
                                   cpos(c, Dt, dyn), cneg(c, Dt, dyn), cpos(d, Dt, dyn), cneg(d, Dt, dyn));
   const double t = qx[2];
-  double pv2 = zdiv(Dt * t * (b - a), dxe);
-  pv2 += zdiv(Dt * t * (d - c), dyn);
+  double pv2 = ldiv(Dt * t * (b - a), dxe);
+  pv2 += ldiv(Dt * t * (d - c), dyn);
   double acc = pv1 + pv2;
   const double sigma = s.polar ? PF(s, P_STR, IX(W, i, j)) : s.sigma_tr;  // calc.c:152-161
   acc -= 2.0 * Dt * (sigma) * t;
@@ -326,7 +339,7 @@ __device__ __forceinline__ double advu_cell(const DevState& s, const F7& f, int 
   const double p1 = tvd_sum<SCH>(qx, qy, cpos2(uwm, u0, Dt, dxc), cneg2(uwm, u0, Dt, dxc), cpos2(u0, uep, Dt, dxc),
                                  cneg2(u0, uep, Dt, dxc), cpos2(vs0, vs1, Dt, dyv), cneg2(vs0, vs1, Dt, dyv),
                                  cpos2(vn0, vn1, Dt, dyv), cneg2(vn0, vn1, Dt, dyv));
-  const double p2 = Dt * (zdiv(u0 * (uep - uwm), RW(s, R_DXE2, j)) + zdiv(u0 * ((vn0 + vn1) / 2. - (vs0 + vs1) / 2.), dyv));
+  const double p2 = Dt * (ldiv(u0 * (uep - uwm), RW(s, R_DXE2, j)) + ldiv(u0 * ((vn0 + vn1) / 2. - (vs0 + vs1) / 2.), dyv));
   return p1 + p2;
 }
 
@@ -350,7 +363,7 @@ __device__ __forceinline__ double advv_cell(const DevState& s, const F7& f, int 
   const double p1 = tvd_sum<SCH>(qx, qy, cpos2(uw1, uw0, Dt, dxv), cneg2(uw1, uw0, Dt, dxv), cpos2(ue1, ue0, Dt, dxv),
                                  cneg2(ue1, ue0, Dt, dxv), cpos2(vsm, v0, Dt, dyc), cneg2(vsm, v0, Dt, dyc),
                                  cpos2(v0, vnp, Dt, dyc), cneg2(v0, vnp, Dt, dyc));
-  const double p2 = Dt * (zdiv(v0 * ((ue0 + ue1) / 2. - (uw0 + uw1) / 2.), dxv) + zdiv(v0 * (vnp - vsm), RW(s, R_DYNS, j)));
+  const double p2 = Dt * (ldiv(v0 * ((ue0 + ue1) / 2. - (uw0 + uw1) / 2.), dxv) + ldiv(v0 * (vnp - vsm), RW(s, R_DYNS, j)));
   return p1 + p2;
 }
 
@@ -407,22 +420,24 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 //      second term's divisions) and the products that enter them are taken
 //      from the operands' bits (sigmath.cuh: IEEE results); the FP64 unit
 //      keeps the additions and the products around them.
-// Ranges: each value that a warp reads is zero or of magnitude 2^-300 ..
+// Ranges. Each value that a warp reads is zero or of magnitude 2^-850 ..
 // 2^100 (in_range); otherwise the warp's cells are recomputed literally for
 // the rest of its strip. Differences and sums of such values are zero or at
-// least 2^-352 (they are multiples of the smallest unit among them), so no
-// quotient or product leaves the normal range, and no slope ratio, of the
-// side in use or not, exceeds 2^453, for which every limiter (squares
-// included) is finite.
+// least 2^-902 (they are multiples of the smallest unit among them), so slope
+// ratios and Courant numbers are normal; products of several factors are
+// tested, and taken on the FP64 unit where they could be subnormal. The
+// skipped side is finite if its slope ratio is below 2^498 (then every
+// limiter, squares included, is), which a difference of at least 2^-397
+// ensures; below that the ratio's exponent is looked at (make_face).
 // Zero sums. A sum that is zero because nonzero terms cancel is +0, as the
 // reference's is (x - x = +0, and +0 plus or minus a zero is +0). When every
-// term is zero the reference's sum is +0 if its first term is +0, which holds
-// when the + side's velocity at the west face is not positive and that
-// side's face value is not negative (west_plus_zero): a flow at rest.
-// Otherwise the cell is recomputed literally.
+// term is zero the reference's sum is +0 if its first term is +0: the + side
+// at the west face, whose Courant number is never negative, with a face value
+// that is not negative (first_term_plus_zero). So it is in a flow at rest and
+// for a tracer that is zero. Otherwise the cell is recomputed literally.
 // The Van Leer limiter in its reference form (0/0 at r = -1) keeps the
 // literal kernels, and so do cases whose Dt or metric factors lie outside
-// [2^-127, 2^129) (DevState::sig_ok).
+// 2^-20 .. 2^60 (DevState::sig_ok).
 constexpr int FW = 31;      // cells per strip along x (32 faces)
 constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the launch's queue
 // Resident blocks per SM the register allocation must allow: 7 blocks (28
@@ -466,9 +481,12 @@ __device__ __forceinline__ unsigned long long mag(double x) {
 }
 __device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)((unsigned long long)dbits(x) >> 32); }
 __device__ __forceinline__ bool usable(double x) { return in_window(hi_word(x)); }
-// zero, or 2^-300 <= |x| < 2^100
+// the upper word of |x|, and of 2^k
+__device__ __forceinline__ unsigned hi_mag(double x) { return hi_word(x) & 0x7fffffffu; }
+#define HI_POW2(k) ((unsigned)(1023 + (k)) << 20)
+// zero, or 2^-850 <= |x| < 2^100
 __device__ __forceinline__ bool in_range(double x) {
-  return ((hi_word(x) & 0x7fffffffu) - (723u << 20)) < (400u << 20) || !nz(x);
+  return hi_mag(x) - HI_POW2(-850) < (950u << 20) || !nz(x);
 }
 __device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
 // p ? a : b, opaque: one operation on the selected value stays one FP64
@@ -520,11 +538,16 @@ __device__ __forceinline__ double mdiv(double a, const Metric& x) {
   return div_fp64(a, from_bits(x.b));
 }
 
-// RN(RN(a*b)*2^k / x) of zero or in-range a and b (k20 = k << 20).
+// (a*(b*2^k))/x of zero or in-range a and b (k20 = k << 20, k = 0 or -1: b*2^k
+// is exact). Where the product could be subnormal, on the FP64 unit.
+__device__ __noinline__ double product_over_fp64(double a, double b, double x) { return zdiv(a * b, x); }
 __device__ __forceinline__ double product_over(double a, double b, unsigned k20, const Metric& x) {
-  const unsigned long long p = sig_mul(mag(a), mag(b), k20);
-  const unsigned long long q = sig_div_known(p, x.b, x.y);
-  return (nz(a) && nz(b)) ? from_bits(q | (sign_of(a) ^ sign_of(b))) : 0.0;
+  if (!nz(a) || !nz(b)) return 0.0;
+  if (min(hi_mag(a), hi_mag(b)) >= HI_POW2(-450)) {
+    const unsigned long long q = sig_div_known(sig_mul(mag(a), mag(b), k20), x.b, x.y);
+    return from_bits(q | (sign_of(a) ^ sign_of(b)));
+  }
+  return product_over_fp64(a, from_bits((unsigned long long)dbits(b) + ((unsigned long long)k20 << 32)), from_bits(x.b));
 }
 
 // a/b on the integer pipe where both are usable (the quotient is then normal),
@@ -588,10 +611,11 @@ struct Face {
   bool pos, act, both;
 };
 // PAIR: w is a sum of two velocities, to be halved. n1: q0 - qm when v.pos,
-// q2 - q1 otherwise; q2 is read when both sides are in use.
-template <int SCH, bool PAIR>
-__device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, double q0, double q1, double q2,
-                                          unsigned long long dt) {
+// q2 - q1 otherwise; n2(): the other of the two. bad is set where the skipped
+// side might not be finite.
+template <int SCH, bool PAIR, typename N2>
+__device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, N2 n2, double q0, double q1,
+                                          unsigned long long dt, bool& bad) {
   constexpr unsigned K = PAIR ? 0xfff00000u : 0u;  // exponent of the halving
   Face F;
   F.d = d;
@@ -601,6 +625,7 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, dou
   F.act = v.act;
   F.both = v.both;
   F.hp = half_psi<SCH>(n1, d);
+  if (hi_mag(d) < HI_POW2(-397) && nz(d)) bad = bad || hi_mag(n2()) >= hi_mag(d) + (490u << 20);
   F.p = sig_mul(mag(v.w), dt, K);
   F.hp2 = 0.0;
   F.p2 = 0;
@@ -610,20 +635,25 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, dou
         const bool apos = dbits(v.a) > 0;
         F.p = sig_mul(mag(apos ? v.a : v.b), dt, K);
         F.p2 = sig_mul(mag(apos ? v.b : v.a), dt, K);
-        F.hp2 = half_psi<SCH>(q2 - q1, d);
+        F.hp2 = half_psi<SCH>(n2(), d);
       }
     }
   }
   return F;
 }
 
-// (hp*g)*d of zero or in-range factors, rounded twice as written. On the
+// (hp*g)*d, rounded twice as written. On the
 // integer pipe: k_adv_u at 2048x1024 0.146 ms with both products on the FP64
 // unit, 0.136 with one of them, 0.133 with none (the mass body 0.118, 0.109,
 // 0.101); c*B, whose B may be anything, stays there.
+__device__ __noinline__ double product3_fp64(double a, double b, double c) { return (a * b) * c; }
 __device__ __forceinline__ double slope_term(double hp, double g, double d) {
-  const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
-  return (nz(hp) && nz(g) && nz(d)) ? from_bits(sig_mul(sig_mul(mag(hp), mag(g)), mag(d)) | sg) : 0.0;
+  if (!nz(hp) || !nz(d)) return 0.0;
+  if (usable(hp) && usable(g) && hi_mag(d) >= HI_POW2(-700)) {
+    const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
+    return from_bits(sig_mul(sig_mul(mag(hp), mag(g)), mag(d)) | sg);
+  }
+  return product3_fp64(hp, g, d);
 }
 // C*B of one side with c = |C|: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or
 // B2BM = q1 - psi*0.5*(1-c)*(q1-q0) (C- = -c; q1 - X = q1 + (-X) exactly).
@@ -672,15 +702,18 @@ __device__ __noinline__ double sum_faces8(double wP, double wM, double eP, doubl
   S = S - nM;
   return S;
 }
-// Whether the reference's first term at a west face qm | q0 | q1 whose + side
-// has no positive velocity is +0: its face value q0 + X must not be negative.
-// With the Courant number 0, X is a zero where q1 = q0, and otherwise
-// |X| <= |q1-q0| + |q0-qm| for every limiter (|psi(r)| <= 2 + |r|).
-__device__ __forceinline__ bool west_plus_zero(bool act, double qm, double q0, double q1) {
-  if (act || dbits(q0) < 0) return false;
+// Whether the reference's first term, C+*B of the west face qm | q0 | q1, is
+// +0 when it is a zero: C+ is +0 or positive, so its sign is that of the face
+// value B = q0 + X. If the + side is in use, t is that term. Otherwise C+ is
+// +0, X is a zero where q1 = q0, and |X| <= |q1-q0| + |q0-qm| for every limiter
+// (|psi(r)| <= 2 + |r|).
+__device__ __forceinline__ bool first_term_plus_zero(bool act, bool pos, double t, double qm, double q0, double q1) {
+  if (dbits(q0) == (long long)kSign) return false;  // -0 + X: the sign of X's zero matters
+  if (act && pos) return dbits(t) >= 0;
+  if (dbits(q0) < 0) return false;
   const double d = q1 - q0, n = q0 - qm;
   if (!nz(d)) return true;
-  return max(hi_word(d) & 0x7fffffffu, hi_word(n) & 0x7fffffffu) + (3u << 20) <= hi_word(q0);
+  return max(hi_mag(d), hi_mag(n)) + (3u << 20) <= hi_word(q0);
 }
 
 // The sum for the lane's cell: w its west face (whose east neighbour's is taken
@@ -703,7 +736,7 @@ __device__ __forceinline__ double sum_faces(const Side& w, const Side& so, const
   }
   const double S = ((w.t - te) + so.t) - n.t;
   slow = false;
-  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !west_plus_zero(act, qm, q0, q1);
+  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1);
   return S;
 }
 
@@ -725,9 +758,17 @@ __device__ __forceinline__ XN x_neighbours(double v, double aux, int lane) {
 }
 // The face west of the lane's column from its x neighbours: q0 = m1, q1 = v.
 template <int SCH, bool PAIR>
-__device__ __forceinline__ Face x_face(const Vel& vel, const XN& n, double v, unsigned long long dt) {
+__device__ __forceinline__ Face x_face(const Vel& vel, const XN& n, double v, unsigned long long dt, bool& bad) {
   const double n1 = pick(vel.pos, n.m1, n.p1) - pick(vel.pos, n.m2, v);
-  return make_face<SCH, PAIR>(vel, v - n.m1, n1, n.m1, v, n.p1, dt);
+  auto n2 = [&]() { return pick(vel.pos, n.p1, n.m1) - pick(vel.pos, v, n.m2); };
+  return make_face<SCH, PAIR>(vel, v - n.m1, n1, n2, n.m1, v, dt, bad);
+}
+// The face between rows with differences dm, d, d1 (below, across, above): q0 | q1.
+template <int SCH, bool PAIR>
+__device__ __forceinline__ Face y_face(const Vel& vel, double dm, double d, double d1, double q0, double q1,
+                                       unsigned long long dt, bool& bad) {
+  auto n2 = [&]() { return vel.pos ? d1 : dm; };
+  return make_face<SCH, PAIR>(vel, d, vel.pos ? dm : d1, n2, q0, q1, dt, bad);
 }
 
 // A strip is 31 columns x s.fk rows (chosen per launch, see fast_launch).
@@ -794,7 +835,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
     const Vel b = vel_one(vs);
     dm = h2 - h1;
     d0 = h3 - h2;
-    const Face F = make_face<SCH, false>(b, dm, b.pos ? h1 - h0 : d0, h1, h2, h3, dt);
+    const Face F = y_face<SCH, false>(b, h1 - h0, dm, d0, h1, h2, dt, bad);
     ts = side_of<false>(F, METRIC(DYN, j0));
   }
   for (int j = j0; j <= jn; j++) {
@@ -804,13 +845,13 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
     // x face west of column i, row j
     const double a = UF(iu, j);
     const XN xn = x_neighbours(h2, ha, lane);
-    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt);
+    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt, bad);
     const Side tw = side_of<false>(FX, METRIC(DXE, j));
     // y face north of row j: shared by this cell and the cell above
     const double vn = VF(ic, j);
     bad = bad || !in_range(a) || !in_range(vn);
     const Vel b = vel_one(vn);
-    const Face FY = make_face<SCH, false>(b, d0, b.pos ? dm : d1, h2, h3, h4, dt);
+    const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, METRIC(DYN, j));
     const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
     bool slow;
@@ -849,7 +890,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(De
     const Vel b = vel_one(vs);
     dm = h2 - h1;
     d0 = h3 - h2;
-    const Face F = make_face<SCH, false>(b, dm, b.pos ? h1 - h0 : d0, h1, h2, h3, dt);
+    const Face F = y_face<SCH, false>(b, h1 - h0, dm, d0, h1, h2, dt, bad);
     ts = side_of<false>(F, METRIC(DYN, j0));
   }
   for (int j = j0; j <= jn; j++) {
@@ -859,12 +900,12 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(De
     const double a = UF(iu, j);
     const Metric mx = METRIC(DXE, j), my = METRIC(DYN, j);
     const XN xn = x_neighbours(h2, ha, lane);
-    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt);
+    const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt, bad);
     const Side tw = side_of<false>(FX, mx);
     const double vn = VF(ic, j);
     bad = bad || !in_range(a) || !in_range(vn);
     const Vel b = vel_one(vn);
-    const Face FY = make_face<SCH, false>(b, d0, b.pos ? dm : d1, h2, h3, h4, dt);
+    const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, my);
     const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
     bool slow;
@@ -907,7 +948,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
     const Vel v = vel_pair(a, b, vs);
     dm = u2 - u1;
     d0 = u3 - u2;
-    const Face F = make_face<SCH, true>(v, dm, v.pos ? u1 - u0 : d0, u1, u2, u3, dt);
+    const Face F = y_face<SCH, true>(v, u1 - u0, dm, d0, u1, u2, dt, bad);
     ts = side_of<true>(F, METRIC(DYV, j0));
   }
   for (int j = j0; j <= jn; j++) {
@@ -916,14 +957,14 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
     bad = bad || !in_range(u4) || !in_range(ua);
     // x face west of column i, row j: velocities u(i-1), u(i)
     const XN xn = x_neighbours(u2, ua, lane);
-    const Face FX = x_face<SCH, true>(vel_pair(xn.m1, u2, xn.m1 + u2), xn, u2, dt);
+    const Face FX = x_face<SCH, true>(vel_pair(xn.m1, u2, xn.m1 + u2), xn, u2, dt, bad);
     const Side tw = side_of<true>(FX, METRIC(DXC, j));
     // y face north of row j: velocities v(i, j), v(i+1, j)
     const double va = VF(ic, j), vb = VF(ic1, j), vn = va + vb;
     bad = bad || !in_range(va);  // vb is the next lane's
     const Metric my = METRIC(DYV, j);
     const Vel v = vel_pair(va, vb, vn);
-    const Face FY = make_face<SCH, true>(v, d0, v.pos ? dm : d1, u2, u3, u4, dt);
+    const Face FY = y_face<SCH, true>(v, dm, d0, d1, u2, u3, dt, bad);
     const Side tn = side_of<true>(FY, my);
     const Side ns = side_of<true>(FY, METRIC(DYV, j + 1));
     bool slow;
@@ -967,7 +1008,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     const Vel v = vel_pair(v1, v2, v1 + v2);
     dm = v2 - v1;
     d0 = v3 - v2;
-    const Face F = make_face<SCH, true>(v, dm, v.pos ? v1 - v0 : d0, v1, v2, v3, dt);
+    const Face F = y_face<SCH, true>(v, v1 - v0, dm, d0, v1, v2, dt, bad);
     ts = side_of<true>(F, METRIC(DYC, j0));
   }
   for (int j = j0; j <= jn; j++) {
@@ -979,11 +1020,11 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     const Metric mx = METRIC(DXV, j);
     // x face west of column i, row j: velocities u(i-1, j+1), u(i-1, j)
     const XN xn = x_neighbours(v2, va, lane);
-    const Face FX = x_face<SCH, true>(vel_pair(uw1, uw0, uw), xn, v2, dt);
+    const Face FX = x_face<SCH, true>(vel_pair(uw1, uw0, uw), xn, v2, dt, bad);
     const Side tw = side_of<true>(FX, mx);
     // y face north of row j: velocities v(i, j), v(i, j+1)
     const Vel v = vel_pair(v2, v3, v2 + v3);
-    const Face FY = make_face<SCH, true>(v, d0, v.pos ? dm : d1, v2, v3, v4, dt);
+    const Face FY = y_face<SCH, true>(v, dm, d0, d1, v2, v3, dt, bad);
     const Side tn = side_of<true>(FY, METRIC(DYC, j));
     const Side ns = side_of<true>(FY, METRIC(DYC, j + 1));
     bool slow;

@@ -71,7 +71,7 @@ bool grid_ok(const sw2g_case* c);
 // Host geometry (geometry.cpp): fills rows[R_NUM*H]; returns the at-rest CFL
 // maxima used by compute_Dt when the flow is at rest (calc.c:715-725).
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my);
-// Whether Dt and every metric divisor of the rows lie in [2^-127, 2^129) (sigmath.cuh: in_window).
+// Whether Dt and every metric divisor of the rows lie in [2^-20, 2^60).
 bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows);
 // The fields of a polar cap (P_NUM x (nx+4)(ny+4)) and the at-rest CFL maxima
 // computed with them.
