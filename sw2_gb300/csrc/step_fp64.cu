@@ -425,7 +425,7 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 // the rest of its strip. Differences and sums of such values are zero or at
 // least 2^-902 (they are multiples of the smallest unit among them), so slope
 // ratios and Courant numbers are normal; products of several factors are
-// tested, and taken on the FP64 unit where they could be subnormal. The
+// tested (slope_term, two_products). The
 // skipped side is finite if its slope ratio is below 2^498 (then every
 // limiter, squares included, is), which a difference of at least 2^-397
 // ensures; below that the ratio's exponent is looked at (make_face).
@@ -538,16 +538,24 @@ __device__ __forceinline__ double mdiv(double a, const Metric& x) {
   return div_fp64(a, from_bits(x.b));
 }
 
-// (a*(b*2^k))/x of zero or in-range a and b (k20 = k << 20, k = 0 or -1: b*2^k
-// is exact). Where the product could be subnormal, on the FP64 unit.
-__device__ __noinline__ double product_over_fp64(double a, double b, double x) { return zdiv(a * b, x); }
+// (a*(b*2^kx))/X + (a*(c*2^ky))/Y of zero or in-range a, b, c (kx20 = kx << 20,
+// kx 0 or -1, and ky alike: the scalings are exact). Where a product could be
+// subnormal, on the FP64 unit, out of line.
+__device__ __forceinline__ double scaled(double b, unsigned k20) {
+  return nz(b) ? from_bits((unsigned long long)dbits(b) + ((unsigned long long)k20 << 32)) : b;
+}
+__device__ __noinline__ double two_products_fp64(double a, double b, double x, double c, double y) {
+  return zdiv(a * b, x) + zdiv(a * c, y);
+}
 __device__ __forceinline__ double product_over(double a, double b, unsigned k20, const Metric& x) {
-  if (!nz(a) || !nz(b)) return 0.0;
-  if (min(hi_mag(a), hi_mag(b)) >= HI_POW2(-450)) {
-    const unsigned long long q = sig_div_known(sig_mul(mag(a), mag(b), k20), x.b, x.y);
-    return from_bits(q | (sign_of(a) ^ sign_of(b)));
-  }
-  return product_over_fp64(a, from_bits((unsigned long long)dbits(b) + ((unsigned long long)k20 << 32)), from_bits(x.b));
+  const unsigned long long q = sig_div_known(sig_mul(mag(a), mag(b), k20), x.b, x.y);
+  return (nz(a) && nz(b)) ? from_bits(q | (sign_of(a) ^ sign_of(b))) : 0.0;
+}
+__device__ __forceinline__ double two_products(double a, double b, unsigned kx20, const Metric& X, double c,
+                                               unsigned ky20, const Metric& Y) {
+  if (min(hi_mag(a) - 1, min(hi_mag(b) - 1, hi_mag(c) - 1)) < HI_POW2(-450) - 1)  // zeros wrap
+    return two_products_fp64(a, scaled(b, kx20), from_bits(X.b), scaled(c, ky20), from_bits(Y.b));
+  return product_over(a, b, kx20, X) + product_over(a, c, ky20, Y);
 }
 
 // a/b on the integer pipe where both are usable (the quotient is then normal),
@@ -646,21 +654,20 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, N2 
 // integer pipe: k_adv_u at 2048x1024 0.146 ms with both products on the FP64
 // unit, 0.136 with one of them, 0.133 with none (the mass body 0.118, 0.109,
 // 0.101); c*B, whose B may be anything, stays there.
-__device__ __noinline__ double product3_fp64(double a, double b, double c) { return (a * b) * c; }
-__device__ __forceinline__ double slope_term(double hp, double g, double d) {
-  if (!nz(hp) || !nz(d)) return 0.0;
-  if (usable(hp) && usable(g) && hi_mag(d) >= HI_POW2(-700)) {
-    const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
-    return from_bits(sig_mul(sig_mul(mag(hp), mag(g)), mag(d)) | sg);
-  }
-  return product3_fp64(hp, g, d);
+// bad is set where the product or hp is not a normal number.
+__device__ __forceinline__ double slope_term(double hp, double g, double d, bool& bad) {
+  const unsigned eh = hi_mag(hp) >> 20, e = eh + (hi_mag(g) >> 20) + (hi_mag(d) >> 20);
+  const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
+  const bool zero = !nz(hp) || !nz(d);
+  bad = bad || (!zero && (eh - 1 >= 2046u || e - 2050 >= 2030u));
+  return zero ? 0.0 : from_bits(sig_mul(sig_mul(mag(hp), mag(g)), mag(d)) | sg);
 }
 // C*B of one side with c = |C|: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or
 // B2BM = q1 - psi*0.5*(1-c)*(q1-q0) (C- = -c; q1 - X = q1 + (-X) exactly).
 __device__ __forceinline__ double side_term(bool pos, unsigned long long p, const Metric& dx, double hp, double q0,
-                                            double q1, double d) {
+                                            double q1, double d, bool& bad) {
   const double c = from_bits(sig_div_known(p, dx.b, dx.y));
-  const double X = slope_term(hp, 1.0 - c, d);
+  const double X = slope_term(hp, 1.0 - c, d, bad);
   const unsigned long long neg = pos ? 0 : kSign;
   return flip(c * (pick(pos, q0, q1) + flip(X, neg)), neg);
 }
@@ -672,16 +679,18 @@ struct Side {
   bool pos, both;
 };
 template <bool PAIR>
-__device__ __forceinline__ Side side_of(const Face& F, const Metric& dx) {
+__device__ __forceinline__ Side side_of(const Face& F, const Metric& dx, bool& bad) {
   Side r;
-  const double t = side_term(F.pos, F.p, dx, F.hp, F.q0, F.q1, F.d);
+  bool far = false;  // says nothing of a face that is not in use
+  const double t = side_term(F.pos, F.p, dx, F.hp, F.q0, F.q1, F.d, far);
   r.t = F.act ? t : 0.0;
+  bad = bad || (F.act && far);
   r.m = 0.0;
   r.pos = F.pos;
   r.both = F.both;
   if constexpr (PAIR) {
     if (__any_sync(FULL, F.both)) {
-      if (F.both) r.m = side_term(false, F.p2, dx, F.hp2, F.q0, F.q1, F.d);
+      if (F.both) r.m = side_term(false, F.p2, dx, F.hp2, F.q0, F.q1, F.d, bad);
     }
   }
   return r;
@@ -836,7 +845,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
     dm = h2 - h1;
     d0 = h3 - h2;
     const Face F = y_face<SCH, false>(b, h1 - h0, dm, d0, h1, h2, dt, bad);
-    ts = side_of<false>(F, METRIC(DYN, j0));
+    ts = side_of<false>(F, METRIC(DYN, j0), bad);
   }
   for (int j = j0; j <= jn; j++) {
     const double h4 = HF(ic, j + 2), ha = HF(ia, j);
@@ -846,14 +855,14 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
     const double a = UF(iu, j);
     const XN xn = x_neighbours(h2, ha, lane);
     const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt, bad);
-    const Side tw = side_of<false>(FX, METRIC(DXE, j));
+    const Side tw = side_of<false>(FX, METRIC(DXE, j), bad);
     // y face north of row j: shared by this cell and the cell above
     const double vn = VF(ic, j);
     bad = bad || !in_range(a) || !in_range(vn);
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
-    const Side tn = side_of<false>(FY, METRIC(DYN, j));
-    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
+    const Side tn = side_of<false>(FY, METRIC(DYN, j), bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);  // calc.c:100 in its order: +w -e +s -n
     slow = __any_sync(FULL, bad) || slow;
@@ -891,7 +900,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(De
     dm = h2 - h1;
     d0 = h3 - h2;
     const Face F = y_face<SCH, false>(b, h1 - h0, dm, d0, h1, h2, dt, bad);
-    ts = side_of<false>(F, METRIC(DYN, j0));
+    ts = side_of<false>(F, METRIC(DYN, j0), bad);
   }
   for (int j = j0; j <= jn; j++) {
     const double h4 = f.tr[IX(W, ic, j + 2)], ha = f.tr[IX(W, ia, j)];
@@ -901,19 +910,19 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(De
     const Metric mx = METRIC(DXE, j), my = METRIC(DYN, j);
     const XN xn = x_neighbours(h2, ha, lane);
     const Face FX = x_face<SCH, false>(vel_one(a), xn, h2, dt, bad);
-    const Side tw = side_of<false>(FX, mx);
+    const Side tw = side_of<false>(FX, mx, bad);
     const double vn = VF(ic, j);
     bad = bad || !in_range(a) || !in_range(vn);
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
-    const Side tn = side_of<false>(FY, my);
-    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1));
+    const Side tn = side_of<false>(FY, my, bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);
     slow = __any_sync(FULL, bad) || slow;
     // Dt*TRACER*(UW(E)-UW(W))/DXE + Dt*TRACER*(VW(N)-VW(S))/DYN (calc.c:146-149)
     const double du = __shfl_sync(FULL, a, (lane + 1) & 31) - a, dv = vn - vs, tt = Dt * h2;
-    const double p2 = product_over(tt, du, 0, mx) + product_over(tt, dv, 0, my);
+    const double p2 = two_products(tt, du, 0, mx, dv, 0, my);
     if (own) {
       double r;
       if (slow) r = tracer_cell_ool<SCH>(s, f, i, j);
@@ -949,7 +958,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
     dm = u2 - u1;
     d0 = u3 - u2;
     const Face F = y_face<SCH, true>(v, u1 - u0, dm, d0, u1, u2, dt, bad);
-    ts = side_of<true>(F, METRIC(DYV, j0));
+    ts = side_of<true>(F, METRIC(DYV, j0), bad);
   }
   for (int j = j0; j <= jn; j++) {
     const double u4 = UF(ic, j + 2), ua = UF(ia, j);
@@ -958,22 +967,22 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
     // x face west of column i, row j: velocities u(i-1), u(i)
     const XN xn = x_neighbours(u2, ua, lane);
     const Face FX = x_face<SCH, true>(vel_pair(xn.m1, u2, xn.m1 + u2), xn, u2, dt, bad);
-    const Side tw = side_of<true>(FX, METRIC(DXC, j));
+    const Side tw = side_of<true>(FX, METRIC(DXC, j), bad);
     // y face north of row j: velocities v(i, j), v(i+1, j)
     const double va = VF(ic, j), vb = VF(ic1, j), vn = va + vb;
     bad = bad || !in_range(va);  // vb is the next lane's
     const Metric my = METRIC(DYV, j);
     const Vel v = vel_pair(va, vb, vn);
     const Face FY = y_face<SCH, true>(v, dm, d0, d1, u2, u3, dt, bad);
-    const Side tn = side_of<true>(FY, my);
-    const Side ns = side_of<true>(FY, METRIC(DYV, j + 1));
+    const Side tn = side_of<true>(FY, my, bad);
+    const Side ns = side_of<true>(FY, METRIC(DYV, j + 1), bad);
     bool slow;
     const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, u2, slow);
     slow = __any_sync(FULL, bad) || slow;
     // calc.c:198: u0*(uep-uwm)/(2 DXE) + u0*((vn0+vn1)/2 - (vs0+vs1)/2)/DYV; the
     // halving commutes with the difference (its operands are zero or at least 2^-352)
     const double ux = xn.p1 - xn.m1, vy = vn - vs;
-    const double p2 = Dt * (product_over(u2, ux, 0, METRIC(DXE2, j)) + product_over(u2, vy, 0xfff00000u, my));
+    const double p2 = Dt * two_products(u2, ux, 0, METRIC(DXE2, j), vy, 0xfff00000u, my);
     if (own) {
       double r;
       if (slow) r = advu_cell_ool<SCH>(s, f, i, j);
@@ -1009,7 +1018,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     dm = v2 - v1;
     d0 = v3 - v2;
     const Face F = y_face<SCH, true>(v, v1 - v0, dm, d0, v1, v2, dt, bad);
-    ts = side_of<true>(F, METRIC(DYC, j0));
+    ts = side_of<true>(F, METRIC(DYC, j0), bad);
   }
   for (int j = j0; j <= jn; j++) {
     const double v4 = VF(ic, j + 2), va = VF(ia, j);
@@ -1021,12 +1030,12 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     // x face west of column i, row j: velocities u(i-1, j+1), u(i-1, j)
     const XN xn = x_neighbours(v2, va, lane);
     const Face FX = x_face<SCH, true>(vel_pair(uw1, uw0, uw), xn, v2, dt, bad);
-    const Side tw = side_of<true>(FX, mx);
+    const Side tw = side_of<true>(FX, mx, bad);
     // y face north of row j: velocities v(i, j), v(i, j+1)
     const Vel v = vel_pair(v2, v3, v2 + v3);
     const Face FY = y_face<SCH, true>(v, dm, d0, d1, v2, v3, dt, bad);
-    const Side tn = side_of<true>(FY, METRIC(DYC, j));
-    const Side ns = side_of<true>(FY, METRIC(DYC, j + 1));
+    const Side tn = side_of<true>(FY, METRIC(DYC, j), bad);
+    const Side ns = side_of<true>(FY, METRIC(DYC, j + 1), bad);
     bool slow;
     const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, v2, slow);
     slow = __any_sync(FULL, bad) || slow;
@@ -1034,7 +1043,7 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     // sums of u symmetric in their operands
     const double ue = __shfl_sync(FULL, uw, (lane + 1) & 31);
     const double ux = ue - uw, vy = v3 - v1;
-    const double p2 = Dt * (product_over(v2, ux, 0xfff00000u, mx) + product_over(v2, vy, 0, METRIC(DYNS, j)));
+    const double p2 = Dt * two_products(v2, ux, 0xfff00000u, mx, vy, 0, METRIC(DYNS, j));
     if (own) {
       double r;
       if (slow) r = advv_cell_ool<SCH>(s, f, i, j);
