@@ -649,8 +649,7 @@ sw2g_status sw2g_create(const sw2g_case* c, int precision, int device, sw2g_ctx*
                       &b.deta[0], &b.deta[1], &b.deta[2], &b.du[0], &b.du[1], &b.du[2],
                       &b.dv[0], &b.dv[1], &b.dv[2], &b.dtr[0], &b.dtr[1], &b.dtr[2],
                       &b.detaAB, &b.duAB, &b.dvAB, &b.dtrAB, &b.duadv, &b.dvadv,
-                      &b.Le[0], &b.Le[1], &b.Le[2], &b.L[0], &b.L[1], &b.L[2], &b.L[3], &b.L[4], &b.L[5],
-                      &b.psi, &b.xi, &b.ze, &b.di};
+                      &b.Le[0], &b.Le[1], &b.Le[2], &b.L[0], &b.L[1], &b.L[2], &b.L[3], &b.L[4], &b.L[5]};
     for (double** p : all)
       if ((st = dalloc(x, p, S)) != SW2G_OK) return fail(st);
   } else {

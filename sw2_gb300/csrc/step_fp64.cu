@@ -22,10 +22,18 @@ namespace {
 constexpr int TX = 128;
 
 
+
 __device__ __forceinline__ int IX(int W, int i, int j) { return (i + 1) + (j + 1) * W; }
 __device__ __forceinline__ double RW(const DevState& s, int t, int j) { return s.rows[t * s.H + j + 1]; }
 // A field of a polar cap at padded index q.
 __device__ __forceinline__ double PF(const DevState& s, int t, int q) { return s.pf[(size_t)t * s.W * s.H + q]; }
+
+// Brings the line of a value that a later row reads into L1, without a
+// register to hold it: a load whose result nothing uses.
+__device__ __forceinline__ void touch(const double* p) {
+  double x;
+  asm volatile("ld.global.ca.f64 %0, [%1];" : "=d"(x) : "l"(p));
+}
 
 // The bit pattern of a double, through an opaque move: tests written on the
 // integer image (sign, exponent, zero) then stay integer operations; given
@@ -519,21 +527,31 @@ __device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j
 // the FP64 unit, out of line, otherwise. c: a factor that is finite and not
 // zero (a row constant or a coefficient): a zero times it is that zero.
 __device__ __forceinline__ bool mid(double x) { return ((hi_word(x) - 0x30000000u) & 0x60000000u) == 0; }
+// 2^-700 <= |x| < 2^257: times or over a factor of `mid` magnitude still normal
+__device__ __forceinline__ bool wide(double x) { return hi_mag(x) - HI_POW2(-700) < (957u << 20); }
 __device__ __noinline__ double mul_fp64(double a, double b) { return a * b; }
 __device__ __forceinline__ double smul(double a, double b) {
   if (mid(a) && mid(b)) return from_bits(sig_mul(mag(a), mag(b)) | ((unsigned long long)(dbits(a) ^ dbits(b)) & kSign));
   return mul_fp64(a, b);
 }
+// s.sig_ok says that the row constants and hyperviscosity coefficients are in
+// that range; k: such a factor.
+__device__ __forceinline__ double rmul(const DevState& s, double k, double a) {
+  const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(k)) & kSign;
+  if (wide(a) && s.sig_ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
+  if (!nz(a)) return from_bits(sg);
+  return mul_fp64(k, a);
+}
 __device__ __forceinline__ double cmul(double c, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(c)) & kSign;
-  if (mid(a) && mid(c)) return from_bits(sig_mul(mag(a), mag(c)) | sg);
+  if (wide(a) && mid(c)) return from_bits(sig_mul(mag(a), mag(c)) | sg);
   if (!nz(a)) return from_bits(sg);
   return mul_fp64(c, a);
 }
 __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
-// a / x.b (x.b > 0; s.sig_ok): a zero gives itself.
-__device__ __forceinline__ double mdiv(double a, const Metric& x) {
-  if (mid(a) && x.y) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
+// a / x.b (x.b > 0): a zero gives itself.
+__device__ __forceinline__ double mdiv(const DevState& s, double a, const Metric& x) {
+  if (wide(a) && s.sig_ok) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
   if (!nz(a)) return a;
   return div_fp64(a, from_bits(x.b));
 }
@@ -1211,12 +1229,9 @@ __global__ void k_add(DevState s, double* x, const double* dx) {
 //   wrap, it has no walls):
 //     LE (laplacian_eta, laplacian.c:131-146): rows ny+1, ny+2 <- row ny,
 //        row 0 <- row 1, row -1 <- row ny-1;
-//     ZE (laplacian.c:79): row 0 = 0, the other rows wrap;
-//     DI (laplacian.c:73): row ny+1 = the wall difference of u (written by
-//        the kernel), the other rows wrap;
 //     LU (laplacian.c:94-107): row ny+1 <- row ny, row 0 <- row 1, others wrap;
 //     LV: rows ny+1 and 0 = 0, others wrap.
-enum HaloKind { HK_WRAP, HK_LE, HK_ZE, HK_DI, HK_LU, HK_LV };
+enum HaloKind { HK_WRAP, HK_LE, HK_LU, HK_LV };
 constexpr int NOIMG = -1000000;
 template <int K>
 __device__ __forceinline__ void put_images(const DevState& s, double* f, int i, int j, double v) {
@@ -1245,17 +1260,6 @@ __device__ __forceinline__ void put_images(const DevState& s, double* f, int i, 
     }
     if (j == 1) f[IX(W, i, 0)] = v;
     if (j == ny - 1) f[IX(W, i, -1)] = v;
-  } else if (K == HK_ZE) {
-    if (j == ny - 1) f[IX(W, i, -1)] = v;
-    if (j == 1) {
-      f[IX(W, i, 0)] = 0.0;
-      f[IX(W, i, ny + 1)] = v;
-    }
-    if (j == 2) f[IX(W, i, ny + 2)] = v;
-  } else if (K == HK_DI) {
-    if (j == ny - 1) f[IX(W, i, -1)] = v;
-    if (j == ny) f[IX(W, i, 0)] = v;
-    if (j == 2) f[IX(W, i, ny + 2)] = v;
   } else if (K == HK_LU) {
     if (j == ny - 1) f[IX(W, i, -1)] = v;
     if (j == 1) f[IX(W, i, 0)] = v;
@@ -1269,27 +1273,55 @@ __device__ __forceinline__ void put_images(const DevState& s, double* f, int i, 
   }
 }
 
-// laplacian_eta first pass (laplacian.c:120-123)
-__global__ void k_lape_pass1(DevState s, const double* e, double* psi, double* xi) {
+// laplacian_eta (laplacian.c:114-127), both passes in one: a warp takes 31
+// columns and marches up `rows` rows; the psi west of a cell comes from the
+// lane before (one lane more than cells), the xi south of it from the row
+// before. psi and xi are zero on the halo (laplacian.c:116-118). In two
+// launches, psi and xi through memory: 0.045 ms a level at 2048x1024; fused
+// 0.036, and inside the eta kernel, which took 0.043 alone, 0.031.
+struct LapEta {
+  int c, cc;    // the lane's column, and the same kept inside the grid
+  bool own;     // the lane's cell is one of the strip's
+  double e0, xs;
+  // rows from j0 on
+  __device__ __forceinline__ bool begin(const DevState& s, const double* e, int j0) {
+    const int W = s.W, lane = threadIdx.x & 31;
+    const int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * FW + 1;
+    c = base - 1 + lane;
+    cc = min(c, s.nx);
+    own = lane > 0 && c <= s.nx;
+    if (base > s.nx) return false;
+    e0 = e[IX(W, cc, j0)];
+    xs = 0.0;
+    if (j0 > 1) xs = mdiv(s, rmul(s, RW(s, R_KY, j0 - 1), e0 - e[IX(W, cc, j0 - 1)]), METRIC(DYC, j0 - 1));
+    return true;
+  }
+  // the value at row j (warp-wide)
+  __device__ __forceinline__ double next(const DevState& s, const double* e, int j) {
+    const int W = s.W;
+    touch(e + IX(W, cc, min(j + 2, s.ny + 1)));
+    const double ee = e[IX(W, cc + 1, j)], en = e[IX(W, cc, j + 1)];
+    double psi = mdiv(s, rmul(s, RW(s, R_KX, j), ee - e0), METRIC(DXC, j));
+    if (c == 0) psi = 0.0;
+    const double pw = __shfl_up_sync(FULL, psi, 1);
+    const double xi = mdiv(s, rmul(s, RW(s, R_KY, j), en - e0), METRIC(DYC, j));
+    const double v = rmul(s, RW(s, R_KC, j), mdiv(s, psi - pw, METRIC(DXE, j)) + mdiv(s, xi - xs, METRIC(DYN, j)));
+    e0 = en;
+    xs = xi;
+    return v;
+  }
+};
+// One level, with its halo update and wall rows (laplacian.c:129-146).
+__global__ void __launch_bounds__(TX, 16) k_lape(DevState s, const double* e, double* eo, int rows) {
   SW2G_PDL_ENTRY();
-  INTERIOR_IJ
-  const int q = IX(W, i, j);
-  psi[q] = mdiv(cmul(RW(s, R_KX, j), e[IX(W, i + 1, j)] - e[q]), METRIC(DXC, j));
-  xi[q] = mdiv(cmul(RW(s, R_KY, j), e[IX(W, i, j + 1)] - e[q]), METRIC(DYC, j));
+  const int j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, s.ny);
+  LapEta L;
+  if (!L.begin(s, e, j0)) return;
+  for (int j = j0; j <= jn; j++) {
+    const double v = L.next(s, e, j);
+    if (L.own) put_images<HK_LE>(s, eo, L.c, j, v);
+  }
 }
-
-// laplacian_eta second pass (laplacian.c:125-127)
-// (with its halo update and wall rows written from here, laplacian.c:129-146)
-__global__ void k_lape_pass2(DevState s, const double* psi, const double* xi, double* eo) {
-  SW2G_PDL_ENTRY();
-  INTERIOR_IJ
-  const int q = IX(W, i, j);
-  const double v =
-      cmul(RW(s, R_KC, j), mdiv(psi[q] - psi[IX(W, i - 1, j)], METRIC(DXE, j)) +
-                              mdiv(xi[q] - xi[IX(W, i, j - 1)], METRIC(DYN, j)));
-  put_images<HK_LE>(s, eo, i, j, v);
-}
-
 
 // Deta_n += nu*Dt*L (calc.c:346-350); Du/Dv the same (core.c:258-266), with
 // nu*Dt formed once on the host by the same multiplication. A term whose nu
@@ -1308,21 +1340,27 @@ __device__ __noinline__ double add_product(double x, double nd, double v) { retu
 // NZ = 8: no hyperviscosity block at all (every nu zero: the reference skips it).
 constexpr int kNoHyper = 8;
 template <int NZ>
-__device__ __forceinline__ double hyper_terms(const DevState& s, double x, const double* l2, const double* l4,
-                                              const double* l6, int q) {
+__device__ __forceinline__ double hyper_terms(const DevState& s, double x, double v2, double v4, double v6) {
   if constexpr (NZ == kNoHyper) {
     return x;
   } else {
-    const double V[3] = {l2[q], l4[q], l6[q]};  // all loads issued before any branch
+    const double V[3] = {v2, v4, v6};
     const double nd[3] = {s.nu2dt, s.nu4dt, s.nu6dt};
 #pragma unroll
     for (int t = 0; t < 3; t++) {
       const double v = V[t];
-      if ((NZ >> t) & 1) x = x + cmul(nd[t], v);
+      if ((NZ >> t) & 1) x = x + rmul(s, nd[t], v);
       else if (!zero_term_is_exact(x, v)) x = add_product(x, nd[t], v);
     }
     return x;
   }
+}
+// The levels of Laplacian that run (calc.c:332-345); the others stay zero.
+template <int NZ>
+constexpr int kLevels = NZ == kNoHyper ? 0 : (NZ & 4) ? 3 : (NZ & 2) ? 2 : 1;
+template <int NZ>
+__device__ __forceinline__ double level(const double* l, int t, int q) {
+  return t < kLevels<NZ> ? l[q] : 0.0;
 }
 
 template <int NZ>
@@ -1330,13 +1368,13 @@ __global__ void k_hyper_add(DevState s, double* d, const double* l2, const doubl
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  d[q] = hyper_terms<NZ>(s, d[q], l2, l4, l6, q);
+  d[q] = hyper_terms<NZ>(s, d[q], l2[q], l4[q], l6[q]);
 }
 
 // The coefficient mask of the hyperviscosity terms (kNoHyper when every nu is zero).
 int hyper_mask(const DevState& s) {
   if (s.nu2 == 0 && s.nu4 == 0 && s.nu6 == 0) return kNoHyper;
-  return (s.nu2dt != 0.0 ? 1 : 0) | (s.nu4dt != 0.0 ? 2 : 0) | (s.nu6dt != 0.0 ? 4 : 0);
+  return (s.nu2 != 0 ? 1 : 0) | (s.nu4 != 0 ? 2 : 0) | (s.nu6 != 0 ? 4 : 0);
 }
 
 void hyper_add(const DevState& s, dim3 g, cudaStream_t st, double* d, const double* l2, const double* l4,
@@ -1368,78 +1406,118 @@ __device__ __noinline__ double minus_damping(double x, double U, double sigma, d
 
 // UD (a band with sigma = 0): the dissipation terms are zeros, subtracted
 // only where the sum is zero or an operand is not finite.
+// The new tendency of u (v): advection + pressure - damping.
+template <bool UD>
+__device__ __forceinline__ double u_tendency(const DevState& s, const double* e, double duadv, double U, int i, int j) {
+  const int W = s.W, q = IX(W, i, j);
+  const double mge = s.polar ? -PF(s, P_GE, q) * s.Dt : RW(s, R_MGEDT, j);  // -GE*Dt, calc.c:517
+  const double a = duadv + mdiv(s, cmul(mge, e[IX(W, i + 1, j)] - e[q]), METRIC(DXC, j));
+  if constexpr (UD) return zero_term_is_exact(a, U) ? a : minus_damping(a, U, s.sigma, s.Dt);
+  return a - U * (s.polar ? PF(s, P_SU, q) : s.sigma) * s.Dt;  // calc.c:374-394
+}
+template <bool UD>
+__device__ __forceinline__ double v_tendency(const DevState& s, const double* e, double dvadv, double V, int i, int j) {
+  const int W = s.W, q = IX(W, i, j);
+  const double mgn = s.polar ? -PF(s, P_GN, q) * s.Dt : RW(s, R_MGNDT, j);  // calc.c:538
+  const double a = dvadv + mdiv(s, cmul(mgn, e[IX(W, i, j + 1)] - e[q]), METRIC(DYC, j + 1));
+  if constexpr (UD) return zero_term_is_exact(a, V) ? a : minus_damping(a, V, s.sigma, s.Dt);
+  return a - V * (s.polar ? PF(s, P_SV, q) : s.sigma) * s.Dt;
+}
 template <bool UD>
 __global__ void k_pres_sum(DevState s, F7 f, const double* duadv, const double* dvadv, double* dun, double* dvn) {
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  const double* e = f.eta;
-  const double mge = s.polar ? -PF(s, P_GE, q) * s.Dt : RW(s, R_MGEDT, j);  // -GE*Dt, calc.c:517
-  const double mgn = s.polar ? -PF(s, P_GN, q) * s.Dt : RW(s, R_MGNDT, j);
-  const double dup = mdiv(cmul(mge, e[IX(W, i + 1, j)] - e[q]), METRIC(DXC, j));
-  const double dvp = mdiv(cmul(mgn, e[IX(W, i, j + 1)] - e[q]), METRIC(DYC, j + 1));
-  double a = duadv[q] + dup;
-  double b = dvadv[q] + dvp;
-  if constexpr (UD) {
-    const double U = f.u[q], V = f.v[q];
-    if (!zero_term_is_exact(a, U)) a = minus_damping(a, U, s.sigma, s.Dt);
-    if (!zero_term_is_exact(b, V)) b = minus_damping(b, V, s.sigma, s.Dt);
-  } else {
-    const double su = s.polar ? PF(s, P_SU, q) : s.sigma, sv = s.polar ? PF(s, P_SV, q) : s.sigma;  // calc.c:374-394
-    a = a - f.u[q] * su * s.Dt;
-    b = b - f.v[q] * sv * s.Dt;
-  }
-  dun[q] = a;
-  dvn[q] = b;
+  dun[q] = u_tendency<UD>(s, f.eta, duadv[q], f.u[q], i, j);
+  dvn[q] = v_tendency<UD>(s, f.eta, dvadv[q], f.v[q], i, j);
 }
 
-// laplacian_vels first pass (laplacian.c:59-65)
-// (with the halo update and wall fixes of ze and di written from here,
-// laplacian.c:67-81). A thread marches down LV_ROWS rows of its column, so
-// the products DXC(j+1)*u(i,j+1) and DXV(j)*v(i,j) of one row are the
-// DXC(j)*u(i,j) and DXV(j-1)*v(i,j-1) of the next: the same operands and the
-// same products, formed once. Four rows (measured against 2, 8 and 16 at
-// 2048x1024) keep enough threads in flight for the integer-pipe additions.
-constexpr int LV_ROWS = 4;
-__global__ void k_lapv_pass1(DevState s, const double* uu, const double* vv, double* ze, double* di) {
+// laplacian_vels (laplacian.c:51-111), both passes in one: a warp takes 30
+// columns (its first and last lane give the ze west and the di east of the
+// others) and marches up `rows` rows, carrying ze and di and the products
+// DXC*u and DXV*v from row to row (the same operands, formed once). The
+// reference wraps ze and di in x and fixes their wall rows (laplacian.c:67-81):
+// the values of columns 0 and nx+1 are those of columns nx and 1, evaluated
+// there; ze is zero in row 0 and di in row ny+1 the wall difference of u, or
+// on a polar cap, which has no walls, those of rows ny and 1. `images`: with
+// the halo update and wall fixes of lu and lv (laplacian.c:91-107), which the
+// next level reads. Bound by the FP64 unit (13 additions a cell, 70 % busy) and
+// the issue slots. In two launches, ze and di through memory: 0.075 ms a level
+// at 2048x1024; fused 0.072, and one launch less on small grids. Resident
+// blocks 5 (117 registers), 8, 9 and 10: 0.089, 0.071, 0.072, 0.075 (at
+// 4096x2048 0.324, 0.243, 0.237, 0.235).
+constexpr int LVW = 30;
+__global__ void __launch_bounds__(TX, 9) k_lapv(DevState s, const double* uu, const double* vv, double* lu, double* lv,
+                                             int rows, bool images) {
   SW2G_PDL_ENTRY();
-  const int W = s.W;
-  const int i = blockIdx.x * TX + threadIdx.x + 1;
-  const int j0 = blockIdx.y * LV_ROWS + 1;
-  if (i > s.nx) return;
-  const int j1 = min(j0 + LV_ROWS - 1, s.ny);
-  double pu = cmul(RW(s, R_DXC, j0), uu[IX(W, i, j0)]);
-  double qv = cmul(RW(s, R_DXV, j0 - 1), vv[IX(W, i, j0 - 1)]);
-  for (int j = j0; j <= j1; j++) {
-    const int q = IX(W, i, j);
-    const double pu1 = cmul(RW(s, R_DXC, j + 1), uu[IX(W, i, j + 1)]);
-    const double qv1 = cmul(RW(s, R_DXV, j), vv[q]);
-    // x + (-b)*y is x - b*y
-    const double z = cmul(RW(s, R_IDXV, j), (vv[IX(W, i + 1, j)] - vv[q]) - cmul(RW(s, R_IDYC, j + 1), pu1 - pu));
-    const double d = cmul(RW(s, R_IDXE, j), (uu[q] - uu[IX(W, i - 1, j)]) + cmul(RW(s, R_IDYN, j), qv1 - qv));
-    put_images<HK_ZE>(s, ze, i, j, z);
-    put_images<HK_DI>(s, di, i, j, d);
-    if (j == s.ny && s.polar == 0)  // laplacian.c:73
-      di[IX(W, i, s.ny + 1)] = (uu[IX(W, i, s.ny)] - uu[IX(W, i - 1, s.ny)]) / RW(s, R_DXE, s.ny);
+  const int W = s.W, nx = s.nx, ny = s.ny, lane = threadIdx.x & 31;
+  const int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * LVW + 1;
+  if (base > nx) return;
+  const int j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, ny);
+  const int c = base - 1 + lane;
+  const int sc = c == 0 ? nx : (c <= nx ? c : 1);  // where the column's ze and di are evaluated
+  const bool own = lane > 0 && lane <= LVW && c <= nx;
+  // ze and di at row j of the column, the products of u (rows j, j+1) and v (rows j-1, j) given
+  auto zeta = [&](int j, double v0, double ve, double pu, double pu1) {
+    return rmul(s, RW(s, R_IDXV, j), (ve - v0) - rmul(s, RW(s, R_IDYC, j + 1), pu1 - pu));
+  };
+  auto divg = [&](int j, double u0, double uw, double qs, double qv) {
+    return rmul(s, RW(s, R_IDXE, j), (u0 - uw) + rmul(s, RW(s, R_IDYN, j), qv - qs));
+  };
+  auto PU = [&](int j, double u) { return rmul(s, RW(s, R_DXC, j), u); };
+  auto QV = [&](int j, double v) { return rmul(s, RW(s, R_DXV, j), v); };
+  auto u_at = [&](int i, int j) { return uu[IX(W, i, j)]; };
+  auto v_at = [&](int i, int j) { return vv[IX(W, i, j)]; };
+  double u0 = u_at(sc, j0), v0 = v_at(sc, j0);
+  double pu = PU(j0, u0), qv = QV(j0, v0);
+  double d = divg(j0, u0, u_at(sc - 1, j0), QV(j0 - 1, v_at(sc, j0 - 1)), qv);
+  double zs = 0.0;
+  if (j0 > 1) {
+    zs = zeta(j0 - 1, v_at(sc, j0 - 1), v_at(sc + 1, j0 - 1), PU(j0 - 1, u_at(sc, j0 - 1)), pu);
+  } else if (s.polar != 0) {
+    zs = zeta(ny, v_at(sc, ny), v_at(sc + 1, ny), PU(ny, u_at(sc, ny)), PU(ny + 1, u_at(sc, ny + 1)));
+  }
+  for (int j = j0; j <= jn; j++) {
+    // the next row's values, a row ahead (0.078 -> 0.070 ms; held in registers,
+    // with fewer warps resident, 0.078)
+    const int jp = min(j + 2, ny + 1);
+    touch(uu + IX(W, sc, jp));
+    touch(uu + IX(W, sc - 1, jp));
+    touch(vv + IX(W, sc, jp));
+    touch(vv + IX(W, sc + 1, j + 1));
+    const double u1 = u_at(sc, j + 1), v1 = v_at(sc, j + 1);
+    const double pu1 = PU(j + 1, u1);
+    const double z = zeta(j, v0, v_at(sc + 1, j), pu, pu1);
+    double qv1 = 0.0, dn;
+    if (j < ny) {
+      qv1 = QV(j + 1, v1);
+      dn = divg(j + 1, u1, u_at(sc - 1, j + 1), qv, qv1);
+    } else if (s.polar == 0) {  // laplacian.c:73
+      dn = mdiv(s, u0 - u_at(sc - 1, ny), METRIC(DXE, ny));
+    } else {
+      dn = divg(1, u_at(sc, 1), u_at(sc - 1, 1), QV(0, v_at(sc, 0)), QV(1, v_at(sc, 1)));
+    }
+    const double zw = __shfl_up_sync(FULL, z, 1), de = __shfl_down_sync(FULL, d, 1);
+    // (-a)*x + b*y = b*y - a*x
+    const double xu = rmul(s, RW(s, R_IDXC, j), de - d) - rmul(s, RW(s, R_IDYN, j), z - zs);
+    const double xv = rmul(s, RW(s, R_IDXV, j), z - zw) + rmul(s, RW(s, R_IDYC, j + 1), dn - d);
+    if (own) {
+      if (images) {
+        put_images<HK_LU>(s, lu, c, j, xu);
+        put_images<HK_LV>(s, lv, c, j, xv);
+      } else {
+        lu[IX(W, c, j)] = xu;
+        lv[IX(W, c, j)] = xv;
+      }
+    }
+    u0 = u1;
+    v0 = v1;
     pu = pu1;
     qv = qv1;
+    d = dn;
+    zs = z;
   }
 }
-
-// laplacian_vels second pass (laplacian.c:83-89)
-// (with the halo update and wall fixes of lu and lv written from here, laplacian.c:91-107)
-__global__ void k_lapv_pass2(DevState s, const double* ze, const double* di, double* lu, double* lv) {
-  SW2G_PDL_ENTRY();
-  INTERIOR_IJ
-  const int q = IX(W, i, j);
-  const double z = ze[q], d = di[q];
-  // (-a)*x + b*y = b*y - a*x
-  const double vu = cmul(RW(s, R_IDXC, j), di[IX(W, i + 1, j)] - d) - cmul(RW(s, R_IDYN, j), z - ze[IX(W, i, j - 1)]);
-  const double vl = cmul(RW(s, R_IDXV, j), z - ze[IX(W, i - 1, j)]) + cmul(RW(s, R_IDYC, j + 1), di[IX(W, i, j + 1)] - d);
-  put_images<HK_LU>(s, lu, i, j, vu);
-  put_images<HK_LV>(s, lv, i, j, vl);
-}
-
 
 // solve_Coriolis_u (calc.c:542-569), in place
 __global__ void k_coriolis_u(DevState s, double* u, const double* v, const double* duab) {
@@ -1495,13 +1573,14 @@ __device__ __forceinline__ void check_range(int* bad, double x, int i, int j) {
   if (bad && range_bad(x, i == 1 && j == 1)) atomicOr(bad, 1);
 }
 
+// The new eta of a cell (calc.c:403-422, core.c:203-210), given the tendency's
+// hyperviscosity values.
 template <int NZ, bool PL>
-__global__ void k_eta_ab3(DevState s, F7 f, double* eta, double* dn, const double* dm1, const double* dm2,
-                          const double* l2, const double* l4, const double* l6, int* bad) {
-  SW2G_PDL_ENTRY();
-  INTERIOR_IJ
-  const int q = IX(W, i, j);
-  const double x = hyper_terms<NZ>(s, dn[q], l2, l4, l6, q);
+__device__ __forceinline__ void eta_ab3_cell(const DevState& s, const F7& f, double* eta, double* dn,
+                                             const double* dm1, const double* dm2, double v2, double v4, double v6,
+                                             int* bad, int i, int j) {
+  const int W = s.W, q = IX(W, i, j);
+  const double x = hyper_terms<NZ>(s, dn[q], v2, v4, v6);
   if constexpr (NZ != kNoHyper) dn[q] = x;
   double ab = ab3(x, dm1[q], dm2[q]);
   const double e = f.eta[q];
@@ -1515,41 +1594,71 @@ __global__ void k_eta_ab3(DevState s, F7 f, double* eta, double* dn, const doubl
   put_images<HK_WRAP>(s, eta, i, j, en);  // with eta's halo update (core.c:206-210)
   check_range(bad, en, i, j);
 }
-
-template <int NZ>
-__global__ void k_coriolis_u_ab3(DevState s, double* u, const double* v, double* dn, const double* dm1,
-                                 const double* dm2, const double* l2, const double* l4, const double* l6,
-                                 int* bad) {
+template <int NZ, bool PL>
+__global__ void k_eta_ab3(DevState s, F7 f, double* eta, double* dn, const double* dm1, const double* dm2,
+                          const double* l2, const double* l4, const double* l6, int* bad) {
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  const double x = hyper_terms<NZ>(s, dn[q], l2, l4, l6, q);
-  if constexpr (NZ != kNoHyper) dn[q] = x;
-  const double duab = ab3(x, dm1[q], dm2[q]);
+  eta_ab3_cell<NZ, PL>(s, f, eta, dn, dm1, dm2, level<NZ>(l2, 0, q), level<NZ>(l4, 1, q), level<NZ>(l6, 2, q), bad,
+                       i, j);
+}
+// The same with the last level of laplacian_eta (of the field e), which only
+// the cell itself reads: neither it nor its halo goes through memory.
+template <int NZ, bool PL>
+__global__ void __launch_bounds__(TX, 16) k_eta_lap_ab3(DevState s, F7 f, double* eta, double* dn, const double* dm1,
+                                                    const double* dm2, const double* l2, const double* l4,
+                                                    const double* e, int* bad, int rows) {
+  SW2G_PDL_ENTRY();
+  constexpr int last = kLevels<NZ> - 1;
+  const int W = s.W, j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, s.ny);
+  LapEta L;
+  if (!L.begin(s, e, j0)) return;
+  for (int j = j0; j <= jn; j++) {
+    const double v = L.next(s, e, j);
+    if (!L.own) continue;
+    const int q = IX(W, L.c, j);
+    const double v2 = last == 0 ? v : l2[q], v4 = last == 1 ? v : level<NZ>(l4, 1, q), v6 = last == 2 ? v : 0.0;
+    eta_ab3_cell<NZ, PL>(s, f, eta, dn, dm1, dm2, v2, v4, v6, bad, L.c, j);
+  }
+}
+
+template <int NZ, bool UD>
+__global__ void __launch_bounds__(TX, 16) k_coriolis_u_ab3(DevState s, double* u, const double* v, const double* eta, const double* duadv,
+                                 double* dn, const double* dm1, const double* dm2, const double* l2,
+                                 const double* l4, const double* l6, int* bad) {
+  SW2G_PDL_ENTRY();
+  INTERIOR_IJ
+  const int q = IX(W, i, j);
   const double u0 = u[q];
+  const double x = hyper_terms<NZ>(s, u_tendency<UD>(s, eta, duadv[q], u0, i, j), level<NZ>(l2, 0, q),
+                                   level<NZ>(l4, 1, q), level<NZ>(l6, 2, q));
+  dn[q] = x;
+  const double duab = ab3(x, dm1[q], dm2[q]);
   const double semi = QUARTER(v[IX(W, i, j)] + v[IX(W, i + 1, j)] + v[IX(W, i, j - 1)] + v[IX(W, i + 1, j - 1)]);
   const double dtf = s.polar ? s.Dt * PF(s, P_FE, q) : RW(s, R_DTFE, j);
-  const double al = dtf + mdiv(cmul(s.Dt, u0) * RW(s, R_SINC, j), METRIC(RZC, j));
+  const double al = dtf + mdiv(s, cmul(s.Dt, u0) * RW(s, R_SINC, j), METRIC(RZC, j));
   const double be = smul(QUARTER(al), al);
   const double un = quotient(((u0 + duab) - smul(be, u0)) + smul(al, semi), 1.0 + be);
   u[q] = un;
   check_range(bad, un, i, j);
 }
 
-template <int NZ>
-__global__ void k_coriolis_v_ab3(DevState s, const double* u, double* v, double* dn, const double* dm1,
-                                 const double* dm2, const double* l2, const double* l4, const double* l6,
-                                 int* bad) {
+template <int NZ, bool UD>
+__global__ void __launch_bounds__(TX, 16) k_coriolis_v_ab3(DevState s, const double* u, double* v, const double* eta, const double* dvadv,
+                                 double* dn, const double* dm1, const double* dm2, const double* l2,
+                                 const double* l4, const double* l6, int* bad) {
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
-  const double x = hyper_terms<NZ>(s, dn[q], l2, l4, l6, q);
-  if constexpr (NZ != kNoHyper) dn[q] = x;
-  const double dvab = ab3(x, dm1[q], dm2[q]);
   const double v0 = v[q];
+  const double x = hyper_terms<NZ>(s, v_tendency<UD>(s, eta, dvadv[q], v0, i, j), level<NZ>(l2, 0, q),
+                                   level<NZ>(l4, 1, q), level<NZ>(l6, 2, q));
+  dn[q] = x;
+  const double dvab = ab3(x, dm1[q], dm2[q]);
   const double semi = QUARTER(u[IX(W, i - 1, j + 1)] + u[IX(W, i, j + 1)] + u[IX(W, i, j)] + u[IX(W, i - 1, j)]);
   const double dtf = s.polar ? s.Dt * PF(s, P_FN, q) : RW(s, R_DTFN, j);
-  const double al = dtf + mdiv(cmul(s.Dt, semi) * RW(s, R_SINN, j), METRIC(RZN, j));
+  const double al = dtf + mdiv(s, cmul(s.Dt, semi) * RW(s, R_SINN, j), METRIC(RZN, j));
   const double be = smul(QUARTER(al), al);
   const double vn = quotient(((v0 + dvab) - smul(be, v0)) - smul(al, semi), 1.0 + be);
   v[q] = vn;
@@ -1558,36 +1667,63 @@ __global__ void k_coriolis_v_ab3(DevState s, const double* u, double* v, double*
   if (s.polar != 0 || j != s.ny) check_range(bad, vn, i, j);
 }
 
+// Launch shape of the kernels that march: `width` columns per warp, and as
+// many rows (a power of two up to `rows`) as still leave 24 warps for each SM,
+// so that small grids spread over the chip. k_lapv takes up to 8 rows, the
+// eta kernels 4: at 2048x1024 with 4, 8 and 16 rows k_lapv 0.073, 0.071 and
+// 0.073 ms, k_lape 0.037, 0.038 and 0.043, k_eta_lap_ab3 0.077, 0.085, 0.092.
+struct March {
+  dim3 grid;
+  int rows;
+};
+March march(const DevState& s, int width, int rows) {
+  const int bx = (s.nx + width * (TX / 32) - 1) / (width * (TX / 32));
+  while (rows > 1 && (long long)bx * (TX / 32) * ((s.ny + rows - 1) / rows) < 152 * 24) rows /= 2;
+  return March{dim3(bx, (s.ny + rows - 1) / rows), rows};
+}
+
+// which: 0 eta (hyper + AB3 + geofactor + update), 1 u, 2 v (pressure, damping,
+// hyper + AB3 + Coriolis); bad: the step's range flag when the range check is
+// done here, else null; last_src: the field whose laplacian_eta is the last
+// level, computed by the eta kernel, or null if that level is in Le already
 template <int NZ>
-void fused_tails(const DevState& s, dim3 g, cudaStream_t st, const F7& f, Fp64Buffers& b, int which, int* bad) {
+void fused_tails(const DevState& s, dim3 g, cudaStream_t st, const F7& f, Fp64Buffers& b, int which, int* bad,
+                 const double* last_src) {
+  const bool ud = s.polar == 0 && s.sigma == 0.0;
   if (which == 0) {
-    if (s.plain)
-      pdl_launch(k_eta_ab3<NZ, true>, dim3(g), dim3(TX), st, s, f, b.f[0], b.deta[0], b.deta[1], b.deta[2], b.Le[0], b.Le[1], b.Le[2],
-                                            bad);
-    else
-      pdl_launch(k_eta_ab3<NZ, false>, dim3(g), dim3(TX), st, s, f, b.f[0], b.deta[0], b.deta[1], b.deta[2], b.Le[0], b.Le[1],
-                                             b.Le[2], bad);
+    if constexpr (NZ != kNoHyper) {
+      if (last_src) {
+        const March m = march(s, FW, 4);
+        auto k = s.plain ? k_eta_lap_ab3<NZ, true> : k_eta_lap_ab3<NZ, false>;
+        pdl_launch(k, m.grid, dim3(TX), st, s, f, b.f[0], b.deta[0], b.deta[1], b.deta[2], b.Le[0], b.Le[1], last_src,
+                   bad, m.rows);
+        return;
+      }
+    }
+    auto k = s.plain ? k_eta_ab3<NZ, true> : k_eta_ab3<NZ, false>;
+    pdl_launch(k, g, dim3(TX), st, s, f, b.f[0], b.deta[0], b.deta[1], b.deta[2], b.Le[0], b.Le[1], b.Le[2], bad);
   } else if (which == 1) {
-    pdl_launch(k_coriolis_u_ab3<NZ>, dim3(g), dim3(TX), st, s, b.f[1], b.f[2], b.du[0], b.du[1], b.du[2], b.L[0], b.L[2], b.L[4],
-                                           bad);
+    auto k = ud ? k_coriolis_u_ab3<NZ, true> : k_coriolis_u_ab3<NZ, false>;
+    pdl_launch(k, g, dim3(TX), st, s, b.f[1], b.f[2], b.f[0], b.duadv, b.du[0], b.du[1], b.du[2], b.L[0], b.L[2],
+               b.L[4], bad);
   } else {
-    pdl_launch(k_coriolis_v_ab3<NZ>, dim3(g), dim3(TX), st, s, b.f[1], b.f[2], b.dv[0], b.dv[1], b.dv[2], b.L[1], b.L[3], b.L[5],
-                                           bad);
+    auto k = ud ? k_coriolis_v_ab3<NZ, true> : k_coriolis_v_ab3<NZ, false>;
+    pdl_launch(k, g, dim3(TX), st, s, b.f[1], b.f[2], b.f[0], b.dvadv, b.dv[0], b.dv[1], b.dv[2], b.L[1], b.L[3],
+               b.L[5], bad);
   }
 }
-// which: 0 eta (hyper + AB3 + geofactor + update), 1 u, 2 v (hyper + AB3 + Coriolis);
-// bad: the step's range flag when the range check is done here, else null
-void fused_tail(const DevState& s, dim3 g, cudaStream_t st, const F7& f, Fp64Buffers& b, int which, int* bad) {
+void fused_tail(const DevState& s, dim3 g, cudaStream_t st, const F7& f, Fp64Buffers& b, int which, int* bad,
+                const double* last_src = nullptr) {
   switch (hyper_mask(s)) {
-    case 0: fused_tails<0>(s, g, st, f, b, which, bad); break;
-    case 1: fused_tails<1>(s, g, st, f, b, which, bad); break;
-    case 2: fused_tails<2>(s, g, st, f, b, which, bad); break;
-    case 3: fused_tails<3>(s, g, st, f, b, which, bad); break;
-    case 4: fused_tails<4>(s, g, st, f, b, which, bad); break;
-    case 5: fused_tails<5>(s, g, st, f, b, which, bad); break;
-    case 6: fused_tails<6>(s, g, st, f, b, which, bad); break;
-    case 7: fused_tails<7>(s, g, st, f, b, which, bad); break;
-    default: fused_tails<kNoHyper>(s, g, st, f, b, which, bad); break;
+    case 0: fused_tails<0>(s, g, st, f, b, which, bad, last_src); break;
+    case 1: fused_tails<1>(s, g, st, f, b, which, bad, last_src); break;
+    case 2: fused_tails<2>(s, g, st, f, b, which, bad, last_src); break;
+    case 3: fused_tails<3>(s, g, st, f, b, which, bad, last_src); break;
+    case 4: fused_tails<4>(s, g, st, f, b, which, bad, last_src); break;
+    case 5: fused_tails<5>(s, g, st, f, b, which, bad, last_src); break;
+    case 6: fused_tails<6>(s, g, st, f, b, which, bad, last_src); break;
+    case 7: fused_tails<7>(s, g, st, f, b, which, bad, last_src); break;
+    default: fused_tails<kNoHyper>(s, g, st, f, b, which, bad, last_src); break;
   }
 }
 
@@ -1631,6 +1767,57 @@ __global__ void k_channel(int nx, int ny, double* u, double* v, double* wx, doub
   wy[IX(W, i, ny)] = 0; wy[IX(W, i, ny + 1)] = 0; wy[IX(W, i, ny + 2)] = 0;
   u[IX(W, i, ny + 1)] = u[IX(W, i, ny)]; u[IX(W, i, ny + 2)] = u[IX(W, i, ny + 1)];
   wx[IX(W, i, ny + 1)] = wx[IX(W, i, ny)]; wx[IX(W, i, ny + 2)] = wx[IX(W, i, ny + 1)];
+}
+
+// A whole step's halo update of u and v followed by do_channel, in one launch
+// (a band): the x-halo columns of the interior rows and the corners take the
+// wrap, the interior columns of the wall rows do_channel's values. do_channel
+// zeroes row ny of v, whose cells next to the seam the halo update copies
+// first: one thread does both for them. winds: do_channel's rows of windx and
+// windy, which it leaves as they are when they are +0.0 everywhere.
+__global__ void k_halo_channel(int nx, int ny, double* u, double* v, double* wx, double* wy, bool winds) {
+  SW2G_PDL_ENTRY();
+  const int W = nx + 4;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  auto halo_col = [&](int c) { return c < 2 ? c - 1 : nx + c - 1; };  // columns -1, 0, nx+1, nx+2
+  auto wrap = [&](int i) { return i < 1 ? i + nx : (i > nx ? i - nx : i); };
+  if (t < nx) {  // do_channel (calc.c:600-649)
+    const int i = t + 1;
+    const double lo = u[IX(W, i, 1)], hi = u[IX(W, i, ny)];
+    u[IX(W, i, 0)] = lo; u[IX(W, i, -1)] = lo;
+    u[IX(W, i, ny + 1)] = hi; u[IX(W, i, ny + 2)] = hi;
+    v[IX(W, i, 0)] = 0; v[IX(W, i, -1)] = 0;
+    v[IX(W, i, ny + 1)] = 0; v[IX(W, i, ny + 2)] = 0;
+    if (i > 2 && i < nx - 1) v[IX(W, i, ny)] = 0;
+    if (winds) {
+      const double wlo = wx[IX(W, i, 1)], whi = wx[IX(W, i, ny)];
+      wx[IX(W, i, 0)] = wlo; wx[IX(W, i, -1)] = wlo;
+      wx[IX(W, i, ny + 1)] = whi; wx[IX(W, i, ny + 2)] = whi;
+      wy[IX(W, i, 0)] = 0; wy[IX(W, i, -1)] = 0;
+      wy[IX(W, i, ny)] = 0; wy[IX(W, i, ny + 1)] = 0; wy[IX(W, i, ny + 2)] = 0;
+    }
+    return;
+  }
+  const int h = t - nx;
+  if (h < 4 * (ny - 1)) {  // x halos of rows 1 .. ny-1
+    const int c = h / (ny - 1), j = h - c * (ny - 1) + 1, i = halo_col(c), si = wrap(i);
+    u[IX(W, i, j)] = u[IX(W, si, j)];
+    v[IX(W, i, j)] = v[IX(W, si, j)];
+  } else if (h == 4 * (ny - 1)) {  // row ny and the corners, sppde_hupdate.c:274-342
+    const int rows[4] = {-1, 0, ny + 1, ny + 2}, from[4] = {ny - 1, ny, 1, 2};
+    double vn[4];
+    for (int c = 0; c < 4; c++) vn[c] = v[IX(W, wrap(halo_col(c)), ny)];
+    for (int c = 0; c < 4; c++) {
+      const int i = halo_col(c), si = wrap(i);
+      u[IX(W, i, ny)] = u[IX(W, si, ny)];
+      v[IX(W, i, ny)] = vn[c];
+      for (int r = 0; r < 4; r++) {
+        u[IX(W, i, rows[r])] = u[IX(W, si, from[r])];
+        v[IX(W, i, rows[r])] = r == 1 ? vn[c] : v[IX(W, si, from[r])];
+      }
+    }
+    for (int c = 0; c < 4; c++) v[IX(W, wrap(halo_col(c)), ny)] = 0;
+  }
 }
 
 // compute_Dt maxima (calc.c:705-712): max |u+wx|/DXE and |v+wy|/DYN over the
@@ -1891,7 +2078,7 @@ namespace {
 // their own tendencies, so the order changes no value, and a caller that
 // copies eta in can overlap that copy with them (StepHooks).
 int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, StepChecks chk, int slot,
-              cudaStream_t st, Timers* tm, bool fused_checks, StepHooks hk) {
+              cudaStream_t st, Timers* tm, bool fused_checks, bool whole, StepHooks hk) {
   int* const fbad = fused_checks ? chk.bad + slot : nullptr;
   const dim3 g((s.nx + TX - 1) / TX, s.ny);
   int nl = 0;
@@ -1899,26 +2086,29 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   const bool hyper = (s.nu2 != 0 || s.nu4 != 0 || s.nu6 != 0);
 
   // The Laplacians of the mass equation's hyperviscosity (calc.c:325-335,
-  // laplacian.c:110-146). The reference zeroes Le, psi and xi before them
-  // (calc.c:325-327, laplacian.c:116-118). Here they are zeroed once at
-  // allocation: every level that runs rewrites all cells of its Le
-  // (interior, halo wrap, wall rows) and the interior of psi and xi, whose
-  // halos stay zero; levels that do not run leave their Le zero.
-  auto eta_laplacians = [&]() {
-    const double* src = s.lape_eta ? b.f[0] : b.f[1];  // the reference passes u, not eta (calc.c:332)
-    const int nlap = (s.nu4 != 0 || s.nu6 != 0) ? ((s.nu6 != 0) ? 3 : 2) : 1;
-    for (int q = 0; q < nlap; q++) {
-      LAUNCH("lape_pass1", pdl_launch(k_lape_pass1, dim3(g), dim3(TX), st, s, q == 0 ? src : b.Le[q - 1], b.psi, b.xi));
-      // halo and wall rows of Le are written by the pass (a polar cap has no walls)
-      LAUNCH("lape_pass2", pdl_launch(k_lape_pass2, dim3(g), dim3(TX), st, s, b.psi, b.xi, b.Le[q]));
-    }
+  // laplacian.c:110-146). The reference zeroes Le before them (calc.c:325-327).
+  // Here it is zeroed once at allocation: every level that runs rewrites all
+  // cells of its Le (interior, halo wrap, wall rows), and levels that do not
+  // run leave their Le zero.
+  const int nlap = !hyper ? 0 : (s.nu6 != 0) ? 3 : (s.nu4 != 0) ? 2 : 1;
+  auto lap_eta_source = [&](int q) -> const double* {
+    // the reference passes u, not eta (calc.c:332)
+    return q > 0 ? b.Le[q - 1] : s.lape_eta ? b.f[0] : b.f[1];
+  };
+  auto eta_laplacians = [&](int levels) {
+    const March m = march(s, FW, 4);
+    for (int q = 0; q < levels; q++)
+      LAUNCH("lape", pdl_launch(k_lape, m.grid, dim3(TX), st, s, lap_eta_source(q), b.Le[q], m.rows));
   };
   // Reading u alone, and nothing that the kernels before their place in the
   // reference's order write, they run first when a caller copies the fields
   // in, which then overlaps the copies of v and eta with them (StepHooks);
   // otherwise they keep their place after the mass body.
   const bool laplacians_first = hyper && !s.lape_eta && hk.v_in;
-  if (laplacians_first) eta_laplacians();
+  // From the third step the eta kernel computes the last level itself, except
+  // where that level's source is eta, which the kernel changes.
+  const bool last_in_eta = hyper && k >= 2 && !laplacians_first && !(s.lape_eta && nlap == 1);
+  if (laplacians_first) eta_laplacians(nlap);
   if (hk.v_in) cudaStreamWaitEvent(st, hk.v_in, 0);
 
   // compute_Dt (core.c:155-159): maxima at the start of the step
@@ -1942,11 +2132,11 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   if (hk.eta_in) cudaStreamWaitEvent(st, hk.eta_in, 0);
   LAUNCH("mass", body(0, sch, g, st, s, F(), b.deta[0]));
   if (hyper) {
-    if (!laplacians_first) eta_laplacians();
+    if (!laplacians_first) eta_laplacians(last_in_eta ? nlap - 1 : nlap);
     if (k < 2) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
   }
   if (k >= 2) {
-    LAUNCH("eta_ab3", fused_tail(s, g, st, F(), b, 0, fbad));  // writes eta's halo images too
+    LAUNCH("eta_ab3", fused_tail(s, g, st, F(), b, 0, fbad, last_in_eta ? lap_eta_source(nlap - 1) : nullptr));  // writes eta's halo images too
     rotate3(b.deta);
   } else {
     LAUNCH("ab", pdl_launch(k_ab, dim3(g), dim3(TX), st, s, k, b.detaAB, b.deta[0], b.deta[1], b.deta[2]));
@@ -1958,21 +2148,20 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   if (hk.eta_out) cudaEventRecord(hk.eta_out, st);  // eta is final for this step
 
   // momentum (core.c:212-280)
-  if (s.polar == 0 && s.sigma == 0.0)
+  // (from the third step in the Coriolis kernels)
+  if (k >= 2) {
+  } else if (s.polar == 0 && s.sigma == 0.0)
     LAUNCH("pres_sum", pdl_launch(k_pres_sum<true>, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
   else
     LAUNCH("pres_sum", pdl_launch(k_pres_sum<false>, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
   if (hyper) {
-    // As above: each level rewrites every cell of ze, di and its two L fields
-    // (interior, halo wraps, wall fixes), and L of levels not run stay zero.
-    const int nlap = (s.nu4 != 0 || s.nu6 != 0) ? ((s.nu6 != 0) ? 3 : 2) : 1;
-    for (int q = 0; q < nlap; q++) {
-      const double* uu = q == 0 ? b.f[1] : b.L[2 * q - 2];
-      const double* vv = q == 0 ? b.f[2] : b.L[2 * q - 1];
-      // halos and wall fixes of ze, di and of the outputs are written by the passes
-      LAUNCH("lapv_pass1", pdl_launch(k_lapv_pass1, dim3(dim3(g.x, (s.ny + LV_ROWS - 1) / LV_ROWS)), dim3(TX), st, s, uu, vv, b.ze, b.di));
-      LAUNCH("lapv_pass2", pdl_launch(k_lapv_pass2, dim3(g), dim3(TX), st, s, b.ze, b.di, b.L[2 * q], b.L[2 * q + 1]));
-    }
+    // As above: each level but the last rewrites every cell of its two L fields
+    // (interior, halo wraps, wall fixes), the last their interior, which is all
+    // that is read of it; L of levels not run stay zero.
+    const March m = march(s, LVW, 8);
+    for (int q = 0; q < nlap; q++)
+      LAUNCH("lapv", pdl_launch(k_lapv, m.grid, dim3(TX), st, s, q == 0 ? b.f[1] : b.L[2 * q - 2],
+                                q == 0 ? b.f[2] : b.L[2 * q - 1], b.L[2 * q], b.L[2 * q + 1], m.rows, q + 1 < nlap));
     if (k < 2) {
       LAUNCH("hyper_add", hyper_add(s, g, st, b.du[0], b.L[0], b.L[2], b.L[4]));
       LAUNCH("hyper_add", hyper_add(s, g, st, b.dv[0], b.L[1], b.L[3], b.L[5]));
@@ -1998,7 +2187,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   }
 
   // halos (core.c:287-290)
-  LAUNCH("halo", halo_wrap2(b.f[1], b.f[2], s.nx, s.ny, st));
+  if (!whole) LAUNCH("halo", halo_wrap2(b.f[1], b.f[2], s.nx, s.ny, st));
   return nl;
 }
 
@@ -2007,11 +2196,12 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
 // forcing (core.c:296-300) is done by the forcing calls themselves, so the
 // tail is do_channel and the range checks (core.c:303-312).
 int step_tail(const DevState& s, Fp64Buffers& b, bool tracer, StepChecks chk, int slot, cudaStream_t st,
-              Timers* tm, bool fused_checks) {
+              Timers* tm, bool fused_checks, bool whole) {
   const dim3 g((s.nx + TX - 1) / TX, s.ny);
   const int gw = (s.nx + 127) / 128;
   int nl = 0;
-  if (s.polar == 0) LAUNCH("channel", pdl_launch(k_channel, dim3(gw), dim3(128), st, s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5]));
+  if (whole) LAUNCH("halo_channel", pdl_launch(k_halo_channel, dim3((s.nx + 4 * (s.ny - 1) + 1 + 127) / 128), dim3(128), st, s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5], s.plain == 0));
+  else if (s.polar == 0) LAUNCH("channel", pdl_launch(k_channel, dim3(gw), dim3(128), st, s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5]));
 
   // range checks of tracer, eta, u, v (core.c:309-312); an all-zero tracer
   // passes trivially
@@ -2031,8 +2221,9 @@ int fp64_step(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
               cudaStream_t st, Timers* tm, int parts, StepHooks hk) {
   int nl = 0;
   const bool fused_checks = (parts == STEP_FULL) && !tracer && k >= 2;
-  if (parts & STEP_HEAD) nl += step_head(s, b, sch, k, tracer, chk, slot, st, tm, fused_checks, hk);
-  if (parts & STEP_TAIL) nl += step_tail(s, b, tracer, chk, slot, st, tm, fused_checks);
+  const bool whole = (parts == STEP_FULL) && s.polar == 0;  // halos and do_channel in one launch
+  if (parts & STEP_HEAD) nl += step_head(s, b, sch, k, tracer, chk, slot, st, tm, fused_checks, whole, hk);
+  if (parts & STEP_TAIL) nl += step_tail(s, b, tracer, chk, slot, st, tm, fused_checks, whole);
   return nl;
 }
 

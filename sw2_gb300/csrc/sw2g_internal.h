@@ -118,7 +118,6 @@ struct Fp64Buffers {
   double* detaAB; double* duAB; double* dvAB; double* dtrAB;
   double* duadv; double* dvadv;
   double* Le[3]; double* L[6];
-  double* psi; double* xi; double* ze; double* di;
 };
 
 struct StepChecks {
