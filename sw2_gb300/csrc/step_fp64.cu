@@ -31,7 +31,7 @@ __device__ __forceinline__ double PF(const DevState& s, int t, int q) { return s
 // Brings the line of a value that a later row reads into L1, without a
 // register to hold it: a load whose result nothing uses.
 __device__ __forceinline__ void touch(const double* p) {
-  double x;
+  [[maybe_unused]] double x;
   asm volatile("ld.global.ca.f64 %0, [%1];" : "=d"(x) : "l"(p));
 }
 
@@ -275,15 +275,13 @@ __device__ __forceinline__ double mass_cell(const DevState& s, const F7& f, int 
 
 // Programmatic dependent launch of the step's kernels: each kernel starts by
 // waiting for the previous kernel of the stream to complete (a no-op for a
-// kernel launched without the attribute) and then lets the next one be
-// scheduled, which happens once all of its own blocks are resident; so a
-// launch's scheduling overlaps the drain of the kernel before it, and no
-// kernel reads or writes memory before its predecessor has finished.
-#define SW2G_PDL_ENTRY()                                            \
-  do {                                                              \
-    asm volatile("griddepcontrol.wait;" ::: "memory");              \
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); \
-  } while (0)
+// kernel launched without the attribute), so its launch overlaps the kernel
+// before it, and no kernel reads or writes memory before its predecessor has
+// finished. None lets its dependents in before it ends
+// (griddepcontrol.launch_dependents): blocks that wait where the predecessor's
+// last blocks still run cost more than they save (a step at 256x128 98 us with
+// it, 88 without; at 1201x607 660 and 631; at 2048x1024 0.2 % less with it).
+#define SW2G_PDL_ENTRY() asm volatile("griddepcontrol.wait;" ::: "memory")
 
 template <typename... KArgs, typename... Args>
 void pdl_launch(void (*k)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
@@ -1623,6 +1621,19 @@ __global__ void __launch_bounds__(TX, 16) k_eta_lap_ab3(DevState s, F7 f, double
   }
 }
 
+// The tracer's update (calc.c:651-699, core.c:161-182): AB3, tracer += D and its
+// halo update. As k_ab, k_add and k_halo in turn 0.031 ms at 1201x607, so
+// 0.012.
+__global__ void __launch_bounds__(TX, 16) k_tracer_ab3(DevState s, double* tr, const double* dn, const double* dm1,
+                                                       const double* dm2, int* bad) {
+  SW2G_PDL_ENTRY();
+  INTERIOR_IJ
+  const int q = IX(W, i, j);
+  const double t = tr[q] + ab3(dn[q], dm1[q], dm2[q]);
+  put_images<HK_WRAP>(s, tr, i, j, t);
+  check_range(bad, t, i, j);
+}
+
 template <int NZ, bool UD>
 __global__ void __launch_bounds__(TX, 16) k_coriolis_u_ab3(DevState s, double* u, const double* v, const double* eta, const double* duadv,
                                  double* dn, const double* dm1, const double* dm2, const double* l2,
@@ -2071,8 +2082,8 @@ namespace {
   } while (0)
 
 // Head of a step: core.c:134-290, through the velocity halos.
-// fused_checks: the range checks of eta, u and v are done by the kernels that
-// write their new values (a whole step with a zero tracer, from the third step).
+// fused_checks: the range checks are done by the kernels that write the new
+// values (a whole step, from the third step).
 // The advection sweeps of u and v (core.c:212-215) run before the mass
 // update: they read only u, v, the winds and the geometry, and write only
 // their own tendencies, so the order changes no value, and a caller that
@@ -2118,10 +2129,15 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   // the step then provably leaves unchanged
   if (tracer) {
     LAUNCH("tracer", body(1, sch, g, st, s, F(), b.dtr[0]));
-    LAUNCH("ab", pdl_launch(k_ab, dim3(g), dim3(TX), st, s, k, b.dtrAB, b.dtr[0], b.dtr[1], b.dtr[2]));
-    rotate3(b.dtr);
-    LAUNCH("add", pdl_launch(k_add, dim3(g), dim3(TX), st, s, b.f[3], b.dtrAB));
-    LAUNCH("halo", halo_wrap(b.f[3], s.nx, s.ny, st));
+    if (k >= 2) {
+      LAUNCH("tracer_ab3", pdl_launch(k_tracer_ab3, g, dim3(TX), st, s, b.f[3], b.dtr[0], b.dtr[1], b.dtr[2], fbad));
+      rotate3(b.dtr);
+    } else {
+      LAUNCH("ab", pdl_launch(k_ab, dim3(g), dim3(TX), st, s, k, b.dtrAB, b.dtr[0], b.dtr[1], b.dtr[2]));
+      rotate3(b.dtr);
+      LAUNCH("add", pdl_launch(k_add, dim3(g), dim3(TX), st, s, b.f[3], b.dtrAB));
+      LAUNCH("halo", halo_wrap(b.f[3], s.nx, s.ny, st));
+    }
   }
 
   // advection of u and v (core.c:212-215)
@@ -2220,7 +2236,7 @@ int step_tail(const DevState& s, Fp64Buffers& b, bool tracer, StepChecks chk, in
 int fp64_step(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, StepChecks chk, int slot,
               cudaStream_t st, Timers* tm, int parts, StepHooks hk) {
   int nl = 0;
-  const bool fused_checks = (parts == STEP_FULL) && !tracer && k >= 2;
+  const bool fused_checks = (parts == STEP_FULL) && k >= 2;
   const bool whole = (parts == STEP_FULL) && s.polar == 0;  // halos and do_channel in one launch
   if (parts & STEP_HEAD) nl += step_head(s, b, sch, k, tracer, chk, slot, st, tm, fused_checks, whole, hk);
   if (parts & STEP_TAIL) nl += step_tail(s, b, tracer, chk, slot, st, tm, fused_checks, whole);
