@@ -12,7 +12,10 @@ namespace sw2g {
 namespace f32 {
 
 
-__global__ void kb_advance(int* counter) { *counter += 1; }
+__global__ void kb_advance(int* counter) {
+  pdl_entry();
+  *counter += 1;
+}
 
 // FP32 shadow of an FP64 field over all padded cells (pitch W -> pitch P).
 __global__ void k_shadow(float* dst, const double* src, int nx, int ny, int W, int P) {
@@ -194,7 +197,8 @@ int batch_step_n(int sch, int sr, const MemberDesc* desc, int nmem, const int4* 
     if (nu6) run_phase<kb_lap3<N>, N>("f32_lap3", kSmemLap, a, nl);
     run_phase<kb_main2<N>, N>("f32_main2", kSmemMain2, a, nl);
   }
-  kb_advance<<<1, 1, 0, st>>>(counter);
+  const PdlLaunch l(dim3(1), dim3(1), 0, st);
+  cudaLaunchKernelEx(&l.cfg, kb_advance, counter);
   nl++;
   return nl;
 }

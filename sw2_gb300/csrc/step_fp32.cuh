@@ -1378,12 +1378,20 @@ __device__ __forceinline__ bool strip_main2(const MemberDesc& d, const View& vw,
 }
 
 // ------------------------------------------------------------------ kernels
+// Programmatic dependent launch of the step's kernels: each sets up its
+// barriers and then waits for its predecessor to complete before it reads or
+// writes global memory, so its launch and set-up overlap the kernel before.
+// None lets its dependents in before it ends: their blocks, resident early
+// beside the last of the predecessor's, made a step at 4096x2048 8 % slower.
+__device__ __forceinline__ void pdl_entry() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Each warp of a block is an independent strip worker with its own ring.
 // A warp that gave up on a wait (timeout) takes no further strips.
 #define SW2G_STRIP_LOOP(NF, D, CALL)                                   \
   extern __shared__ __align__(128) unsigned char sm[];                  \
   Ring<NF, D> rg;                                                      \
   ring_init(sm, rg);                                                   \
+  pdl_entry();                                                         \
   const int n = *counter;                                              \
   bool first = true;                                                   \
   for (;;) {                                                           \
@@ -1429,6 +1437,7 @@ __global__ void __launch_bounds__(NT, EXTRA ? 2 : 3) kb_main1(SW2G_KPARAMS) {
   ring_init_at(a, 0, main1_bars<EXTRA>(), rg);
   ring_init_at(a, NWARP * kDMain1 * 8, main1_lrows<EXTRA>(), rl);
   const unsigned stg = smem_u32(a + main1_stage<EXTRA>() + (threadIdx.x >> 5) * kStageMain1);
+  pdl_entry();
   const int n = *counter;
   bool first = true;
   for (;;) {
@@ -1494,6 +1503,22 @@ struct PhaseArgs {
   Timers* tm;
 };
 
+// A launch with programmatic stream serialization (pdl_entry).
+struct PdlLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  PdlLaunch(dim3 g, dim3 b, int smem, cudaStream_t st) {
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+  }
+};
+
 // One launch of kernel K over the strips: at most as many blocks as are
 // resident (the warps take the strips from the queue), under the named timer.
 // A single member's strips are as high as makes their number a whole
@@ -1512,7 +1537,8 @@ void run_phase(const char* tag, int smem, const PhaseArgs<N>& a, int& nl) {
     nstrips = a.nbx * ((a.ny + sr - 1) / sr);
   }
   const int want = (nstrips + NWARP - 1) / NWARP;
-  K<<<want < cap ? want : cap, NT, smem, a.st>>>(*a.ds, a.tiles, nstrips, a.nbx, sr, a.counter, a.queue);
+  const PdlLaunch l(dim3(want < cap ? want : cap), dim3(NT), smem, a.st);
+  cudaLaunchKernelEx(&l.cfg, K, *a.ds, a.tiles, nstrips, a.nbx, sr, (const int*)a.counter, a.queue);
   if (a.tm && a.tm->on) a.tm->end(a.st);
   nl++;
 }
