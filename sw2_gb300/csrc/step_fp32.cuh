@@ -455,6 +455,12 @@ __device__ __forceinline__ bool ring_wait(const Ring<NF, D>& r, int t, int* bad)
   for (int u = t; u < r.issued; u++) r.try_row(u, TILE_DRAIN_LIMIT);
   return false;
 }
+// Before a warp leaves: waits (bounded) for the rows from t on that it has
+// issued and not waited for.
+template <int NF, int D>
+__device__ __forceinline__ void ring_drain(const Ring<NF, D>& r, int t) {
+  for (int u = t; u < r.issued; u++) r.try_row(u, TILE_DRAIN_LIMIT);
+}
 // Failure-path test: after row 0 has arrived, also wait for the next phase
 // of its slot, which nothing completes before row D is issued; gives up
 // after `waits` tries like a real timeout.
@@ -752,27 +758,56 @@ __device__ __forceinline__ bool strip_lap(const MemberDesc& d, const View& vw, i
 }
 
 // ---------------------------------------------------------------- kb_main1
-// Two rings per warp: rows j0-2 .. j1+2 (ring row t <-> j0-2+t) of the eta,
-// u and v shadows, and with EXTRA the winds and the bottom height (UWINDX,
-// VWINDY of sw.h:216-217 and H = eta + depth - hB, sw.h:213); and rows
-// j0-1 .. j1+1 (ring row t <-> j0-1+t) of the first Laplacian level Lu, Lv,
-// of which row j needs only j and j+1.
-constexpr int kDLapIn = 3;  // depth of the Laplacian-level ring of kb_main1
+// The momentum tendencies and the mass update, as two kinds of strips of one
+// launch, which its warps take from the queue, the longer momentum strips
+// first. In one strip their windows, carried faces and rings took 168
+// registers and 19 KB of shared memory a warp, which left 12 warps per SM;
+// apart they take 96 registers and 11 KB, and 20 are resident, for u and v read
+// twice: 0.229 -> 0.199 ms at 4096x2048 (bound by instruction latency: issue on
+// two thirds of the cycles before).
+//
+// Mass: rows j0-2 .. j1+2 (ring row t <-> j0-2+t) of the eta shadow, with
+// EXTRA of the bottom height (H = eta + depth - hB, sw.h:213); and rows j0-1 ..
+// j1 (ring row t <-> j0-1+t) of the u and v shadows, with EXTRA of the winds
+// (UWINDX, VWINDY of sw.h:216-217), of which row j needs j-1 and j.
+// Momentum: rows j0-2 .. j1+2 of u, v and the winds; and rows j0-1 .. j1+1 of
+// the first Laplacian level Lu, Lv, of which row j needs j and j+1.
+constexpr int kDNear = 3;  // depth of the rings of two rows a cell
 template <bool EXTRA>
-__host__ __device__ constexpr int main1_fields() { return EXTRA ? 6 : 3; }
+using RingEta = Ring<EXTRA ? 2 : 1, kDMain1>;
 template <bool EXTRA>
-__host__ __device__ constexpr int main1_bars() {
-  return (NWARP * (kDMain1 + kDLapIn) * 8 + 127) / 128 * 128;
-}
+using RingFlow = Ring<EXTRA ? 4 : 2, kDNear>;
 template <bool EXTRA>
-__host__ __device__ constexpr int main1_lrows() {
-  return main1_bars<EXTRA>() + NWARP * kDMain1 * main1_fields<EXTRA>() * RS * 4;
-}
-// own-cell staging of a warp: two rows of [eta (32 lanes x 4 doubles), h1, h2 (32 x 4 floats)]
+using RingVel = Ring<EXTRA ? 4 : 2, kDMain1>;
+using RingLap = Ring<2, kDNear>;
+// Shared memory of a block: the barriers of the four rings of each warp, then
+// for each warp an area that holds the rows of the kind of strip it works on.
+// own-cell staging of a mass strip: two rows of [eta (32 lanes x 4 doubles), h1, h2 (32 x 4 floats)]
 constexpr int kStageMain1 = 2 * 2048;
+constexpr int kBarsMain1 = (NWARP * (2 * kDMain1 + 2 * kDNear) * 8 + 127) / 128 * 128;
 template <bool EXTRA>
-__host__ __device__ constexpr int main1_stage() {
-  return main1_lrows<EXTRA>() + NWARP * kDLapIn * 2 * RS * 4;
+__host__ __device__ constexpr int main1_mass() {  // rows of a mass strip, then its staging
+  return (kDMain1 * (EXTRA ? 2 : 1) + kDNear * (EXTRA ? 4 : 2)) * RS * 4;
+}
+template <bool EXTRA>
+__host__ __device__ constexpr int main1_area() {
+  const int mass = main1_mass<EXTRA>() + kStageMain1, mom = (kDMain1 * (EXTRA ? 4 : 2) + kDNear * 2) * RS * 4;
+  return mass > mom ? mass : mom;
+}
+
+// A ring with its barriers at bar and its rows at buf (the warp's own).
+template <int NF, int D>
+__device__ __forceinline__ void ring_place(unsigned char* bar, unsigned char* buf, Ring<NF, D>& r) {
+  r.bar = reinterpret_cast<unsigned long long*>(bar);
+  r.buf = reinterpret_cast<float*>(buf);
+  r.base = 0;
+  r.issued = 0;
+  if (lane_id() == 0) {
+    for (int s = 0; s < D; s++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&r.bar[s])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
 }
 
 // Sections of a row are separated by a compiler fence, so that windows are
@@ -781,106 +816,35 @@ __host__ __device__ constexpr int main1_stage() {
 __device__ __forceinline__ void section() { asm volatile("" ::: "memory"); }
 
 template <int SCH, bool EXTRA, bool POLAR>
-__device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw, int sx, int sy, int SR,
-                                            Ring<main1_fields<EXTRA>(), kDMain1>& rg, Ring<2, kDLapIn>& rl,
-                                            unsigned stg, bool test) {
-  enum { FE, FU, FV, FWX, FWY, FHB };
+__device__ __forceinline__ bool strip_mass(const MemberDesc& d, const View& vw, int sx, int sy, int SR,
+                                           RingEta<EXTRA>& re, RingFlow<EXTRA>& ru, unsigned stg, bool test) {
+  enum { FE, FHB };
+  enum { FU, FV, FWX, FWY };
   const int nx = d.nx, ny = d.ny, P = d.P, W = nx + 4;
   const float* q = d.q;
   const int i0 = sx * SW + 1, j0 = sy * SR + 1, j1 = min(j0 + SR - 1, ny);
   const int ib = i0 + 4 * lane_id();
   int* bad = d.bad + vw.slot;
-  rg.map[FE] = map_of(d, TM_ES + vw.cur);
-  rg.map[FU] = map_of(d, TM_US + vw.cur);
-  rg.map[FV] = map_of(d, TM_VS + vw.cur);
+  re.map[FE] = map_of(d, TM_ES + vw.cur);
+  ru.map[FU] = map_of(d, TM_US + vw.cur);
+  ru.map[FV] = map_of(d, TM_VS + vw.cur);
   if constexpr (EXTRA) {
-    rg.map[FWX] = map_of(d, TM_WX);
-    rg.map[FWY] = map_of(d, TM_WY);
-    rg.map[FHB] = map_of(d, TM_HB);
+    re.map[FHB] = map_of(d, TM_HB);
+    ru.map[FWX] = map_of(d, TM_WX);
+    ru.map[FWY] = map_of(d, TM_WY);
   }
-  rg.x = sx * SW;
-  rg.y0 = j0 - 1;  // tensor row of j0 - 2
-  rg.T = j1 - j0 + 5;
-  rl.map[0] = map_of(d, TM_LU);
-  rl.map[1] = map_of(d, TM_LV);
-  rl.x = sx * SW;
-  rl.y0 = j0;  // tensor row of j0 - 1
-  rl.T = j1 - j0 + 3;
-  ring_begin(rg);
-  ring_begin(rl);
-  for (int t = 0; t < 4; t++)
-    if (!ring_wait(rg, t, bad)) return false;
-  if (!ring_wait(rl, 0, bad) || !ring_wait(rl, 1, bad)) return false;
-  if (test && !ring_test(rg, d.tile_test, bad)) return false;
-
-  // windows of the stencil fields, with the winds added to u, v and the
-  // bottom height taken from eta when the member has them
-  auto E8 = [&](int t, float (&w)[8]) {
-    win8(rg.row(t, FE), w);
-    if constexpr (EXTRA) { float x[8]; win8(rg.row(t, FHB), x); addw(w, x, -1.f); }
-  };
-  auto E4 = [&](int t, float (&w)[4]) {
-    own4(rg.row(t, FE), w);
-    if constexpr (EXTRA) { float x[4]; own4(rg.row(t, FHB), x); addw(w, x, -1.f); }
-  };
-  auto U8 = [&](int t, float (&w)[8]) {
-    win8(rg.row(t, FU), w);
-    if constexpr (EXTRA) { float x[8]; win8(rg.row(t, FWX), x); addw(w, x, 1.f); }
-  };
-  auto U4 = [&](int t, float (&w)[4]) {
-    own4(rg.row(t, FU), w);
-    if constexpr (EXTRA) { float x[4]; own4(rg.row(t, FWX), x); addw(w, x, 1.f); }
-  };
-  auto V8 = [&](int t, float (&w)[8]) {
-    win8(rg.row(t, FV), w);
-    if constexpr (EXTRA) { float x[8]; win8(rg.row(t, FWY), x); addw(w, x, 1.f); }
-  };
-  auto V4 = [&](int t, float (&w)[4]) {
-    own4(rg.row(t, FV), w);
-    if constexpr (EXTRA) { float x[4]; own4(rg.row(t, FWY), x); addw(w, x, 1.f); }
-  };
-
-  // carried from row to row: the y faces south of the row (mass: limited
-  // slope and upwind value relative to the reference of the row below; u, v:
-  // limited slopes), ZE of the row below and DI of the row
-  float2 ysm[4], ysu[4], ysv[4];
-  float zm[4], dj[5];
-  {
-    const int jm = j0 - 1;
-    float ea[4], eb[4], ec[4], ed[4], vb[4];
-    E4(0, ea); E4(1, eb); E4(2, ec); E4(3, ed); V4(1, vb);
-    const float dm1 = Qr(q, Q_DHBM1, jm), dp1 = Qr(q, Q_DHBP1, jm), dp2 = Qr(q, Q_DHBP2, jm);
-#pragma unroll
-    for (int c = 0; c < 4; c++) ysm[c] = face1_shared<SCH>(ea[c] + dm1, eb[c], ec[c] + dp1, ed[c] + dp2, vb[c] > 0.f);
-    float a[4], b[4], cc[4], dd[4];
-    U4(0, a); U4(1, b); U4(2, cc); U4(3, dd);
-#pragma unroll
-    for (int c = 0; c < 4; c++) ysu[c] = face2_shared<SCH>(a[c], b[c], cc[c], dd[c]);
-    V4(0, a); V4(2, cc); V4(3, dd);
-#pragma unroll
-    for (int c = 0; c < 4; c++) ysv[c] = face2_shared<SCH>(a[c], vb[c], cc[c], dd[c]);
-    float la[8], lb[8], ma[8], mb[8], zt[5];
-    win8(rl.row(0, 0), la); win8(rl.row(1, 0), lb);
-    win8(rl.row(0, 1), ma); win8(rl.row(1, 1), mb);
-    ze5<POLAR>(q, nx, ny, P, ib, jm, la, lb, ma, d.Lu, d.Lv, zt);
-#pragma unroll
-    for (int c = 0; c < 4; c++) zm[c] = zt[c + 1];
-    di5<POLAR>(q, nx, ny, P, ib, j0, lb, mb, ma, la, d.Lu, d.Lv, dj);
-  }
-
-  const float sig2dt = d.sig2dt, sigdt = d.sigdt, nu2dt = d.nu2dt, nu4dt = d.nu4dt;
-  const bool keep_ll = (d.nu6dt != 0.f);
-  const int PR = P * (ny + 4);  // stride of a cap's per-cell fields
+  re.x = ru.x = sx * SW;
+  re.y0 = j0 - 1;  // tensor row of j0 - 2
+  re.T = j1 - j0 + 5;
+  ru.y0 = j0;  // tensor row of j0 - 1
+  ru.T = j1 - j0 + 2;
+  ring_begin(re);
+  ring_begin(ru);
+  // own-cell inputs of a row, staged a row ahead (slot k & 1 of the row j0 + k)
   const double* eta_in = d.eta[vw.cur];
-  double* eta_out = d.eta[1 - vw.cur];
-  float* es_out = d.es[1 - vw.cur];
   const float* h1p = d.heta[vw.h1];
   const float* h2p = d.heta[vw.h2];
-  float* hw = d.heta[vw.w];
   const int kab = vw.k;
-  float mxu = 0.f, mxv = 0.f;
-  bool oor = false;
-  // own-cell inputs of a row, staged a row ahead (slot k & 1 of the row j0 + k)
   const int l = lane_id();
   auto stage = [&](int jr, int slot) {
     const unsigned b = stg + slot * 2048;
@@ -890,14 +854,64 @@ __device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw,
   };
   stage(j0, 0);
   cpa_commit();
+  for (int t = 0; t < 4; t++)
+    if (!ring_wait(re, t, bad)) {
+      ring_drain(ru, 0);
+      cpa_wait0();
+      return false;
+    }
+  if (!ring_wait(ru, 0, bad) || (test && !ring_test(re, d.tile_test, bad))) {
+    ring_drain(re, 4);
+    ring_drain(ru, 1);
+    cpa_wait0();
+    return false;
+  }
 
+  // windows of the stencil fields, with the winds added to u, v and the
+  // bottom height taken from eta when the member has them
+  auto E8 = [&](int t, float (&w)[8]) {
+    win8(re.row(t, FE), w);
+    if constexpr (EXTRA) { float x[8]; win8(re.row(t, FHB), x); addw(w, x, -1.f); }
+  };
+  auto E4 = [&](int t, float (&w)[4]) {
+    own4(re.row(t, FE), w);
+    if constexpr (EXTRA) { float x[4]; own4(re.row(t, FHB), x); addw(w, x, -1.f); }
+  };
+  auto U8 = [&](int t, float (&w)[8]) {
+    win8(ru.row(t, FU), w);
+    if constexpr (EXTRA) { float x[8]; win8(ru.row(t, FWX), x); addw(w, x, 1.f); }
+  };
+  auto V4 = [&](int t, float (&w)[4]) {
+    own4(ru.row(t, FV), w);
+    if constexpr (EXTRA) { float x[4]; own4(ru.row(t, FWY), x); addw(w, x, 1.f); }
+  };
+
+  // carried from row to row: the y faces south of the row (limited slope and
+  // upwind value relative to the reference of the row below)
+  float2 ysm[4];
+  {
+    const int jm = j0 - 1;
+    float ea[4], eb[4], ec[4], ed[4], vb[4];
+    E4(0, ea); E4(1, eb); E4(2, ec); E4(3, ed); V4(0, vb);
+    const float dm1 = Qr(q, Q_DHBM1, jm), dp1 = Qr(q, Q_DHBP1, jm), dp2 = Qr(q, Q_DHBP2, jm);
+#pragma unroll
+    for (int c = 0; c < 4; c++) ysm[c] = face1_shared<SCH>(ea[c] + dm1, eb[c], ec[c] + dp1, ed[c] + dp2, vb[c] > 0.f);
+  }
+  const float sig2dt = d.sig2dt;
+  const int PR = P * (ny + 4);  // stride of a cap's per-cell fields
+  double* eta_out = d.eta[1 - vw.cur];
+  float* es_out = d.es[1 - vw.cur];
+  float* hw = d.heta[vw.w];
+  bool oor = false;
   for (int j = j0; j <= j1; j++) {
-    const int k = j - j0, t = k + 2;  // ring row of j (the Laplacian ring: k + 1)
-    ring_refill(rg, k);
-    ring_refill(rl, k);
+    const int k = j - j0, t = k + 2;  // ring row of j (u, v: k + 1)
+    ring_refill(re, k);
+    if (k > 0) ring_refill(ru, k - 1);
     if (j < j1) stage(j + 1, (k + 1) & 1);
     cpa_commit();
-    if (!ring_wait(rg, t + 2, bad) || !ring_wait(rl, k + 2, bad)) {
+    if (!ring_wait(re, t + 2, bad) || !ring_wait(ru, k + 1, bad)) {
+      ring_drain(re, t + 3);
+      ring_drain(ru, k + 2);
       cpa_wait0();
       return false;
     }
@@ -917,7 +931,7 @@ __device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw,
     // ---- mass (BODYH, calc.c:70-113), H relative to the row reference Hb(j)
     {
       float e0[8], u0[8], vm[4], v0[4], em[4], e1[4], e2[4];
-      E8(t, e0); U8(t, u0); V4(t - 1, vm); V4(t, v0);
+      E8(t, e0); U8(k + 1, u0); V4(k, vm); V4(k + 1, v0);
       E4(t - 1, em); E4(t + 1, e1); E4(t + 2, e2);
       const float kx = Qr(q, Q_KXE, j), ky = Qr(q, Q_KYN, j), hb = Qr(q, Q_HB, j), eref = Qr(q, Q_EREF, j);
       const float geo = Qr(q, Q_GEO, j), dm1 = Qr(q, Q_DHBM1, j), dp1 = Qr(q, Q_DHBP1, j), dp2 = Qr(q, Q_DHBP2, j);
@@ -925,7 +939,7 @@ __device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw,
 #pragma unroll
       for (int m = 0; m < 5; m++) fx[m] = face1<SCH>(e0[m], e0[m + 1], e0[m + 2], e0[m + 3], u0[m + 1] * kx);
       float eraw[4];
-      if constexpr (EXTRA) own4(rg.row(t, FE), eraw);
+      if constexpr (EXTRA) own4(re.row(t, FE), eraw);
       float damp[4] = {sig2dt, sig2dt, sig2dt, sig2dt};  // 2*Dt*sigma; per cell with a cap's sponge
       if constexpr (POLAR) arr(ld4f(d.pf + PQ_SH2 * PR, P, ib, j), damp);
       float hist[4], esn[4];
@@ -952,8 +966,100 @@ __device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw,
       put4<IMG_ETA, 1>(eta_out, W, nx, ny, ib, j, en);
       put4<IMG_ETA, 3>(es_out, P, nx, ny, ib, j, esn);
     }
-    section();
+  }
+  ring_end(re);
+  ring_end(ru);
+  cpa_wait0();
+  flush_checks(d, vw, 0.f, 0.f, oor);
+  return true;
+}
 
+template <int SCH, bool EXTRA, bool POLAR>
+__device__ __forceinline__ bool strip_momentum(const MemberDesc& d, const View& vw, int sx, int sy, int SR,
+                                               RingVel<EXTRA>& rg, RingLap& rl, bool test) {
+  enum { FU, FV, FWX, FWY };
+  const int nx = d.nx, ny = d.ny, P = d.P;
+  const float* q = d.q;
+  const int i0 = sx * SW + 1, j0 = sy * SR + 1, j1 = min(j0 + SR - 1, ny);
+  const int ib = i0 + 4 * lane_id();
+  int* bad = d.bad + vw.slot;
+  rg.map[FU] = map_of(d, TM_US + vw.cur);
+  rg.map[FV] = map_of(d, TM_VS + vw.cur);
+  if constexpr (EXTRA) {
+    rg.map[FWX] = map_of(d, TM_WX);
+    rg.map[FWY] = map_of(d, TM_WY);
+  }
+  rg.x = sx * SW;
+  rg.y0 = j0 - 1;  // tensor row of j0 - 2
+  rg.T = j1 - j0 + 5;
+  rl.map[0] = map_of(d, TM_LU);
+  rl.map[1] = map_of(d, TM_LV);
+  rl.x = sx * SW;
+  rl.y0 = j0;  // tensor row of j0 - 1
+  rl.T = j1 - j0 + 3;
+  ring_begin(rg);
+  ring_begin(rl);
+  for (int t = 0; t < 4; t++)
+    if (!ring_wait(rg, t, bad)) {
+      ring_drain(rl, 0);
+      return false;
+    }
+  if (!ring_wait(rl, 0, bad) || !ring_wait(rl, 1, bad) || (test && !ring_test(rg, d.tile_test, bad))) {
+    ring_drain(rg, 4);
+    ring_drain(rl, 2);
+    return false;
+  }
+
+  auto U8 = [&](int t, float (&w)[8]) {
+    win8(rg.row(t, FU), w);
+    if constexpr (EXTRA) { float x[8]; win8(rg.row(t, FWX), x); addw(w, x, 1.f); }
+  };
+  auto U4 = [&](int t, float (&w)[4]) {
+    own4(rg.row(t, FU), w);
+    if constexpr (EXTRA) { float x[4]; own4(rg.row(t, FWX), x); addw(w, x, 1.f); }
+  };
+  auto V8 = [&](int t, float (&w)[8]) {
+    win8(rg.row(t, FV), w);
+    if constexpr (EXTRA) { float x[8]; win8(rg.row(t, FWY), x); addw(w, x, 1.f); }
+  };
+  auto V4 = [&](int t, float (&w)[4]) {
+    own4(rg.row(t, FV), w);
+    if constexpr (EXTRA) { float x[4]; own4(rg.row(t, FWY), x); addw(w, x, 1.f); }
+  };
+
+  // carried from row to row: the limited slopes of the y faces south of the
+  // row, ZE of the row below and DI of the row
+  float2 ysu[4], ysv[4];
+  float zm[4], dj[5];
+  {
+    float a[4], b[4], cc[4], dd[4];
+    U4(0, a); U4(1, b); U4(2, cc); U4(3, dd);
+#pragma unroll
+    for (int c = 0; c < 4; c++) ysu[c] = face2_shared<SCH>(a[c], b[c], cc[c], dd[c]);
+    V4(0, a); V4(1, b); V4(2, cc); V4(3, dd);
+#pragma unroll
+    for (int c = 0; c < 4; c++) ysv[c] = face2_shared<SCH>(a[c], b[c], cc[c], dd[c]);
+    float la[8], lb[8], ma[8], mb[8], zt[5];
+    win8(rl.row(0, 0), la); win8(rl.row(1, 0), lb);
+    win8(rl.row(0, 1), ma); win8(rl.row(1, 1), mb);
+    ze5<POLAR>(q, nx, ny, P, ib, j0 - 1, la, lb, ma, d.Lu, d.Lv, zt);
+#pragma unroll
+    for (int c = 0; c < 4; c++) zm[c] = zt[c + 1];
+    di5<POLAR>(q, nx, ny, P, ib, j0, lb, mb, ma, la, d.Lu, d.Lv, dj);
+  }
+  const float sigdt = d.sigdt, nu2dt = d.nu2dt, nu4dt = d.nu4dt;
+  const bool keep_ll = (d.nu6dt != 0.f);
+  const int PR = P * (ny + 4);  // stride of a cap's per-cell fields
+  float mxu = 0.f, mxv = 0.f;
+  for (int j = j0; j <= j1; j++) {
+    const int k = j - j0, t = k + 2;  // ring row of j (the Laplacian ring: k + 1)
+    ring_refill(rg, k);
+    ring_refill(rl, k);
+    if (!ring_wait(rg, t + 2, bad) || !ring_wait(rl, k + 2, bad)) {
+      ring_drain(rg, t + 3);
+      ring_drain(rl, k + 3);
+      return false;
+    }
     // ---- second Laplacian level of (u, v) from L (laplacian.c:51-111),
     // and the hyperviscosity terms nu2*Dt*L + nu4*Dt*LL of both tendencies
     float visu[4], visv[4];
@@ -1045,8 +1151,7 @@ __device__ __forceinline__ bool strip_main1(const MemberDesc& d, const View& vw,
   }
   ring_end(rg);
   ring_end(rl);
-  cpa_wait0();
-  flush_checks(d, vw, mxu, mxv, oor);
+  flush_checks(d, vw, mxu, mxv, false);
   return true;
 }
 
@@ -1428,27 +1533,41 @@ __global__ void __launch_bounds__(NT) kb_tracer(SW2G_KPARAMS) {
                   (!d.trd || strip_tracer<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, test)))
 }
 
+// Momentum strips, then mass strips (see strip_mass); nstrips counts both. In
+// turn instead, warps of both kinds side by side, 0.245 ms at 4096x2048
+// against 0.200; 6 blocks (80 registers) 0.214.
 template <int SCH, bool EXTRA, int N, bool POLAR = false>
-__global__ void __launch_bounds__(NT, EXTRA ? 2 : 3) kb_main1(SW2G_KPARAMS) {
+__global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS) {
   extern __shared__ __align__(128) unsigned char sm[];
-  Ring<main1_fields<EXTRA>(), kDMain1> rg;
-  Ring<2, kDLapIn> rl;
+  RingEta<EXTRA> re;
+  RingFlow<EXTRA> ru;
+  RingVel<EXTRA> rg;
+  RingLap rl;
   unsigned char* a = smem_base(sm);
-  ring_init_at(a, 0, main1_bars<EXTRA>(), rg);
-  ring_init_at(a, NWARP * kDMain1 * 8, main1_lrows<EXTRA>(), rl);
-  const unsigned stg = smem_u32(a + main1_stage<EXTRA>() + (threadIdx.x >> 5) * kStageMain1);
+  const int w = threadIdx.x >> 5;
+  unsigned char* area = a + kBarsMain1 + w * main1_area<EXTRA>();
+  unsigned char* bars = a + w * (2 * kDMain1 + 2 * kDNear) * 8;
+  ring_place(bars, area, re);
+  ring_place(bars + kDMain1 * 8, area + kDMain1 * (EXTRA ? 2 : 1) * RS * 4, ru);
+  ring_place(bars + (kDMain1 + kDNear) * 8, area, rg);
+  ring_place(bars + (2 * kDMain1 + kDNear) * 8, area + kDMain1 * (EXTRA ? 4 : 2) * RS * 4, rl);
+  const unsigned stg = smem_u32(area + main1_mass<EXTRA>());
   pdl_entry();
   const int n = *counter;
   bool first = true;
   for (;;) {
     const int s = take_strip(queue);
     if (s >= nstrips) break;
-    const int4 tl = strip_at<N>(tiles, s, nbx);
+    const int half = nstrips >> 1;
+    const bool momentum = s < half;
+    const int4 tl = strip_at<N>(tiles, momentum ? s : s - half, nbx);
     const MemberDesc& d = ds.m[N == 1 ? 0 : tl.x];
     const View v = view_of(d, n);
     const bool test = first && d.tile_test > 0;
     first = false;
-    if (!strip_main1<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, rl, stg, test)) break;
+    const bool ok = momentum ? strip_momentum<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, rl, test)
+                            : strip_mass<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, re, ru, stg, test);
+    if (!ok) break;
   }
   warp_done(queue);
 }
@@ -1467,7 +1586,7 @@ constexpr int smem_bytes() {
 constexpr int kSmemLap = smem_bytes<2, kDLap>();
 constexpr int kSmemMain2 = smem_bytes<3, kDMain2>();
 template <bool EX>
-constexpr int smem_main1() { return 128 + main1_stage<EX>() + NWARP * kStageMain1; }
+constexpr int smem_main1() { return 128 + kBarsMain1 + NWARP * main1_area<EX>(); }
 template <bool EX>
 constexpr int smem_tracer() { return smem_bytes<EX ? 5 : 3, kDMain1>(); }
 
@@ -1519,23 +1638,44 @@ struct PdlLaunch {
   }
 };
 
+// Height of a single member's strips: cols strip columns (of all kinds) on
+// `slots` resident warps. A strip costs its rows and `lead` rows more (its first
+// rows and carried faces); the queue evens out the warps' speeds, which costs
+// about half a strip's time at the end when a warp takes several, and `one`
+// when each takes one (a quarter, or half with strips of two kinds). At 4096x2048: kb_lap1 18 rows (one strip a warp) 0.057
+// ms and 5 rows 0.050; kb_main2 27 and 7 rows 0.179 and 0.168; kb_main1 44, 22
+// and 11 rows 0.246, 0.212 and 0.200. At 1501x755, where strips are short, the
+// tracer's 5 rows (one strip a warp) 0.029 and 2 rows 0.036, kb_main1's 10 rows
+// 0.067 and 5 rows 0.058.
+inline int strip_height(int ny, int cols, int slots, double lead, double one) {
+  int best = 1;
+  double least = 0;
+  for (int sr = 1; sr <= 64; sr++) {
+    const double rounds = (double)cols * ((ny + sr - 1) / sr) / slots;
+    const double time = rounds + (rounds <= 1.0 ? one : 0.5);
+    const double cost = (sr + lead) * (time > 1.0 ? time : 1.0);
+    if (sr == 1 || cost < least) {
+      least = cost;
+      best = sr;
+    }
+  }
+  return best;
+}
+
 // One launch of kernel K over the strips: at most as many blocks as are
 // resident (the warps take the strips from the queue), under the named timer.
-// A single member's strips are as high as makes their number a whole
-// multiple (or just under) of the kernel's resident warps, so that no round
-// of strips runs on a few warps only: at 4096 x 2048 and 1824 resident warps,
-// 57 strip rows of 36 rows rather than 64 of 32 (2048 strips, the last 224 of
-// them running alone).
-template <auto K, int N>
+// KINDS: kinds of strips of the kernel, each covering the grid.
+template <auto K, int N, int KINDS = 1>
 void run_phase(const char* tag, int smem, const PhaseArgs<N>& a, int& nl) {
   if (a.tm && a.tm->on) a.tm->begin(tag, a.st);
   const int cap = grid_cap<K>(smem);
   int nstrips = a.nstrips, sr = a.sr;
   if constexpr (N == 1) {
-    const int slots = cap * NWARP, rows = slots / a.nbx > 0 ? slots / a.nbx : 1;
-    sr = (a.ny + rows - 1) / rows;
+        const int slots = cap * NWARP;
+    sr = strip_height(a.ny, a.nbx * KINDS, slots, KINDS > 1 ? 1.3 : 0.7, KINDS > 1 ? 0.5 : 0.25);
     nstrips = a.nbx * ((a.ny + sr - 1) / sr);
   }
+  nstrips *= KINDS;
   const int want = (nstrips + NWARP - 1) / NWARP;
   const PdlLaunch l(dim3(want < cap ? want : cap), dim3(NT), smem, a.st);
   cudaLaunchKernelEx(&l.cfg, K, *a.ds, a.tiles, nstrips, a.nbx, sr, (const int*)a.counter, a.queue);

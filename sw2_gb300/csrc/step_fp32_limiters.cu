@@ -14,12 +14,12 @@ template <int SCH, int N>
 void sch_main1(bool extra, bool polar, const PhaseArgs<N>& a, int& nl) {
   if constexpr (N == 1) {
     if (polar) {
-      run_phase<kb_main1<SCH, true, 1, true>, 1>("f32_main1", smem_main1<true>(), a, nl);
+      run_phase<kb_main1<SCH, true, 1, true>, 1, 2>("f32_main1", smem_main1<true>(), a, nl);
       return;
     }
   }
-  if (extra) run_phase<kb_main1<SCH, true, N>, N>("f32_main1", smem_main1<true>(), a, nl);
-  else run_phase<kb_main1<SCH, false, N>, N>("f32_main1", smem_main1<false>(), a, nl);
+  if (extra) run_phase<kb_main1<SCH, true, N>, N, 2>("f32_main1", smem_main1<true>(), a, nl);
+  else run_phase<kb_main1<SCH, false, N>, N, 2>("f32_main1", smem_main1<false>(), a, nl);
 }
 
 template <int SCH, int N>
