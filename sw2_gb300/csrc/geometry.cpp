@@ -68,8 +68,8 @@ bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows) {
   for (const auto& d : kSigDivisors)
     for (int j = 0; j <= c.ny + 1; j++)  // the rows a step divides by
       if (!positive_in_window(bits_of(rows[(size_t)d.row * H + (j + 1)]))) return false;
-  // the factors of the Laplacians and of their terms: 2^-255 .. 2^257, or zero where never used
-  auto mid = [](double x) { return (((uint32_t)(bits_of(x) >> 32) - 0x30000000u) & 0x60000000u) == 0; };
+  // the factors of the Laplacians and of their terms, where used: 2^-130 .. 2^250
+  auto mid = [](double x) { return std::fabs(x) >= 0x1p-130 && std::fabs(x) < 0x1p250; };
   for (int t : {R_KX, R_KY, R_KC})
     for (int j = 0; j <= c.ny + 1; j++)
       if (!mid(rows[(size_t)t * H + (j + 1)])) return false;

@@ -525,18 +525,20 @@ __device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j
 // the FP64 unit, out of line, otherwise. c: a factor that is finite and not
 // zero (a row constant or a coefficient): a zero times it is that zero.
 __device__ __forceinline__ bool mid(double x) { return ((hi_word(x) - 0x30000000u) & 0x60000000u) == 0; }
-// 2^-700 <= |x| < 2^257: times or over a factor of `mid` magnitude still normal
+// 2^-700 (2^-850) <= |x| < 2^257: times a factor of 2^-255 (2^-130) or more
+// still normal, and over a metric factor
 __device__ __forceinline__ bool wide(double x) { return hi_mag(x) - HI_POW2(-700) < (957u << 20); }
+__device__ __forceinline__ bool wider(double x) { return hi_mag(x) - HI_POW2(-850) < (1107u << 20); }
 __device__ __noinline__ double mul_fp64(double a, double b) { return a * b; }
 __device__ __forceinline__ double smul(double a, double b) {
   if (mid(a) && mid(b)) return from_bits(sig_mul(mag(a), mag(b)) | ((unsigned long long)(dbits(a) ^ dbits(b)) & kSign));
   return mul_fp64(a, b);
 }
-// s.sig_ok says that the row constants and hyperviscosity coefficients are in
-// that range; k: such a factor.
+// s.sig_ok says that the row constants and hyperviscosity coefficients are of
+// magnitude 2^-130 .. 2^250; k: such a factor.
 __device__ __forceinline__ double rmul(const DevState& s, double k, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(k)) & kSign;
-  if (wide(a) && s.sig_ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
+  if (wider(a) && s.sig_ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
   if (!nz(a)) return from_bits(sg);
   return mul_fp64(k, a);
 }
@@ -549,7 +551,7 @@ __device__ __forceinline__ double cmul(double c, double a) {
 __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
 // a / x.b (x.b > 0): a zero gives itself.
 __device__ __forceinline__ double mdiv(const DevState& s, double a, const Metric& x) {
-  if (wide(a) && s.sig_ok) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
+  if (wider(a) && s.sig_ok) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
   if (!nz(a)) return a;
   return div_fp64(a, from_bits(x.b));
 }
@@ -569,8 +571,11 @@ __device__ __forceinline__ double product_over(double a, double b, unsigned k20,
 }
 __device__ __forceinline__ double two_products(double a, double b, unsigned kx20, const Metric& X, double c,
                                                unsigned ky20, const Metric& Y) {
-  if (min(hi_mag(a) - 1, min(hi_mag(b) - 1, hi_mag(c) - 1)) < HI_POW2(-450) - 1)  // zeros wrap
+  if (min(hi_mag(a) - 1, min(hi_mag(b) - 1, hi_mag(c) - 1)) < HI_POW2(-450) - 1) {  // zeros wrap
+    // both products below 2^-1076: zeros, whose signs do not matter
+    if ((hi_mag(a) >> 20) + (max(hi_mag(b), hi_mag(c)) >> 20) < 969u) return 0.0;
     return two_products_fp64(a, scaled(b, kx20), from_bits(X.b), scaled(c, ky20), from_bits(Y.b));
+  }
   return product_over(a, b, kx20, X) + product_over(a, c, ky20, Y);
 }
 
