@@ -13,6 +13,8 @@
 // IEEE sums).
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "sigmath.cuh"
 #include "sw2g_internal.h"
 
@@ -818,24 +820,19 @@ __device__ __forceinline__ void strips_done(unsigned* q, int lane) {
     atomicExch(q + 1, 0u);
   }
 }
-#define FAST_SETUP                                                                          \
+#define STRIP_SETUP                                                                         \
   const int W = s.W, nx = s.nx, ny = s.ny;                                                  \
-  const int lane = threadIdx.x & 31;                                                        \
   const int FK = s.fk;                                                                      \
-  const int nsx = (nx + FW - 1) / FW, nstrips = nsx * ((ny + FK - 1) / FK);                  \
+  const int nsx = (nx + FW - 1) / FW;                                                       \
   const double Dt = s.Dt;                                                                   \
   const unsigned long long dt = (unsigned long long)dbits(Dt);                              \
-  for (int strip = next_strip(s.strips, lane); strip < nstrips; strip = next_strip(s.strips, lane)) { \
-    const int j0 = (strip / nsx) * FK + 1;                                                  \
-    const int jn = min(j0 + FK - 1, ny);                                                    \
-    const int base = (strip % nsx) * FW + 1;                                                \
-    const int i = base + lane;                                                              \
-    const int ic = min(i, nx + 2);                                                          \
-    const int ia = (lane == 0) ? base - 2 : (lane == 1) ? base - 1 : min(base + 32, nx + 2); \
-    const bool own = (lane < FW) && (i <= nx);
-#define FAST_END \
-  }                \
-  strips_done(s.strips, lane);
+  const int j0 = (strip / nsx) * FK + 1;                                                    \
+  const int jn = min(j0 + FK - 1, ny);                                                      \
+  const int base = (strip % nsx) * FW + 1;                                                  \
+  const int i = base + lane;                                                                \
+  const int ic = min(i, nx + 2);                                                            \
+  const int ia = (lane == 0) ? base - 2 : (lane == 1) ? base - 1 : min(base + 32, nx + 2);  \
+  const bool own = (lane < FW) && (i <= nx);
 // Field values of the fast bodies. PL (plain form): windx, windy and hB are
 // +0.0 everywhere, so x - hB = x exactly, and u + windx = u except that -0
 // becomes +0, which the fast path cannot tell apart (see (3) above).
@@ -845,9 +842,8 @@ __device__ __forceinline__ void strips_done(unsigned* q, int lane) {
 
 // BODYH + damping, fast form.
 template <int SCH, bool PL, bool UD>
-__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevState s, F7 f, double* out) {
-  SW2G_PDL_ENTRY();
-  FAST_SETUP
+__device__ __forceinline__ void mass_strip(const DevState& s, const F7& f, double* out, int strip, int lane) {
+  STRIP_SETUP
   const int iu = min(i - 1, nx + 2);
   const double damp = 2.0 * Dt * (s.sigma);  // calc.c:112: (2.0*Dt*sigma)*ETA
   // H at this lane's column, rows j and j+1, the differences of rows j-1 .. j+1,
@@ -900,14 +896,12 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_mass_fast(DevS
     dm = d0;
     d0 = d1;
   }
-  FAST_END
 }
 
 // BODYTRACER, fast form (calc.c:117-163).
 template <int SCH, bool PL>
-__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(DevState s, F7 f, double* out) {
-  SW2G_PDL_ENTRY();
-  FAST_SETUP
+__device__ __forceinline__ void tracer_strip(const DevState& s, const F7& f, double* out, int strip, int lane) {
+  STRIP_SETUP
   const int iu = min(i - 1, nx + 2);
   const double damp = 2.0 * Dt * (s.sigma_tr);  // calc.c:161
   double h2 = f.tr[IX(W, ic, j0)], h3 = f.tr[IX(W, ic, j0 + 1)], dm, d0;
@@ -957,14 +951,12 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_tracer_fast(De
     dm = d0;
     d0 = d1;
   }
-  FAST_END
 }
 
 // BODYU, fast form.
 template <int SCH, bool PL>
-__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(DevState s, F7 f, double* out) {
-  SW2G_PDL_ENTRY();
-  FAST_SETUP
+__device__ __forceinline__ void adv_u_strip(const DevState& s, const F7& f, double* out, int strip, int lane) {
+  STRIP_SETUP
   const int ic1 = min(i + 1, nx + 2);
   // U at this lane's column, rows j and j+1, the differences of rows j-1 .. j+1,
   // and the sum of V at columns i, i+1 of row j-1
@@ -1017,14 +1009,12 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_u_fast(Dev
     dm = d0;
     d0 = d1;
   }
-  FAST_END
 }
 
 // BODYV, fast form.
 template <int SCH, bool PL>
-__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(DevState s, F7 f, double* out) {
-  SW2G_PDL_ENTRY();
-  FAST_SETUP
+__device__ __forceinline__ void adv_v_strip(const DevState& s, const F7& f, double* out, int strip, int lane) {
+  STRIP_SETUP
   const int iu = min(i - 1, nx + 2);
   // V at this lane's column, rows j-1 .. j+1, the differences of rows j-1 ..
   // j+1; U at column i-1, row j
@@ -1079,10 +1069,33 @@ __global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS) k_adv_v_fast(Dev
     dm = d0;
     d0 = d1;
   }
-  FAST_END
 }
-#undef FAST_SETUP
-#undef FAST_END
+#undef STRIP_SETUP
+// The bodies of a step in one launch: the strips of each kind after those of
+// the one before, all from one queue. kinds: four bits each, lowest first.
+enum BodyKind { B_MASS, B_TRACER, B_ADV_U, B_ADV_V };
+struct Bodies {
+  double* out[4];  // by kind
+  unsigned kinds;
+  int n;  // how many kinds
+};
+template <int SCH, bool PL, bool UD>
+__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS)
+    k_bodies(const __grid_constant__ DevState s, const __grid_constant__ F7 f, const __grid_constant__ Bodies o) {
+  SW2G_PDL_ENTRY();
+  const int lane = threadIdx.x & 31;
+  const int per = (s.nx + FW - 1) / FW * ((s.ny + s.fk - 1) / s.fk), all = per * o.n;
+  for (int t = next_strip(s.strips, lane); t < all; t = next_strip(s.strips, lane)) {
+    const int k = t / per, strip = t - k * per;
+    switch ((o.kinds >> (4 * k)) & 15u) {
+      case B_MASS: mass_strip<SCH, PL, UD>(s, f, o.out[B_MASS], strip, lane); break;
+      case B_TRACER: tracer_strip<SCH, PL>(s, f, o.out[B_TRACER], strip, lane); break;
+      case B_ADV_U: adv_u_strip<SCH, PL>(s, f, o.out[B_ADV_U], strip, lane); break;
+      default: adv_v_strip<SCH, PL>(s, f, o.out[B_ADV_V], strip, lane); break;
+    }
+  }
+  strips_done(s.strips, lane);
+}
 #undef UF
 #undef VF
 #undef HF
@@ -1910,23 +1923,25 @@ __global__ void k_range(DevState s, RangeFields r, int* bad) {
 #undef VW
 #undef HH
 
-// Launch of a fast body. Its warps take strips of 31 columns x fk rows from
-// a queue (next_strip), and the grid is the blocks resident on the device at
-// once (or fewer when there are fewer strips). A strip costs its rows and
-// about one row more (the face south of its first row); the queue evens out
-// the warps' different speeds, and the last strips run with part of the warps
-// idle, about 0.3 of a strip's time on average. So the height is the one with
-// the least (fk + 1) * max(1, strips per resident warp + 0.3). Measured
-// (k_adv_u, 4256 resident warps): at 2048x1024 9 rows 0.123 ms and 17 rows,
-// one strip for each warp, 0.140; at 4096x2048 16 rows 0.480, 8 rows 0.492
-// and 32 rows 0.486; at 256x128, where every strip finds a warp, 1 row 0.014
-// and 4 rows 0.022 (with the timers' events).
-int choose_strip_rows(int nx, int ny, long long warps) {
+// Launch of the fast bodies. Warps take strips of 31 columns x fk rows of each
+// body from a queue (next_strip), and the grid is the blocks resident on the
+// device at once (or fewer when there are fewer strips). A strip costs its rows
+// and about one row more (the face south of its first row); the queue evens
+// out the warps' different speeds, and the end of the launch, with part of the
+// warps idle, costs about a strip's time (more in flows from rest, where the
+// cells that need the literal code lie together). So the height is the one
+// with the least (fk + 1) * max(1, strips per resident warp + 1.2). With 0.3,
+// 1.0 and 1.6 in place of 1.2: two forced steps from rest at 1024x512 2.41,
+// 2.03 and 1.93 ms; four steps of a 500x500 cap 0.830, 0.795 and 0.794; four
+// steps at 2048x1024 3.286, 3.290 and 3.318. One launch for the bodies in place
+// of three or four: a step at 256x128 88 -> 80 us, at 2048x1024 0.364 ms of
+// bodies -> 0.340.
+int choose_strip_rows(int nx, int ny, int kinds, long long warps) {
   int best = 1;
   double least = 0;
   for (int fk = 1; fk <= 24; fk++) {
-    const long long strips = (long long)((nx + FW - 1) / FW) * ((ny + fk - 1) / fk);
-    const double rounds = (double)strips / (double)warps + 0.3;
+    const long long strips = (long long)kinds * ((nx + FW - 1) / FW) * ((ny + fk - 1) / fk);
+    const double rounds = (double)strips / (double)warps + 1.2;
     const double cost = (fk + 1) * (rounds > 1.0 ? rounds : 1.0);
     if (fk == 1 || cost < least) {
       least = cost;
@@ -1936,58 +1951,67 @@ int choose_strip_rows(int nx, int ny, long long warps) {
   return best;
 }
 
-template <typename K>
-void fast_launch(K kernel, cudaStream_t st, const DevState& s0, const F7& f, double* out) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * FWARPS, 0);
-  const long long full = (long long)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
-  DevState s = s0;
-  s.fk = choose_strip_rows(s.nx, s.ny, full * FWARPS);
-  const long long strips = (long long)((s.nx + FW - 1) / FW) * ((s.ny + s.fk - 1) / s.fk);
-  const long long need = (strips + FWARPS - 1) / FWARPS;
-  pdl_launch(kernel, dim3((int)(need < full ? need : full)), dim3(32 * FWARPS), st, s, f, out);
+// The blocks of a kernel that are resident on the current device at once.
+constexpr int kMaxDevices = 64;
+template <auto K>
+long long resident_blocks() {
+  static std::atomic<int> cap[kMaxDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
+  int c = cap[dev].load(std::memory_order_relaxed);
+  if (!c) {
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, 32 * FWARPS, 0);
+    c = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+    cap[dev].store(c, std::memory_order_relaxed);
+  }
+  return c;
 }
 
+template <auto K>
+void launch_strips(cudaStream_t st, const DevState& s0, const F7& f, const Bodies& o) {
+  const long long full = resident_blocks<K>();
+  DevState s = s0;
+  s.fk = choose_strip_rows(s.nx, s.ny, o.n, full * FWARPS);
+  const long long strips = (long long)o.n * ((s.nx + FW - 1) / FW) * ((s.ny + s.fk - 1) / s.fk);
+  const long long need = (strips + FWARPS - 1) / FWARPS;
+  pdl_launch(K, dim3((int)(need < full ? need : full)), dim3(32 * FWARPS), st, s, f, o);
+}
+
+// One launch for all the bodies, or, for the literal kernels, one for each;
+// returns how many.
 template <int SCH>
-void launch_bodies(int which, dim3 g, cudaStream_t st, const DevState& s, const F7& f, double* out) {
+int launch_bodies(dim3 g, cudaStream_t st, const DevState& s, const F7& f, const Bodies& o) {
   if constexpr (SCH != 3) {
-    const bool ud = !s.polar && s.sigma == 0.0;
-    if (!s.sig_ok) {
-      // Dt or a metric factor outside the range of the integer-pipe quotients
-    } else if (s.plain) {
-      if (which == 0 && ud) { fast_launch(k_mass_fast<SCH, true, true>, st, s, f, out); return; }
-      if (which == 0) { fast_launch(k_mass_fast<SCH, true, false>, st, s, f, out); return; }
-      if (which == 1) { fast_launch(k_tracer_fast<SCH, true>, st, s, f, out); return; }
-      if (which == 2) { fast_launch(k_adv_u_fast<SCH, true>, st, s, f, out); return; }
-      if (which == 3) { fast_launch(k_adv_v_fast<SCH, true>, st, s, f, out); return; }
-    } else {
-      if (which == 0) { fast_launch(k_mass_fast<SCH, false, false>, st, s, f, out); return; }
-      if (which == 1) { fast_launch(k_tracer_fast<SCH, false>, st, s, f, out); return; }
-      if (which == 2) { fast_launch(k_adv_u_fast<SCH, false>, st, s, f, out); return; }
-      if (which == 3) { fast_launch(k_adv_v_fast<SCH, false>, st, s, f, out); return; }
+    if (s.sig_ok) {  // Dt and the metric factors in the range of the integer-pipe quotients
+      if (!s.plain) launch_strips<k_bodies<SCH, false, false>>(st, s, f, o);
+      else if (!s.polar && s.sigma == 0.0) launch_strips<k_bodies<SCH, true, true>>(st, s, f, o);
+      else launch_strips<k_bodies<SCH, true, false>>(st, s, f, o);
+      return 1;
     }
   }
-  if (which == 0) pdl_launch(k_mass<SCH>, dim3(g), dim3(TX), st, s, f, out);
-  else if (which == 1) pdl_launch(k_tracer<SCH>, dim3(g), dim3(TX), st, s, f, out);
-  else if (which == 2) pdl_launch(k_adv_u<SCH>, dim3(g), dim3(TX), st, s, f, out);
-  else pdl_launch(k_adv_v<SCH>, dim3(g), dim3(TX), st, s, f, out);
+  for (int k = 0; k < o.n; k++) {
+    const int kind = (o.kinds >> (4 * k)) & 15;
+    auto kernel = kind == B_MASS ? k_mass<SCH> : kind == B_TRACER ? k_tracer<SCH> : kind == B_ADV_U ? k_adv_u<SCH> : k_adv_v<SCH>;
+    pdl_launch(kernel, g, dim3(TX), st, s, f, o.out[kind]);
+  }
+  return o.n;
 }
 
-void body(int which, int sch, dim3 g, cudaStream_t st, const DevState& s, const F7& f, double* out) {
+int bodies(int sch, dim3 g, cudaStream_t st, const DevState& s, const F7& f, const Bodies& o) {
   switch (sch) {
-    case 0: launch_bodies<0>(which, g, st, s, f, out); break;
-    case 1: launch_bodies<1>(which, g, st, s, f, out); break;
-    case 2: launch_bodies<2>(which, g, st, s, f, out); break;
-    case 3: launch_bodies<3>(which, g, st, s, f, out); break;
-    case 4: launch_bodies<4>(which, g, st, s, f, out); break;
-    case 5: launch_bodies<5>(which, g, st, s, f, out); break;
-    case 6: launch_bodies<6>(which, g, st, s, f, out); break;
-    case 7: launch_bodies<7>(which, g, st, s, f, out); break;
-    case 8: launch_bodies<8>(which, g, st, s, f, out); break;
-    case 9: launch_bodies<9>(which, g, st, s, f, out); break;
-    default: launch_bodies<kVanLeerSafe>(which, g, st, s, f, out); break;
+    case 0: return launch_bodies<0>(g, st, s, f, o);
+    case 1: return launch_bodies<1>(g, st, s, f, o);
+    case 2: return launch_bodies<2>(g, st, s, f, o);
+    case 3: return launch_bodies<3>(g, st, s, f, o);
+    case 4: return launch_bodies<4>(g, st, s, f, o);
+    case 5: return launch_bodies<5>(g, st, s, f, o);
+    case 6: return launch_bodies<6>(g, st, s, f, o);
+    case 7: return launch_bodies<7>(g, st, s, f, o);
+    case 8: return launch_bodies<8>(g, st, s, f, o);
+    case 9: return launch_bodies<9>(g, st, s, f, o);
+    default: return launch_bodies<kVanLeerSafe>(g, st, s, f, o);
   }
 }
 
@@ -2130,10 +2154,24 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   // compute_Dt (core.c:155-159): maxima at the start of the step
   LAUNCH("cfl", pdl_launch(k_cfl, dim3(s.ny), dim3(CFL_T), st, s, F(), chk.cfl + 2 * slot));
 
-  // tracer (core.c:161-182); skipped while the tracer is identically +0, which
-  // the step then provably leaves unchanged
+  // The bodies of the tracer (core.c:161-182; skipped while the tracer is
+  // identically +0, which the step then provably leaves unchanged), of u and v
+  // (core.c:212-215) and of the mass (core.c:184-210; calc.c:289-355): they read
+  // old fields only, the longest first. A caller whose eta is still on its way
+  // in gets the mass body in a launch of its own behind that copy.
+  Bodies o{{b.deta[0], b.dtr[0], b.duadv, b.dvadv}, B_ADV_U | B_ADV_V << 4, 2};
+  auto add_kind = [&](unsigned k) { o.kinds |= k << (4 * o.n++); };
+  if (tracer) add_kind(B_TRACER);
+  if (!hk.eta_in) add_kind(B_MASS);
+  LAUNCH("bodies", nl += bodies(sch, g, st, s, F(), o) - 1);
+  if (hk.eta_in) {
+    cudaStreamWaitEvent(st, hk.eta_in, 0);
+    o.kinds = B_MASS;
+    o.n = 1;
+    LAUNCH("mass", bodies(sch, g, st, s, F(), o));
+  }
+
   if (tracer) {
-    LAUNCH("tracer", body(1, sch, g, st, s, F(), b.dtr[0]));
     if (k >= 2) {
       LAUNCH("tracer_ab3", pdl_launch(k_tracer_ab3, g, dim3(TX), st, s, b.f[3], b.dtr[0], b.dtr[1], b.dtr[2], fbad));
       rotate3(b.dtr);
@@ -2144,14 +2182,6 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
       LAUNCH("halo", halo_wrap(b.f[3], s.nx, s.ny, st));
     }
   }
-
-  // advection of u and v (core.c:212-215)
-  LAUNCH("adv_u", body(2, sch, g, st, s, F(), b.duadv));
-  LAUNCH("adv_v", body(3, sch, g, st, s, F(), b.dvadv));
-
-  // mass (core.c:184-210; calc.c:289-355)
-  if (hk.eta_in) cudaStreamWaitEvent(st, hk.eta_in, 0);
-  LAUNCH("mass", body(0, sch, g, st, s, F(), b.deta[0]));
   if (hyper) {
     if (!laplacians_first) eta_laplacians(last_in_eta ? nlap - 1 : nlap);
     if (k < 2) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
