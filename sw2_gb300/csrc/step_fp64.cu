@@ -1071,31 +1071,6 @@ __device__ __forceinline__ void adv_v_strip(const DevState& s, const F7& f, doub
   }
 }
 #undef STRIP_SETUP
-// The bodies of a step in one launch: the strips of each kind after those of
-// the one before, all from one queue. kinds: four bits each, lowest first.
-enum BodyKind { B_MASS, B_TRACER, B_ADV_U, B_ADV_V };
-struct Bodies {
-  double* out[4];  // by kind
-  unsigned kinds;
-  int n;  // how many kinds
-};
-template <int SCH, bool PL, bool UD>
-__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS)
-    k_bodies(const __grid_constant__ DevState s, const __grid_constant__ F7 f, const __grid_constant__ Bodies o) {
-  SW2G_PDL_ENTRY();
-  const int lane = threadIdx.x & 31;
-  const int per = (s.nx + FW - 1) / FW * ((s.ny + s.fk - 1) / s.fk), all = per * o.n;
-  for (int t = next_strip(s.strips, lane); t < all; t = next_strip(s.strips, lane)) {
-    const int k = t / per, strip = t - k * per;
-    switch ((o.kinds >> (4 * k)) & 15u) {
-      case B_MASS: mass_strip<SCH, PL, UD>(s, f, o.out[B_MASS], strip, lane); break;
-      case B_TRACER: tracer_strip<SCH, PL>(s, f, o.out[B_TRACER], strip, lane); break;
-      case B_ADV_U: adv_u_strip<SCH, PL>(s, f, o.out[B_ADV_U], strip, lane); break;
-      default: adv_v_strip<SCH, PL>(s, f, o.out[B_ADV_V], strip, lane); break;
-    }
-  }
-  strips_done(s.strips, lane);
-}
 #undef UF
 #undef VF
 #undef HF
@@ -1300,17 +1275,14 @@ struct LapEta {
   bool own;     // the lane's cell is one of the strip's
   double e0, xs;
   // rows from j0 on
-  __device__ __forceinline__ bool begin(const DevState& s, const double* e, int j0) {
-    const int W = s.W, lane = threadIdx.x & 31;
-    const int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * FW + 1;
+  __device__ __forceinline__ void begin(const DevState& s, const double* e, int base, int j0, int lane) {
+    const int W = s.W;
     c = base - 1 + lane;
     cc = min(c, s.nx);
     own = lane > 0 && c <= s.nx;
-    if (base > s.nx) return false;
     e0 = e[IX(W, cc, j0)];
     xs = 0.0;
     if (j0 > 1) xs = mdiv(s, rmul(s, RW(s, R_KY, j0 - 1), e0 - e[IX(W, cc, j0 - 1)]), METRIC(DYC, j0 - 1));
-    return true;
   }
   // the value at row j (warp-wide)
   __device__ __forceinline__ double next(const DevState& s, const double* e, int j) {
@@ -1327,16 +1299,25 @@ struct LapEta {
     return v;
   }
 };
-// One level, with its halo update and wall rows (laplacian.c:129-146).
-__global__ void __launch_bounds__(TX, 16) k_lape(DevState s, const double* e, double* eo, int rows) {
-  SW2G_PDL_ENTRY();
-  const int j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, s.ny);
+// One level, with its halo update and wall rows (laplacian.c:129-146): rows j0
+// to jn of the 31 columns from base on.
+__device__ __forceinline__ void lape_strip(const DevState& s, const double* e, double* eo, int base, int j0, int jn,
+                                           int lane) {
   LapEta L;
-  if (!L.begin(s, e, j0)) return;
+  L.begin(s, e, base, j0, lane);
   for (int j = j0; j <= jn; j++) {
     const double v = L.next(s, e, j);
     if (L.own) put_images<HK_LE>(s, eo, L.c, j, v);
   }
+}
+// The first of the columns of a warp of the marching kernels' blocks.
+__device__ __forceinline__ int march_base(int width) {
+  return (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * width + 1;
+}
+__global__ void __launch_bounds__(TX, 16) k_lape(DevState s, const double* e, double* eo, int rows) {
+  SW2G_PDL_ENTRY();
+  const int j0 = blockIdx.y * rows + 1, base = march_base(FW);
+  if (base <= s.nx) lape_strip(s, e, eo, base, j0, min(j0 + rows - 1, s.ny), threadIdx.x & 31);
 }
 
 // Deta_n += nu*Dt*L (calc.c:346-350); Du/Dv the same (core.c:258-266), with
@@ -1463,13 +1444,9 @@ __global__ void k_pres_sum(DevState s, F7 f, const double* duadv, const double* 
 // blocks 5 (117 registers), 8, 9 and 10: 0.089, 0.071, 0.072, 0.075 (at
 // 4096x2048 0.324, 0.243, 0.237, 0.235).
 constexpr int LVW = 30;
-__global__ void __launch_bounds__(TX, 9) k_lapv(DevState s, const double* uu, const double* vv, double* lu, double* lv,
-                                             int rows, bool images) {
-  SW2G_PDL_ENTRY();
-  const int W = s.W, nx = s.nx, ny = s.ny, lane = threadIdx.x & 31;
-  const int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * LVW + 1;
-  if (base > nx) return;
-  const int j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, ny);
+__device__ __forceinline__ void lapv_strip(const DevState& s, const double* uu, const double* vv, double* lu,
+                                           double* lv, bool images, int base, int j0, int jn, int lane) {
+  const int W = s.W, nx = s.nx, ny = s.ny;
   const int c = base - 1 + lane;
   const int sc = c == 0 ? nx : (c <= nx ? c : 1);  // where the column's ze and di are evaluated
   const bool own = lane > 0 && lane <= LVW && c <= nx;
@@ -1533,6 +1510,13 @@ __global__ void __launch_bounds__(TX, 9) k_lapv(DevState s, const double* uu, co
     d = dn;
     zs = z;
   }
+}
+
+__global__ void __launch_bounds__(TX, 9) k_lapv(DevState s, const double* uu, const double* vv, double* lu, double* lv,
+                                                int rows, bool images) {
+  SW2G_PDL_ENTRY();
+  const int j0 = blockIdx.y * rows + 1, base = march_base(LVW);
+  if (base <= s.nx) lapv_strip(s, uu, vv, lu, lv, images, base, j0, min(j0 + rows - 1, s.ny), threadIdx.x & 31);
 }
 
 // solve_Coriolis_u (calc.c:542-569), in place
@@ -1628,8 +1612,10 @@ __global__ void __launch_bounds__(TX, 16) k_eta_lap_ab3(DevState s, F7 f, double
   SW2G_PDL_ENTRY();
   constexpr int last = kLevels<NZ> - 1;
   const int W = s.W, j0 = blockIdx.y * rows + 1, jn = min(j0 + rows - 1, s.ny);
+  const int base = march_base(FW);
+  if (base > s.nx) return;
   LapEta L;
-  if (!L.begin(s, e, j0)) return;
+  L.begin(s, e, base, j0, threadIdx.x & 31);
   for (int j = j0; j <= jn; j++) {
     const double v = L.next(s, e, j);
     if (!L.own) continue;
@@ -1903,6 +1889,76 @@ __global__ void __launch_bounds__(CFL_T) k_cfl(DevState s, F7 f, unsigned long l
   }
 }
 
+// The maxima of rows j0 to jn on one warp (k_cfl otherwise).
+template <bool PL>
+__device__ __forceinline__ void cfl_rows(const DevState& s, const F7& f, unsigned long long* out, int j0, int jn,
+                                         int lane) {
+  const int W = s.W;
+  for (int j = j0; j <= jn; j++) {
+    long long bx = 0, by = 0;
+#pragma unroll 4
+    for (int i = lane + 1; i <= s.nx; i += 32) {
+      bx = max(bx, mag_bits(PL ? f.u[IX(W, i, j)] : UW(i, j)));
+      by = max(by, mag_bits(PL ? f.v[IX(W, i, j)] : VW(i, j)));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      bx = max(bx, __shfl_xor_sync(FULL, bx, o));
+      by = max(by, __shfl_xor_sync(FULL, by, o));
+    }
+    if (lane == 0) {
+      const double mx = div_rcp(__longlong_as_double(bx), RW(s, R_DXE, j), RW(s, R_IDXE, j));
+      const double my = div_rcp(__longlong_as_double(by), RW(s, R_DYN, j), RW(s, R_IDYN, j));
+      if (mx > 0) atomicMax(out, (unsigned long long)dbits(mx));
+      if (my > 0) atomicMax(out + 1, (unsigned long long)dbits(my));
+    }
+  }
+}
+
+// What a step computes from the old fields alone, in one launch: the CFL
+// maxima, the bodies, and the first levels of the hyperviscosity's Laplacians.
+// Every kind's strips are fk rows high; those of each kind follow those of the
+// one before, all from one queue. kinds: four bits each, lowest first.
+enum BodyKind { B_MASS, B_TRACER, B_ADV_U, B_ADV_V, B_LAPV, B_LAPE, B_CFL };
+struct Bodies {
+  double* out[4];  // of the bodies, by kind
+  const double* le_src;
+  double *Le, *Lu, *Lv;  // the Laplacians' first levels, of le_src and of (u, v)
+  bool images;           // a second level of the velocities reads the first
+  unsigned long long* cfl;
+  unsigned kinds;
+  int n;  // how many kinds
+};
+__host__ __device__ __forceinline__ int strip_columns(int kind, int nx) {
+  return kind == B_CFL ? 1 : kind == B_LAPV ? (nx + LVW - 1) / LVW : (nx + FW - 1) / FW;
+}
+template <int SCH, bool PL, bool UD>
+__global__ void __launch_bounds__(32 * FWARPS, FAST_MIN_BLOCKS)
+    k_bodies(const __grid_constant__ DevState s, const __grid_constant__ F7 f, const __grid_constant__ Bodies o) {
+  SW2G_PDL_ENTRY();
+  const int lane = threadIdx.x & 31, rows = (s.ny + s.fk - 1) / s.fk;
+  for (;;) {
+    int strip = next_strip(s.strips, lane), k = 0, kind = 0, cols = 0;
+    for (; k < o.n; k++) {
+      kind = (o.kinds >> (4 * k)) & 15u;
+      cols = strip_columns(kind, s.nx);
+      if (strip < cols * rows) break;
+      strip -= cols * rows;
+    }
+    if (k == o.n) break;
+    const int j0 = strip / cols * s.fk + 1, jn = min(j0 + s.fk - 1, s.ny), x = strip % cols;
+    switch (kind) {
+      case B_MASS: mass_strip<SCH, PL, UD>(s, f, o.out[B_MASS], strip, lane); break;
+      case B_TRACER: tracer_strip<SCH, PL>(s, f, o.out[B_TRACER], strip, lane); break;
+      case B_ADV_U: adv_u_strip<SCH, PL>(s, f, o.out[B_ADV_U], strip, lane); break;
+      case B_ADV_V: adv_v_strip<SCH, PL>(s, f, o.out[B_ADV_V], strip, lane); break;
+      case B_LAPV: lapv_strip(s, f.u, f.v, o.Lu, o.Lv, o.images, x * LVW + 1, j0, jn, lane); break;
+      case B_LAPE: lape_strip(s, o.le_src, o.Le, x * FW + 1, j0, jn, lane); break;
+      default: cfl_rows<PL>(s, f, o.cfl, j0, jn, lane); break;
+    }
+  }
+  strips_done(s.strips, lane);
+}
+
 struct RangeFields {
   const double* f[4];
   int n;
@@ -1936,11 +1992,11 @@ __global__ void k_range(DevState s, RangeFields r, int* bad) {
 // steps at 2048x1024 3.286, 3.290 and 3.318. One launch for the bodies in place
 // of three or four: a step at 256x128 88 -> 80 us, at 2048x1024 0.364 ms of
 // bodies -> 0.340.
-int choose_strip_rows(int nx, int ny, int kinds, long long warps) {
+int choose_strip_rows(int columns, int ny, long long warps) {
   int best = 1;
   double least = 0;
   for (int fk = 1; fk <= 24; fk++) {
-    const long long strips = (long long)kinds * ((nx + FW - 1) / FW) * ((ny + fk - 1) / fk);
+    const long long strips = (long long)columns * ((ny + fk - 1) / fk);
     const double rounds = (double)strips / (double)warps + 1.2;
     const double cost = (fk + 1) * (rounds > 1.0 ? rounds : 1.0);
     if (fk == 1 || cost < least) {
@@ -1973,8 +2029,10 @@ template <auto K>
 void launch_strips(cudaStream_t st, const DevState& s0, const F7& f, const Bodies& o) {
   const long long full = resident_blocks<K>();
   DevState s = s0;
-  s.fk = choose_strip_rows(s.nx, s.ny, o.n, full * FWARPS);
-  const long long strips = (long long)o.n * ((s.nx + FW - 1) / FW) * ((s.ny + s.fk - 1) / s.fk);
+  int columns = 0;
+  for (int k = 0; k < o.n; k++) columns += strip_columns((o.kinds >> (4 * k)) & 15, s.nx);
+  s.fk = choose_strip_rows(columns, s.ny, full * FWARPS);
+  const long long strips = (long long)columns * ((s.ny + s.fk - 1) / s.fk);
   const long long need = (strips + FWARPS - 1) / FWARPS;
   pdl_launch(K, dim3((int)(need < full ? need : full)), dim3(32 * FWARPS), st, s, f, o);
 }
@@ -1993,6 +2051,16 @@ int launch_bodies(dim3 g, cudaStream_t st, const DevState& s, const F7& f, const
   }
   for (int k = 0; k < o.n; k++) {
     const int kind = (o.kinds >> (4 * k)) & 15;
+    if (kind == B_CFL) {
+      pdl_launch(k_cfl, dim3(s.ny), dim3(CFL_T), st, s, f, o.cfl);
+      continue;
+    }
+    if (kind == B_LAPV || kind == B_LAPE) {
+      const March m = kind == B_LAPV ? march(s, LVW, 8) : march(s, FW, 4);
+      if (kind == B_LAPV) pdl_launch(k_lapv, m.grid, dim3(TX), st, s, f.u, f.v, o.Lu, o.Lv, m.rows, o.images);
+      else pdl_launch(k_lape, m.grid, dim3(TX), st, s, o.le_src, o.Le, m.rows);
+      continue;
+    }
     auto kernel = kind == B_MASS ? k_mass<SCH> : kind == B_TRACER ? k_tracer<SCH> : kind == B_ADV_U ? k_adv_u<SCH> : k_adv_v<SCH>;
     pdl_launch(kernel, g, dim3(TX), st, s, f, o.out[kind]);
   }
@@ -2135,9 +2203,9 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
     // the reference passes u, not eta (calc.c:332)
     return q > 0 ? b.Le[q - 1] : s.lape_eta ? b.f[0] : b.f[1];
   };
-  auto eta_laplacians = [&](int levels) {
+  auto eta_laplacians = [&](int first, int levels) {
     const March m = march(s, FW, 4);
-    for (int q = 0; q < levels; q++)
+    for (int q = first; q < levels; q++)
       LAUNCH("lape", pdl_launch(k_lape, m.grid, dim3(TX), st, s, lap_eta_source(q), b.Le[q], m.rows));
   };
   // Reading u alone, and nothing that the kernels before their place in the
@@ -2148,27 +2216,36 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   // From the third step the eta kernel computes the last level itself, except
   // where that level's source is eta, which the kernel changes.
   const bool last_in_eta = hyper && k >= 2 && !laplacians_first && !(s.lape_eta && nlap == 1);
-  if (laplacians_first) eta_laplacians(nlap);
+  if (laplacians_first) eta_laplacians(0, nlap);
   if (hk.v_in) cudaStreamWaitEvent(st, hk.v_in, 0);
 
-  // compute_Dt (core.c:155-159): maxima at the start of the step
-  LAUNCH("cfl", pdl_launch(k_cfl, dim3(s.ny), dim3(CFL_T), st, s, F(), chk.cfl + 2 * slot));
-
-  // The bodies of the tracer (core.c:161-182; skipped while the tracer is
-  // identically +0, which the step then provably leaves unchanged), of u and v
-  // (core.c:212-215) and of the mass (core.c:184-210; calc.c:289-355): they read
-  // old fields only, the longest first. A caller whose eta is still on its way
-  // in gets the mass body in a launch of its own behind that copy.
-  Bodies o{{b.deta[0], b.dtr[0], b.duadv, b.dvadv}, B_ADV_U | B_ADV_V << 4, 2};
-  auto add_kind = [&](unsigned k) { o.kinds |= k << (4 * o.n++); };
+  // What reads old fields only, in one launch, the longest strips first: the
+  // maxima of compute_Dt at the start of the step (core.c:155-159); the bodies
+  // of u and v (core.c:212-215), of the tracer (core.c:161-182; skipped while
+  // the tracer is identically +0, which the step then provably leaves
+  // unchanged) and of the mass (core.c:184-210; calc.c:289-355); the first
+  // levels of the Laplacians. A caller whose eta is still on its way in gets
+  // what reads eta in a launch of its own behind that copy.
+  const int nle = laplacians_first ? 0 : last_in_eta ? nlap - 1 : nlap;  // eta levels in kernels of their own
+  Bodies o{{b.deta[0], b.dtr[0], b.duadv, b.dvadv}, nullptr, b.Le[0], b.L[0], b.L[1], nlap > 1, chk.cfl + 2 * slot, 0, 0};
+  auto add_kind = [&](unsigned kind) { o.kinds |= kind << (4 * o.n++); };
+  add_kind(B_CFL);
+  add_kind(B_ADV_U);
+  add_kind(B_ADV_V);
   if (tracer) add_kind(B_TRACER);
   if (!hk.eta_in) add_kind(B_MASS);
+  if (hyper) add_kind(B_LAPV);
+  if (nle > 0) {
+    o.le_src = lap_eta_source(0);
+    if (!hk.eta_in) add_kind(B_LAPE);
+  }
   LAUNCH("bodies", nl += bodies(sch, g, st, s, F(), o) - 1);
   if (hk.eta_in) {
     cudaStreamWaitEvent(st, hk.eta_in, 0);
     o.kinds = B_MASS;
     o.n = 1;
-    LAUNCH("mass", bodies(sch, g, st, s, F(), o));
+    if (nle > 0) add_kind(B_LAPE);
+    LAUNCH("mass", nl += bodies(sch, g, st, s, F(), o) - 1);
   }
 
   if (tracer) {
@@ -2183,7 +2260,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
     }
   }
   if (hyper) {
-    if (!laplacians_first) eta_laplacians(last_in_eta ? nlap - 1 : nlap);
+    if (!laplacians_first) eta_laplacians(1, nle);
     if (k < 2) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
   }
   if (k >= 2) {
@@ -2210,9 +2287,9 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
     // (interior, halo wraps, wall fixes), the last their interior, which is all
     // that is read of it; L of levels not run stay zero.
     const March m = march(s, LVW, 8);
-    for (int q = 0; q < nlap; q++)
-      LAUNCH("lapv", pdl_launch(k_lapv, m.grid, dim3(TX), st, s, q == 0 ? b.f[1] : b.L[2 * q - 2],
-                                q == 0 ? b.f[2] : b.L[2 * q - 1], b.L[2 * q], b.L[2 * q + 1], m.rows, q + 1 < nlap));
+    for (int q = 1; q < nlap; q++)
+      LAUNCH("lapv", pdl_launch(k_lapv, m.grid, dim3(TX), st, s, b.L[2 * q - 2], b.L[2 * q - 1], b.L[2 * q],
+                                b.L[2 * q + 1], m.rows, q + 1 < nlap));
     if (k < 2) {
       LAUNCH("hyper_add", hyper_add(s, g, st, b.du[0], b.L[0], b.L[2], b.L[4]));
       LAUNCH("hyper_add", hyper_add(s, g, st, b.dv[0], b.L[1], b.L[3], b.L[5]));
