@@ -156,20 +156,6 @@ int batch_step_n(int sch, int sr, const MemberDesc* desc, int nmem, const int4* 
     nu6 = nu6 || (desc[m].nu6dt != 0.f);
   }
   int nl = 0;
-  if (tracer) {  // reads the step's old u, v and tracer only (core.c:161-182)
-    switch (sch) {
-      case 0: sch_tracer<0, N>(extra, polar, a, nl); break;
-      case 1: sch_tracer<1, N>(extra, polar, a, nl); break;
-      case 2: sch_tracer<2, N>(extra, polar, a, nl); break;
-      case 4: sch_tracer<4, N>(extra, polar, a, nl); break;
-      case 5: sch_tracer<5, N>(extra, polar, a, nl); break;
-      case 6: sch_tracer<6, N>(extra, polar, a, nl); break;
-      case 7: sch_tracer<7, N>(extra, polar, a, nl); break;
-      case 8: sch_tracer<8, N>(extra, polar, a, nl); break;
-      case 9: sch_tracer<9, N>(extra, polar, a, nl); break;
-      default: sch_tracer<kVanLeerSafe, N>(extra, polar, a, nl); break;
-    }
-  }
   if constexpr (N == 1) {
     if (polar) run_phase<kb_lap1<1, true>, 1>("f32_lap1", kSmemLap, a, nl);
     else run_phase<kb_lap1<1>, 1>("f32_lap1", kSmemLap, a, nl);
@@ -177,16 +163,16 @@ int batch_step_n(int sch, int sr, const MemberDesc* desc, int nmem, const int4* 
     run_phase<kb_lap1<N>, N>("f32_lap1", kSmemLap, a, nl);
   }
   switch (sch) {  // the FP32 form runs Van Leer in its safe form (kVanLeerSafe)
-    case 0: sch_main1<0, N>(extra, polar, a, nl); break;
-    case 1: sch_main1<1, N>(extra, polar, a, nl); break;
-    case 2: sch_main1<2, N>(extra, polar, a, nl); break;
-    case 4: sch_main1<4, N>(extra, polar, a, nl); break;
-    case 5: sch_main1<5, N>(extra, polar, a, nl); break;
-    case 6: sch_main1<6, N>(extra, polar, a, nl); break;
-    case 7: sch_main1<7, N>(extra, polar, a, nl); break;
-    case 8: sch_main1<8, N>(extra, polar, a, nl); break;
-    case 9: sch_main1<9, N>(extra, polar, a, nl); break;
-    default: sch_main1<kVanLeerSafe, N>(extra, polar, a, nl); break;
+    case 0: sch_main1<0, N>(extra, polar, tracer, a, nl); break;
+    case 1: sch_main1<1, N>(extra, polar, tracer, a, nl); break;
+    case 2: sch_main1<2, N>(extra, polar, tracer, a, nl); break;
+    case 4: sch_main1<4, N>(extra, polar, tracer, a, nl); break;
+    case 5: sch_main1<5, N>(extra, polar, tracer, a, nl); break;
+    case 6: sch_main1<6, N>(extra, polar, tracer, a, nl); break;
+    case 7: sch_main1<7, N>(extra, polar, tracer, a, nl); break;
+    case 8: sch_main1<8, N>(extra, polar, tracer, a, nl); break;
+    case 9: sch_main1<9, N>(extra, polar, tracer, a, nl); break;
+    default: sch_main1<kVanLeerSafe, N>(extra, polar, tracer, a, nl); break;
   }
   if constexpr (N == 1) {
     if (nu6 && polar) run_phase<kb_lap3<1, true>, 1>("f32_lap3", kSmemLap, a, nl);

@@ -11,13 +11,13 @@
 //   * u, v are FP64; each step adds an FP32 increment to them in FP64;
 //   * the Adams-Bashforth histories and the intermediate fields are FP32.
 // Kernels of one step:
-//   kb_tracer: tracer advection, AB and update (calc.c:117-163, core.c:161-182),
-//              only for members with an active tracer;
 //   kb_lap1  : first Laplacian level of (u, v) (laplacian.c:51-111) -> L, with
 //              the reference's halo images and wall fixes;
 //   kb_main1 : mass sweep + AB + geofactor -> eta (calc.c:70-113, 403-422),
 //              second Laplacian level from L, momentum advection and
-//              dissipation -> partial tendencies, CFL maxima;
+//              dissipation -> partial tendencies, CFL maxima; for members
+//              with an active tracer its advection, AB and update
+//              (calc.c:117-163, core.c:161-182);
 //   kb_lap3  : third Laplacian level (nu6), added to the partial tendencies;
 //   kb_main2 : pressure, AB, semi-implicit Coriolis u then v (calc.c:500-598),
 //              halo images and do_channel (calc.c:600-649) of u and v.
@@ -62,7 +62,7 @@ constexpr int BOXW = SW + 8;     // staged row: columns i0-4 .. i0+SW+3
 constexpr int ROWB = BOXW * 4;   // bytes of one staged row
 constexpr int RS = 160;          // floats per ring slot row: 640 bytes, keeping every copy 128-byte aligned
 constexpr unsigned FULL = 0xffffffffu;
-// Ring depths (staged rows per warp): kb_main1 and kb_tracer read rows j-1..j+2
+// Ring depths (staged rows per warp): kb_main1's strips read rows j-1..j+2
 // for row j and prefetch one row; kb_main2 reads j..j+1 and prefetches two;
 // the Laplacian kernels, whose rows are short, prefetch three.
 constexpr int kDMain1 = 5, kDMain2 = 4, kDLap = 5;
@@ -399,6 +399,15 @@ __device__ __forceinline__ unsigned char* smem_base(unsigned char* sm) {
   return sm + ((128u - (smem_u32(sm) & 127u)) & 127u);
 }
 
+// Initialises n (<= 32) barriers of a warp, one for each lane (one arrival
+// each: the expect_tx of lane 0).
+__device__ __forceinline__ void bars_init(unsigned long long* bar, int n) {
+  if (lane_id() < n) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[lane_id()])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+}
 // Carves the warp's ring out of the block's dynamic shared memory (the
 // blocks' barriers of this ring at bar_off, their rows at row_off, both
 // byte offsets from smem_base) and initialises its barriers (one arrival
@@ -780,11 +789,16 @@ using RingFlow = Ring<EXTRA ? 4 : 2, kDNear>;
 template <bool EXTRA>
 using RingVel = Ring<EXTRA ? 4 : 2, kDMain1>;
 using RingLap = Ring<2, kDNear>;
-// Shared memory of a block: the barriers of the four rings of each warp, then
+// Tracer strips, of members with an active tracer: rows j0-2 .. j1+2 of the
+// tracer, u, v and the winds.
+template <bool EXTRA>
+using RingTracer = Ring<EXTRA ? 5 : 3, kDMain1>;
+// Shared memory of a block: the barriers of the five rings of each warp, then
 // for each warp an area that holds the rows of the kind of strip it works on.
 // own-cell staging of a mass strip: two rows of [eta (32 lanes x 4 doubles), h1, h2 (32 x 4 floats)]
 constexpr int kStageMain1 = 2 * 2048;
-constexpr int kBarsMain1 = (NWARP * (2 * kDMain1 + 2 * kDNear) * 8 + 127) / 128 * 128;
+constexpr int kWarpBarsMain1 = (3 * kDMain1 + 2 * kDNear) * 8;
+constexpr int kBarsMain1 = (NWARP * kWarpBarsMain1 + 127) / 128 * 128;
 template <bool EXTRA>
 __host__ __device__ constexpr int main1_mass() {  // rows of a mass strip, then its staging
   return (kDMain1 * (EXTRA ? 2 : 1) + kDNear * (EXTRA ? 4 : 2)) * RS * 4;
@@ -792,22 +806,17 @@ __host__ __device__ constexpr int main1_mass() {  // rows of a mass strip, then 
 template <bool EXTRA>
 __host__ __device__ constexpr int main1_area() {
   const int mass = main1_mass<EXTRA>() + kStageMain1, mom = (kDMain1 * (EXTRA ? 4 : 2) + kDNear * 2) * RS * 4;
-  return mass > mom ? mass : mom;
+  const int tracer = kDMain1 * (EXTRA ? 5 : 3) * RS * 4, most = mass > mom ? mass : mom;
+  return most > tracer ? most : tracer;
 }
 
-// A ring with its barriers at bar and its rows at buf (the warp's own).
+// A ring with its barriers (initialised) at bar and its rows at buf (the warp's own).
 template <int NF, int D>
 __device__ __forceinline__ void ring_place(unsigned char* bar, unsigned char* buf, Ring<NF, D>& r) {
   r.bar = reinterpret_cast<unsigned long long*>(bar);
   r.buf = reinterpret_cast<float*>(buf);
   r.base = 0;
   r.issued = 0;
-  if (lane_id() == 0) {
-    for (int s = 0; s < D; s++)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&r.bar[s])) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
 }
 
 // Sections of a row are separated by a compiler fence, so that windows are
@@ -1155,7 +1164,7 @@ __device__ __forceinline__ bool strip_momentum(const MemberDesc& d, const View& 
   return true;
 }
 
-// --------------------------------------------------------------- kb_tracer
+// ------------------------------------------------------ tracer strips
 // BODYTRACER (calc.c:117-163): TVD fluxes of the tracer on the four faces,
 // each with both split Courant numbers of its face velocity (winds
 // included), the compression term and the damping -2*Dt*TracerDis*T; then the
@@ -1164,7 +1173,7 @@ __device__ __forceinline__ bool strip_momentum(const MemberDesc& d, const View& 
 // tracer shadow, u and v (and the winds with EXTRA).
 template <int SCH, bool EXTRA, bool POLAR>
 __device__ __forceinline__ bool strip_tracer(const MemberDesc& d, const View& vw, int sx, int sy, int SR,
-                                             Ring<EXTRA ? 5 : 3, kDMain1>& rg, bool test) {
+                                             RingTracer<EXTRA>& rg, bool test) {
   enum { FT, FU, FV, FWX, FWY };
   const TracerDesc& td = *d.trd;
   const int nx = d.nx, ny = d.ny, P = d.P, W = nx + 4;
@@ -1526,18 +1535,15 @@ __global__ void __launch_bounds__(NT, 6) kb_lap3(SW2G_KPARAMS) {
   SW2G_STRIP_LOOP(2, kDLap, (d.nu6dt == 0.f || strip_lap<true, POLAR>(d, v, tl.y, tl.z, SR, rg, test)))
 }
 
-// Tracer advection: members without an active tracer skip their strips.
+// Momentum strips, then mass strips (see strip_mass), then, if a member has an
+// active tracer, tracer strips: `per` of each kind, nstrips in all. In turn
+// instead, warps of both kinds side by side, 0.245 ms at 4096x2048
+// against 0.200; 6 blocks (80 registers) 0.214. The tracer's strips come last:
+// they fill the launch's tail, which a launch of their own has once more (four
+// steps at 1501x1001 with winds and a tracer 0.610 and 0.590 ms, 320x320 caps
+// 0.360 and 0.339).
 template <int SCH, bool EXTRA, int N, bool POLAR = false>
-__global__ void __launch_bounds__(NT) kb_tracer(SW2G_KPARAMS) {
-  SW2G_STRIP_LOOP(EXTRA ? 5 : 3, kDMain1,
-                  (!d.trd || strip_tracer<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, test)))
-}
-
-// Momentum strips, then mass strips (see strip_mass); nstrips counts both. In
-// turn instead, warps of both kinds side by side, 0.245 ms at 4096x2048
-// against 0.200; 6 blocks (80 registers) 0.214.
-template <int SCH, bool EXTRA, int N, bool POLAR = false>
-__global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS) {
+__global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS, int per) {
   extern __shared__ __align__(128) unsigned char sm[];
   RingEta<EXTRA> re;
   RingFlow<EXTRA> ru;
@@ -1546,11 +1552,14 @@ __global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS) {
   unsigned char* a = smem_base(sm);
   const int w = threadIdx.x >> 5;
   unsigned char* area = a + kBarsMain1 + w * main1_area<EXTRA>();
-  unsigned char* bars = a + w * (2 * kDMain1 + 2 * kDNear) * 8;
+  unsigned char* bars = a + w * kWarpBarsMain1;
+  bars_init(reinterpret_cast<unsigned long long*>(bars), kWarpBarsMain1 / 8);
   ring_place(bars, area, re);
   ring_place(bars + kDMain1 * 8, area + kDMain1 * (EXTRA ? 2 : 1) * RS * 4, ru);
   ring_place(bars + (kDMain1 + kDNear) * 8, area, rg);
   ring_place(bars + (2 * kDMain1 + kDNear) * 8, area + kDMain1 * (EXTRA ? 4 : 2) * RS * 4, rl);
+  RingTracer<EXTRA> rt;
+  ring_place(bars + (2 * kDMain1 + 2 * kDNear) * 8, area, rt);
   const unsigned stg = smem_u32(area + main1_mass<EXTRA>());
   pdl_entry();
   const int n = *counter;
@@ -1558,15 +1567,17 @@ __global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS) {
   for (;;) {
     const int s = take_strip(queue);
     if (s >= nstrips) break;
-    const int half = nstrips >> 1;
-    const bool momentum = s < half;
-    const int4 tl = strip_at<N>(tiles, momentum ? s : s - half, nbx);
+    const int kind = s / per;  // momentum, mass, tracer
+    const int4 tl = strip_at<N>(tiles, s - kind * per, nbx);
     const MemberDesc& d = ds.m[N == 1 ? 0 : tl.x];
     const View v = view_of(d, n);
+    if (kind == 2 && !d.trd) continue;  // a member without an active tracer
     const bool test = first && d.tile_test > 0;
     first = false;
-    const bool ok = momentum ? strip_momentum<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, rl, test)
-                            : strip_mass<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, re, ru, stg, test);
+    bool ok;
+    if (kind == 0) ok = strip_momentum<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rg, rl, test);
+    else if (kind == 1) ok = strip_mass<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, re, ru, stg, test);
+    else ok = strip_tracer<SCH, EXTRA, POLAR>(d, v, tl.y, tl.z, SR, rt, test);
     if (!ok) break;
   }
   warp_done(queue);
@@ -1587,8 +1598,6 @@ constexpr int kSmemLap = smem_bytes<2, kDLap>();
 constexpr int kSmemMain2 = smem_bytes<3, kDMain2>();
 template <bool EX>
 constexpr int smem_main1() { return 128 + kBarsMain1 + NWARP * main1_area<EX>(); }
-template <bool EX>
-constexpr int smem_tracer() { return smem_bytes<EX ? 5 : 3, kDMain1>(); }
 
 // Dynamic shared memory and the number of resident blocks of a kernel on the
 // current device (set once per device; fp32_prepare does it for every kernel
@@ -1664,32 +1673,33 @@ inline int strip_height(int ny, int cols, int slots, double lead, double one) {
 
 // One launch of kernel K over the strips: at most as many blocks as are
 // resident (the warps take the strips from the queue), under the named timer.
-// KINDS: kinds of strips of the kernel, each covering the grid.
-template <auto K, int N, int KINDS = 1>
-void run_phase(const char* tag, int smem, const PhaseArgs<N>& a, int& nl) {
+// kinds: kinds of strips of the kernel, each covering the grid (kb_main1, which
+// takes the number of strips of a kind as well).
+template <auto K, int N, bool KINDS = false>
+void run_phase(const char* tag, int smem, const PhaseArgs<N>& a, int& nl, int kinds = 1) {
   if (a.tm && a.tm->on) a.tm->begin(tag, a.st);
   const int cap = grid_cap<K>(smem);
   int nstrips = a.nstrips, sr = a.sr;
   if constexpr (N == 1) {
-        const int slots = cap * NWARP;
-    sr = strip_height(a.ny, a.nbx * KINDS, slots, KINDS > 1 ? 1.3 : 0.7, KINDS > 1 ? 0.5 : 0.25);
+    sr = strip_height(a.ny, a.nbx * kinds, cap * NWARP, kinds > 1 ? 1.3 : 0.7, kinds > 1 ? 0.5 : 0.25);
     nstrips = a.nbx * ((a.ny + sr - 1) / sr);
   }
-  nstrips *= KINDS;
+  const int per = nstrips;
+  nstrips *= kinds;
   const int want = (nstrips + NWARP - 1) / NWARP;
   const PdlLaunch l(dim3(want < cap ? want : cap), dim3(NT), smem, a.st);
-  cudaLaunchKernelEx(&l.cfg, K, *a.ds, a.tiles, nstrips, a.nbx, sr, (const int*)a.counter, a.queue);
+  const int* const counter = a.counter;
+  if constexpr (KINDS) cudaLaunchKernelEx(&l.cfg, K, *a.ds, a.tiles, nstrips, a.nbx, sr, counter, a.queue, per);
+  else cudaLaunchKernelEx(&l.cfg, K, *a.ds, a.tiles, nstrips, a.nbx, sr, counter, a.queue);
   if (a.tm && a.tm->on) a.tm->end(a.st);
   nl++;
 }
 
-// The limiter-dependent phases (mass and momentum sweeps, tracer), one
-// instantiation per limiter in step_fp32_limiters.cu.
+// The limiter-dependent phase (momentum, mass and, with an active tracer,
+// tracer sweeps), one instantiation per limiter in step_fp32_limiters.cu.
 // polar: a single polar-cap member (N = 1; its kernels always read the winds)
 template <int SCH, int N>
-void sch_main1(bool extra, bool polar, const PhaseArgs<N>& a, int& nl);
-template <int SCH, int N>
-void sch_tracer(bool extra, bool polar, const PhaseArgs<N>& a, int& nl);
+void sch_main1(bool extra, bool polar, bool tracer, const PhaseArgs<N>& a, int& nl);
 template <int SCH>
 void sch_prepare();
 
