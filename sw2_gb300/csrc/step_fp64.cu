@@ -1,16 +1,16 @@
-// Reference-exact FP64 step, in core.c's order (core.c:134-338). The first
-// two steps after an upload run one kernel per reference routine; from the
-// third (AB3) the tails of the tendencies are fused, the Laplacian passes
-// write their own halo images and wall fixes, and the range checks are made
-// by the kernels that write the state. Compiled with -fmad=false so that no
-// a*b+c is fused: every expression keeps the association of the reference
-// expression it restates, which makes the results bit-identical to the
-// reference's own single-rank run. Divisions by a per-row metric factor go
-// through div_rcp (the same IEEE quotient with fewer FP64 instructions),
-// scalings by powers of two, zero numerators and bit tests are answered on
-// the integer pipe, since GB300 executes FP64 at 2 lanes per SM per clock,
-// and so are some of the small kernels' additions (sadd, ssub: the same
-// IEEE sums).
+// Reference-exact FP64 step, in core.c's order (core.c:134-338) wherever the
+// order reaches a value. What reads old fields only (CFL maxima, TVD bodies,
+// first Laplacian levels) runs in one launch; the first two steps after an
+// upload then run one kernel per reference routine; from the third (AB3) the
+// tails of the tendencies are fused, the Laplacians write their own halo
+// images and wall fixes, and the range checks are made by the kernels that
+// write the state. Compiled with -fmad=false so that no a*b+c is fused: every
+// expression keeps the association of the reference expression it restates,
+// which makes the results bit-identical to the reference's own single-rank
+// run. GB300 executes FP64 at 2 lanes per SM per clock, so quotients, most
+// products, scalings by powers of two, zero numerators and comparisons are
+// answered on the integer pipe (sigmath.cuh: the same IEEE results), and the
+// FP64 unit keeps the additions.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -22,8 +22,6 @@ namespace sw2g {
 namespace {
 
 constexpr int TX = 128;
-
-
 
 __device__ __forceinline__ int IX(int W, int i, int j) { return (i + 1) + (j + 1) * W; }
 __device__ __forceinline__ double RW(const DevState& s, int t, int j) { return s.rows[t * s.H + j + 1]; }
@@ -127,19 +125,10 @@ __device__ __forceinline__ double div_rcp(double a, double b, double y) {
 // below the normal range) adds on the FP64 unit, out of line. fp64_check_add
 // compares sadd and ssub with the FP64 unit on random and edge-case operands.
 // An integer-pipe addition takes about a hundred instructions where the FP64
-// unit takes one, but GB300 issues 128 integer operations per SM and clock
-// against 2 FP64 lanes: the small kernels below are bound by the FP64 unit
-// with most issue slots idle, so moving some of their additions off it makes
-// them faster, up to the point where issue becomes the bound. Which additions
-// move was measured per kernel at 2048x1024 (CUDA-event times of each mix):
-// all of the Coriolis updates' and of the second velocity-Laplacian pass,
-// the two outer sums of the first pass, the final sum of the second
-// eta-Laplacian pass, the Adams-Bashforth and hyperviscosity sums, the two
-// tendency sums of k_pres_sum; in the TVD bodies only the four-face sum of a
-// cell and, in the mass body, the last sum of each side term (their 96
-// registers per thread leave too few warps to hide longer chains: more
-// integer-pipe additions there made them slower); none in the first
-// eta-Laplacian pass (no gain).
+// unit takes one: it pays only in a kernel whose FP64 work leaves most issue
+// slots idle, as the Coriolis updates of the first two steps do (0.139 ->
+// 0.105 ms each at 2048x1024). Where products and quotients already take the
+// integer pipe (all other kernels) additions stay on the FP64 unit.
 __device__ __noinline__ double add_fp64(double a, double b) { return a + b; }
 __device__ __forceinline__ double sadd(double a, double b) {
   constexpr unsigned long long MAG = 0x7fffffffffffffffULL, FRAC = 0x000fffffffffffffULL, ONE = 1ULL << 52;
@@ -454,7 +443,6 @@ constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the 
 // 0.124 and 0.125 ms.
 #define FAST_MIN_BLOCKS 7
 constexpr unsigned FULL = 0xffffffffu;
-
 
 // Comparisons on the integer pipe (GB300 issues FP64 compares on its narrow
 // FP64 unit). For finite values they agree with the IEEE comparisons except
@@ -2061,7 +2049,10 @@ int launch_bodies(dim3 g, cudaStream_t st, const DevState& s, const F7& f, const
       else pdl_launch(k_lape, m.grid, dim3(TX), st, s, o.le_src, o.Le, m.rows);
       continue;
     }
-    auto kernel = kind == B_MASS ? k_mass<SCH> : kind == B_TRACER ? k_tracer<SCH> : kind == B_ADV_U ? k_adv_u<SCH> : k_adv_v<SCH>;
+    auto kernel = kind == B_MASS     ? k_mass<SCH>
+                  : kind == B_TRACER ? k_tracer<SCH>
+                  : kind == B_ADV_U  ? k_adv_u<SCH>
+                                     : k_adv_v<SCH>;
     pdl_launch(kernel, g, dim3(TX), st, s, f, o.out[kind]);
   }
   return o.n;
@@ -2264,7 +2255,8 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
     if (k < 2) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
   }
   if (k >= 2) {
-    LAUNCH("eta_ab3", fused_tail(s, g, st, F(), b, 0, fbad, last_in_eta ? lap_eta_source(nlap - 1) : nullptr));  // writes eta's halo images too
+    // writes eta's halo images too
+    LAUNCH("eta_ab3", fused_tail(s, g, st, F(), b, 0, fbad, last_in_eta ? lap_eta_source(nlap - 1) : nullptr));
     rotate3(b.deta);
   } else {
     LAUNCH("ab", pdl_launch(k_ab, dim3(g), dim3(TX), st, s, k, b.detaAB, b.deta[0], b.deta[1], b.deta[2]));
@@ -2275,13 +2267,11 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   }
   if (hk.eta_out) cudaEventRecord(hk.eta_out, st);  // eta is final for this step
 
-  // momentum (core.c:212-280)
-  // (from the third step in the Coriolis kernels)
-  if (k >= 2) {
-  } else if (s.polar == 0 && s.sigma == 0.0)
-    LAUNCH("pres_sum", pdl_launch(k_pres_sum<true>, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
-  else
-    LAUNCH("pres_sum", pdl_launch(k_pres_sum<false>, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
+  // momentum (core.c:212-280), from the third step in the Coriolis kernels
+  if (k < 2) {
+    auto pres_sum = s.polar == 0 && s.sigma == 0.0 ? k_pres_sum<true> : k_pres_sum<false>;
+    LAUNCH("pres_sum", pdl_launch(pres_sum, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
+  }
   if (hyper) {
     // As above: each level but the last rewrites every cell of its two L fields
     // (interior, halo wraps, wall fixes), the last their interior, which is all
@@ -2328,7 +2318,8 @@ int step_tail(const DevState& s, Fp64Buffers& b, bool tracer, StepChecks chk, in
   const dim3 g((s.nx + TX - 1) / TX, s.ny);
   const int gw = (s.nx + 127) / 128;
   int nl = 0;
-  if (whole) LAUNCH("halo_channel", pdl_launch(k_halo_channel, dim3((s.nx + 4 * (s.ny - 1) + 1 + 127) / 128), dim3(128), st, s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5], s.plain == 0));
+  if (whole) LAUNCH("halo_channel", pdl_launch(k_halo_channel, dim3((s.nx + 4 * (s.ny - 1) + 1 + 127) / 128), dim3(128), st,
+                                               s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5], s.plain == 0));
   else if (s.polar == 0) LAUNCH("channel", pdl_launch(k_channel, dim3(gw), dim3(128), st, s.nx, s.ny, b.f[1], b.f[2], b.f[4], b.f[5]));
 
   // range checks of tracer, eta, u, v (core.c:309-312); an all-zero tracer

@@ -32,7 +32,7 @@ enum Row {
   R_DXE2,  // DXE+DXE                      calc.c:197
   R_DYNS,  // DYN(j)+DYN(j+1)              calc.c:234
   R_SURF,  // DXC*DYC                      energy.c:40
-  R_IDYV, R_IDXE2, R_IDYNS, R_IRZC, R_IRZN,  // 1.0/x of DYV, DXE2, DYNS, rZ(latc), rZ(latn): divisors of div_rcp
+  R_IRZC, R_IRZN,  // 1.0/x of rZ(latc), rZ(latn), and, with those above, of the divisors of div_rcp
   // 64-bit reciprocals (sig_recip, the integer's bits) of the divisors on the integer pipe
   R_YDXE, R_YDXC, R_YDXV, R_YDYN, R_YDYC, R_YDYV, R_YDXE2, R_YDYNS, R_YRZC, R_YRZN,
   R_NUM
