@@ -46,22 +46,21 @@ UNIT = "cell-updates/s"
 # the fields a kernel must read and write at least once (8 B each; winds and
 # bottom height are zero in these workloads and are not counted).
 KERNEL_BYTES = {
-    "mass": 8 * (3 + 1),        # eta u v -> Deta
-    "adv_u": 8 * (2 + 1),       # u v -> Du_adv
-    "adv_v": 8 * (2 + 1),       # u v -> Dv_adv
+    # eta u v -> Deta Du_adv Dv_adv, nu4's first levels Lu Lv Le
+    "bodies": 8 * (3 + 6),
+    "mass": 8 * (3 + 1),        # eta u v -> Deta, in a launch of its own (host-array steps)
     "pres_sum": 8 * (5 + 2),    # eta u v Du_adv Dv_adv -> Du_n Dv_n
     "ab": 8 * (3 + 1),
-    "coriolis_u": 8 * (6 + 2),  # from the third step: u v, D_n D_n-1 D_n-2, nu4 L -> D_n u (AB3 fused)
-    "coriolis_v": 8 * (6 + 2),
-    "eta_ab3": 8 * (6 + 2),     # eta v, D_n D_n-1 D_n-2, nu4 L -> D_n eta (hyper, AB3, geofactor, update)
-    "lape_pass1": 8 * (1 + 2),
-    "lape_pass2": 8 * (2 + 1),
-    "lapv_pass1": 8 * (2 + 2),
-    "lapv_pass2": 8 * (2 + 2),
+    # from the third step: eta u v, D_adv, D_n-1 D_n-2, two nu4 levels -> D_n u (pressure, AB3 and update fused)
+    "coriolis_u": 8 * (8 + 2),
+    "coriolis_v": 8 * (8 + 2),
+    "eta_ab3": 8 * (6 + 2),     # eta v, D_n D_n-1 D_n-2, Le -> D_n eta (last level, AB3, geofactor, update)
+    "tracer_ab3": 8 * (4 + 1),  # tracer, D_n D_n-1 D_n-2 -> tracer
+    "lape": 8 * (1 + 1),
+    "lapv": 8 * (2 + 2),
     "hyper_add": 8 * (4 + 1),
     "geofactor": 8 * (3 + 1),
     "add": 8 * (2 + 1),
-    "cfl": 8 * 2,
     "range": 8 * 1,
     # FP32 form: FP64 state (8 B), FP32 shadows of the state, histories and
     # intermediates (4 B)
@@ -71,22 +70,20 @@ KERNEL_BYTES = {
     # new eta shadow, u v, their shadows, partials, 4 hist -> u v + shadows, 2 hist
     "f32_main2": 4 + 8 * 2 + 4 * 2 + 4 * 2 + 4 * 4 + 8 * 2 + 4 * 2 + 4 * 2,
     "f32_lap3": 4 * 2 + 4 * 2 + 4 * 2,  # LLu LLv, partials -> partials
-    "f32_tracer": 4 * 3 + 8 + 4 * 2 + 8 + 4 + 4,  # tracer u v shadows, tracer, 2 hist -> tracer + shadow, hist
 }
 # DRAM bytes (read + write) of one launch of the dominant kernels on the
 # 2048x1024 workload, from an ncu capture of the same step (third step, one
-# launch each, the current kernels). With zero winds the plain bodies read eta
-# or u and v only; part of each input is still in L2 from the kernel before,
-# and most of the output leaves L2 later, so DRAM bytes are below the
-# algorithmic bytes.
-NCU_TRAFFIC = {("band2048", "mass"): 52.60e6, ("band2048", "adv_u"): 34.18e6, ("band2048", "adv_v"): 34.26e6}
-# FP64 thread instructions (DADD + DMUL + DFMA) per interior cell of the
-# dominant kernels on the 2048x1024 workload, from ncu's instruction counters
+# launch each, the current kernels). Part of each input is still in L2 from the
+# kernel before, and most of the output leaves L2 later, so DRAM bytes are
+# below the algorithmic bytes.
+NCU_TRAFFIC = {("band2048", "bodies"): 121e6}
+# FP64 instructions per interior cell (warp instructions x 32) of the
+# dominant kernel on the 2048x1024 workload, from ncu's instruction counters
 # of the same capture, and the FP64 unit's busy fraction there; GB300's FP64
 # peak per cycle over the whole GPU (ncu's peak for DFMA: 304 = 2 lanes per SM
 # x 152 SMs). The FP64 form is bound by this unit.
-NCU_FP64_PER_CELL = {("band2048", "mass"): 52.5, ("band2048", "adv_u"): 68.8, ("band2048", "adv_v"): 69.2}
-NCU_FP64_PIPE_BUSY = {("band2048", "mass"): 0.827, ("band2048", "adv_u"): 0.838, ("band2048", "adv_v"): 0.838}
+NCU_FP64_PER_CELL = {("band2048", "bodies"): 89.6}
+NCU_FP64_PIPE_BUSY = {("band2048", "bodies"): 0.717}
 FP64_LANES_PER_CYCLE = 304
 # The whole step: read eta u v, write eta u v, read two history levels of
 # three tendencies, write one (a per-cell count for the step's GB/s figure).
@@ -596,8 +593,8 @@ def main():
         fp64_roof = {"bound": "fp64", "kernel": m64["kernel"], "achieved": ach, "peak": pk,
                      "unit": "FP64 instr/s", "frac": ach / pk, "instr_per_cell": n64,
                      "pipe_busy_ncu": NCU_FP64_PIPE_BUSY.get((args.config, m64["kernel"])),
-                     "peak_kind": "ncu per-cycle FP64 peak x median SM clock under load; frac counts DADD, DMUL "
-                                  "and DFMA only, pipe_busy_ncu every instruction on the FP64 unit"}
+                     "peak_kind": "ncu per-cycle FP64 peak x median SM clock under load; frac counts the warp "
+                                  "instructions on the FP64 unit, 32 lanes each"}
 
     forms = {
         "fp64": form_line(m64, args.config, cells),
@@ -615,14 +612,14 @@ def main():
         "dtype": "f64", "data": "synthetic (seeded balanced jet + Gaussian; no dataset)",
         "config": {"workload": f"{args.config}: {desc}", "nx": p.nx, "ny": p.ny, "form": "fp64-exact",
                    "parallelism": f"replicas x{ws}" if ws > 1 else "single GPU",
-                   "l2": "no flush: each step streams >0.6 GB of fields, far above L2"},
+                   "l2": "no flush: each step streams >0.5 GB of fields, far above L2"},
         "hbm_gbs_step": STEP_BYTES * value / 1e9,
         "roofline": {"bound": "hbm", "kernel": m64["kernel"], "achieved": m64["achieved_gbs"], "peak": peak,
                      "unit": "GB/s", "frac": (m64["achieved_gbs"] / peak) if m64["achieved_gbs"] else None,
                      "traffic": NCU_TRAFFIC.get((args.config, m64["kernel"])), "peak_kind": peak_kind,
                      "bytes_per_cell": m64["bytes_per_cell"],
                      "per_launch_ms": m64["per_launch_ms"], "kernel_share": m64["kernel_share"],
-                     "note": "the FP64 form is bound by GB300's FP64 unit (84 % busy in ncu), not by HBM: "
+                     "note": "the FP64 form is bound by GB300's FP64 unit (72 % busy in ncu), not by HBM: "
                              "see roofline_fp64"},
         "roofline_fp64": fp64_roof,
         "kernels_ms_per_step": m64["kernels_ms_per_step"],

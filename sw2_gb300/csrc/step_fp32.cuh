@@ -1537,7 +1537,7 @@ __global__ void __launch_bounds__(NT, 6) kb_lap3(SW2G_KPARAMS) {
 // instead, warps of both kinds side by side, 0.245 ms at 4096x2048
 // against 0.200; 6 blocks (80 registers) 0.214. The tracer's strips come last:
 // they fill the launch's tail, which a launch of their own has once more (four
-// steps at 1501x1001 with winds and a tracer 0.610 and 0.590 ms, 320x320 caps
+// steps at 1501x755 with winds and a tracer 0.610 and 0.590 ms, 320x320 caps
 // 0.360 and 0.339).
 template <int SCH, bool EXTRA, int N, bool POLAR = false>
 __global__ void __launch_bounds__(NT, EXTRA ? 3 : 5) kb_main1(SW2G_KPARAMS, int per) {

@@ -1979,7 +1979,7 @@ __global__ void k_range(DevState s, RangeFields r, int* bad) {
 // 2.03 and 1.93 ms; four steps of a 500x500 cap 0.830, 0.795 and 0.794; four
 // steps at 2048x1024 3.286, 3.290 and 3.318. One launch for the bodies in place
 // of three or four: a step at 256x128 88 -> 80 us, at 2048x1024 0.364 ms of
-// bodies -> 0.340.
+// bodies -> 0.340; with the CFL maxima and the Laplacians' first levels 80 -> 72.
 int choose_strip_rows(int columns, int ny, long long warps) {
   int best = 1;
   double least = 0;
