@@ -440,7 +440,9 @@ constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the 
 // Resident blocks per SM the register allocation must allow: 7 blocks (28
 // warps) at 72 registers hide the FP64 unit's latency best. k_adv_u at
 // 2048x1024 with 4, 5, 6, 7, 8 and 10 blocks: 0.138, 0.133, 0.128, 0.122,
-// 0.124 and 0.125 ms.
+// 0.124 and 0.125 ms. In one launch with the other kinds, whole steps with 6, 7
+// and 8: four at 2048x1024 3.229, 3.212, 3.197 ms; four of a 500x500 cap 0.763,
+// 0.759, 0.771; two forced ones from rest at 1024x512 2.147, 2.000, 2.051.
 #define FAST_MIN_BLOCKS 7
 constexpr unsigned FULL = 0xffffffffu;
 
