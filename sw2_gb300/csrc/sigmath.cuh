@@ -61,6 +61,14 @@ SIG_FN uint64_t sig_mul(uint64_t a, uint64_t b, uint32_t k20 = 0) {
   return sig_pack(m, sig_exp(a) + sig_exp(b) + k20 - SIG_BIAS + ((sh - 1) << 20));
 }
 
+// |(a * b) * c|, rounded after each product. far is set where a, b or a
+// product is not a normal number: the result is then not the product.
+SIG_FN uint64_t sig_mul3(uint64_t a, uint64_t b, uint64_t c, bool& far) {
+  const uint32_t ea = (uint32_t)(a >> 52), eb = (uint32_t)(b >> 52), s = ea + eb, e = s + (uint32_t)(c >> 52);
+  far = far || (ea > eb ? ea : eb) > 2046u || (ea < eb ? ea : eb) == 0 || s - 1024u >= 2045u || e - 2050u >= 2030u;
+  return sig_mul(sig_mul(a, b), c);
+}
+
 // The last step of a quotient N / mb in [1, 2) (mb: 53 bits): t = floor(N/mb *
 // 2^53) or, where `unsure`, possibly one less than it; the quotient of two
 // doubles is never a tie, so t's last bit (the half) decides the rounding, and

@@ -1,0 +1,119 @@
+"""Values at which an integer-pipe operation or a shortcut of the FP64 step has
+to hand over or to keep a sign: the step against the CPU oracle and the
+operations, compiled for the host, against IEEE arithmetic, bit for bit."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from sw2_gb300 import cases, lib
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+GXX = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+PRELUDE = r"""
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include "sigmath.cuh"
+using namespace sw2g;
+static uint64_t st = 0x9216D5D98979FB1BULL;
+static uint64_t next() {  // SplitMix64
+  uint64_t z = (st += 0x9E3779B97F4A7C15ULL);
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+  return z ^ (z >> 31);
+}
+static double from(uint64_t b) { double d; std::memcpy(&d, &b, 8); return d; }
+static uint64_t bits(double d) { uint64_t b; std::memcpy(&b, &d, 8); return b; }
+static uint64_t frac() { return next() >> 12; }
+"""
+
+
+def host_run(tmp_path, text, *args, defines=()):
+    c, exe = tmp_path / "h.cpp", tmp_path / "h"
+    c.write_text(PRELUDE + text)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fno-fast-math", *defines, "-I",
+                    os.path.join(ROOT, "sw2_gb300", "csrc"), "-o", str(exe), str(c)], check=True)
+    return subprocess.run([str(exe), *map(str, args)], check=True, capture_output=True, text=True).stdout.split()
+
+
+def bitwise(a, b):
+    """Equal bit for bit, NaNs as NaNs."""
+    nan = np.isnan(a) & np.isnan(b)
+    return np.array_equal(a.view(np.int64)[~nan], b.view(np.int64)[~nan]) and np.array_equal(np.isnan(a), np.isnan(b))
+
+
+MUL3 = r"""
+// any exponents: where sig_mul3 does not say `far`, it is the rounded product;
+// and it does not say so for factors and products well inside the range
+int main(int, char** argv) {
+  long long wrong = 0, refused = 0, taken = 0;
+  for (long long i = 0; i < atoll(argv[1]); i++) {
+    const int wide = next() % 2 ? 2046 : 300, lo = wide == 300 ? 873 : 1;
+    uint64_t x[3];
+    for (uint64_t& v : x) v = ((uint64_t)(lo + next() % wide) << 52) | frac();
+    const int k = next() % 16;
+    if (k == 0) x[1] = 0;                                   // a Courant number of 1
+    if (k == 1) x[1] = bits(1.0 - from(bits(1.0) - 1));     // and next to it
+    if (k == 2) x[next() % 2] = frac();                     // subnormal
+    if (k == 3) x[0] = 0x7ff0000000000000ULL | (next() % 2);  // inf, NaN
+    bool far = false;
+    const uint64_t m = sig_mul3(x[0], x[1], x[2], far);
+    if (!far) {
+      taken++;
+      wrong += m != bits(from(x[0]) * from(x[1]) * from(x[2]));
+    }
+    bool inside = true;
+    for (uint64_t v : x) inside = inside && (v >> 52) >= 873 && (v >> 52) < 1173;
+    refused += inside && far;
+  }
+  printf("%lld %lld %d\n", wrong, refused, taken > 1000);
+}
+"""
+
+
+@GXX
+def test_three_factor_products_match_ieee_or_are_refused(tmp_path):
+    assert host_run(tmp_path, MUL3, 5_000_000) == ["0", "0", "1"]
+
+
+def same_steps(case, counts, flags=0, raw=False):
+    s = lib.Solver(case.params, flags=flags)
+    s.upload(*case.fields(), mode=lib.UPLOAD_RAW if raw else lib.UPLOAD_FRAME)
+    o = orc.Oracle(case.params, lape_eta=bool(flags & lib.FLAG_LAPE_ETA))
+    o.load(case.fields(), raw=raw)
+    for n in counts:
+        assert s.step(n) == lib.OK
+        assert o.step(n) == (0, -1)
+        got = s.download()
+        for k in ("eta", "u", "v", "tracer"):
+            assert bitwise(got[k], o.field(k)), (k, s.steps_done())
+    return s
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sch", [1, 9])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_gpu_courant_number_of_one_matches_oracle(sch, sign):
+    """v*Dt = DYN exactly in every row, so 1 - C is a zero, and fields that are
+    zero beside steps of 64 and more: a face's slope term is a zero there."""
+    case = cases.make_case(nx=64, ny=33, sch=sch, seed=3, jet="none", bumps=0, lat0=-30.0, lat1=20.0)
+    p = case.params
+    p.rP, p.depth, p.Dt, p.CFL = p.rE, 0.0, 512.0, 1e30
+    g = cases.Grid(p)
+    dyn = np.array([(g.lat1 - g.lat0) / p.ny * g.rM(g.latc(j)) for j in range(-1, p.ny + 3)])
+    vj = sign * dyn / p.Dt
+    assert np.all(np.abs(vj) * p.Dt / dyn == 1.0)
+    case.v[:] = vj[:, None]
+    case.eta[:] = 0.0
+    for k, x in enumerate((case.eta, case.u, case.tracer)):
+        x[12:20, 10:30] = (1000.0, 64.0, 3e5)[k]
+        x[24, 5:50] = -128.0
+    for x in (case.eta, case.u, case.v, case.tracer):
+        cases.halo_wrap(x)
+    same_steps(case, (1,), raw=True)
