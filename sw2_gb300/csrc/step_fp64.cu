@@ -760,7 +760,10 @@ __device__ __forceinline__ double sum_faces(const Side& w, const Side& so, const
   }
   const double S = ((w.t - te) + so.t) - n.t;
   slow = false;
-  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1);
+  if (!nz(S)) {
+    slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1);
+    return 0.0;  // -0 here where the terms are -0, +0, -0 and +0; the literal sum, from its +0 on, stays +0
+  }
   return S;
 }
 

@@ -117,3 +117,27 @@ def test_gpu_courant_number_of_one_matches_oracle(sch, sign):
     for x in (case.eta, case.u, case.v, case.tracer):
         cases.halo_wrap(x)
     same_steps(case, (1,), raw=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tau", [1e20, 1e6])
+@pytest.mark.parametrize("sch", [0, 2, 9])
+def test_gpu_zero_sums_of_a_diverging_flow_are_plus_zero(sch, tau):
+    """A layer of thickness zero in a flow away from a point: each cell's four
+    terms are zeros, of signs such that a sum without the unused sides' zeros is
+    -0; the reference's, which starts from +0, is +0. Only the histories of a
+    checkpoint show it: eta + (-0) = eta."""
+    case = cases.make_case(nx=64, ny=33, sch=sch, seed=3, jet="none", bumps=0, lat0=-30.0, lat1=20.0, hyper=False, Tau=tau)
+    p = case.params
+    p.depth, p.CFL = 0.0, 1e30
+    case.eta[:] = 0.0
+    case.u[:] = (np.arange(p.nx + 4) - 30.5)[None, :]
+    case.v[:] = (np.arange(p.ny + 4) - 15.5)[:, None]
+    for x in (case.u, case.v):
+        cases.halo_wrap(x)
+    s = lib.Solver(p)
+    s.upload(*case.fields(), mode=lib.UPLOAD_RAW)
+    assert s.step(1) == lib.OK
+    S = (p.nx + 4) * (p.ny + 4)
+    history = s.checkpoint()[-8 * S:][:S].reshape(p.ny + 4, p.nx + 4)  # of eta's tendency, the step's
+    assert not np.any(history) and not np.any(np.signbit(history))
