@@ -100,7 +100,7 @@ SIG_FN uint64_t sig_div_known(uint64_t a, uint64_t b, uint64_t y) {
   return sig_pack(m, sig_exp(a) - sig_exp(b) + SIG_BIAS - (ge ? 0u : 1u << 20));
 }
 
-// 1/f of a float in [1, 2], within one ulp.
+// 1/f of a float in (1, 2], within one ulp (2^-24).
 SIG_FN float sig_rcp(float f) {
 #if defined(__CUDA_ARCH__)
   float r;
@@ -117,16 +117,19 @@ union SigFloat {
 SIG_FN uint32_t sig_mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 
 // |a / b|, by long division in three digits of about 20 bits. y is the
-// reciprocal of b's leading 24 bits rounded up, less three ulps: below 1/b by
-// a factor of at most 1 - 2^-20.6 (the rounding up, one ulp of the
-// approximation, the three ulps), so every digit comes out low, every
-// remainder is positive and below 2^64, and the sum of the digits is at most
-// 510 units of 2^-70 below the quotient.
+// reciprocal of b's leading 24 bits rounded up (at most 2^-23 above b in
+// [1, 2)), less three ulps of 2^-24. With the approximation within one ulp it
+// is below 1/b, by a factor of at most 1 - 9*2^-24. So every digit comes out low
+// and every remainder is positive: below 1154, 651 and 368 units of the digit's
+// place (e -> e*2^20*9*2^-24 + 2, from 2*2^30*9*2^-24 + 2), the first below 2^64. The
+// sum of the digits is at most 368 units of 2^-70 below the quotient; the rounding
+// test allows 520.
 SIG_FN uint64_t sig_div(uint64_t a, uint64_t b) {
   const uint64_t ma = sig_of(a), mb = sig_of(b);
   SigFloat f;
   f.u = (0x3f800000u | ((uint32_t)(mb >> 29) & 0x7fffffu)) + 1u;
   f.f = sig_rcp(f.f);
+  f.u = f.u > 0x3f000000u ? f.u : 0x3f000000u;  // 1/f >= 1/2, where the approximation may be an ulp less (f = 2)
   const uint32_t y = (f.u << 8 | 0x80000000u) - 0x300u;  // units of 2^-32
   const bool ge = ma >= mb;
   const uint64_t N = ge ? ma : ma + ma;

@@ -34,10 +34,10 @@ static uint64_t frac() { return next() >> 12; }
 """
 
 
-def host_run(tmp_path, text, *args, defines=()):
+def host_run(tmp_path, text, *args):
     c, exe = tmp_path / "h.cpp", tmp_path / "h"
     c.write_text(PRELUDE + text)
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fno-fast-math", *defines, "-I",
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fno-fast-math", "-I", str(tmp_path), "-I",
                     os.path.join(ROOT, "sw2_gb300", "csrc"), "-o", str(exe), str(c)], check=True)
     return subprocess.run([str(exe), *map(str, args)], check=True, capture_output=True, text=True).stdout.split()
 
@@ -80,6 +80,39 @@ int main(int, char** argv) {
 @GXX
 def test_three_factor_products_match_ieee_or_are_refused(tmp_path):
     assert host_run(tmp_path, MUL3, 5_000_000) == ["0", "0", "1"]
+
+
+DIV = r"""
+int main(int, char** argv) {
+  long long wrong = 0;
+  for (long long i = 0; i < atoll(argv[1]); i++) {
+    uint64_t a = 0x3ff0000000000000ULL | frac(), b = 0x3ff0000000000000ULL | frac();
+    switch (next() % 8) {
+      case 0: b |= ((1ULL << 23) - 1) << 29; break;             // leading bits that round up to 2
+      case 1: b &= ~(((1ULL << 23) - 1) << 29); break;          // and to the least above 1
+      case 2: b = 0x3fffffffffffffffULL - next() % 64; break;
+      case 3: b = 0x3ff0000000000000ULL + next() % 64; break;
+      case 4: a = bits(from(b) * (from(a) + std::ldexp((double)(next() % 8 + 1), -54))); break;  // next to a midpoint
+      case 5: a = 0x3fffffffffffffffULL - next() % 64; break;
+      default: break;
+    }
+    wrong += sig_div(a, b) != bits(from(a) / from(b));
+  }
+  printf("%lld\n", wrong);
+}
+"""
+
+
+@GXX
+@pytest.mark.parametrize("ulps", [-1, 0, 1])
+def test_quotients_hold_with_a_reciprocal_one_ulp_off(tmp_path, ulps):
+    """The device's reciprocal is an approximation within one ulp of 2^-24."""
+    with open(os.path.join(ROOT, "sw2_gb300", "csrc", "sigmath.cuh")) as f:
+        text = f.read()
+    exact = "return 1.0f / f;"
+    assert text.count(exact) == 1
+    (tmp_path / "sigmath.cuh").write_text(text.replace(exact, f"return 1.0f / f + ({ulps}) * 0x1p-24f;"))
+    assert host_run(tmp_path, DIV, 20_000_000) == ["0"]
 
 
 def same_steps(case, counts, flags=0, raw=False):
