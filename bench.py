@@ -548,10 +548,11 @@ def main():
         large = (cl.params.nx * cl.params.ny, descl, ml64, ml32, accl)
         del cl
     forced = forcing_leg() if args.forcing and rank == 0 else None
-    # the FP64 step's division by row metrics (one Markstein correction)
-    # against IEEE division: 1e10 random and near-midpoint numerators over the
-    # metric factors of the headline workload, and each factor against the
-    # 1024 numerators within 512 ulps below +-2
+    # the FP64 step's quotients (by row metrics with one Markstein correction,
+    # and on the integer pipe) and integer-pipe products against IEEE
+    # arithmetic: 1e10 random and near-midpoint numerators over the metric
+    # factors of the headline workload, and each factor against the 1024
+    # numerators within 512 ulps below +-2
     divs = metric_divisors(case)
     per = int(1e10) // len(divs) + 1
     div_check = {"divisors": len(divs), "samples": per * len(divs), "grid_pairs": 1024 * len(divs),

@@ -7,6 +7,7 @@
 #include <new>
 #include <vector>
 
+#include "sigmath.cuh"
 #include "sw2g_internal.h"
 
 using namespace sw2g;
@@ -1668,17 +1669,21 @@ extern "C" sw2g_status sw2g_selfcheck_division(const double* divisors, int n, lo
   for (int k = 0; k < n; k++)
     if (!(divisors[k] > 0) || !std::isfinite(divisors[k]) || divisors[k] < 1e-300) return SW2G_ERR_BAD_ARG;
   CK(cudaSetDevice(device));
+  std::vector<unsigned long long> recip(n);
+  for (int k = 0; k < n; k++) recip[k] = sig_recip(sig_mag(divisors[k]));
   double* d = nullptr;
-  unsigned long long* bad = nullptr;
+  unsigned long long *y = nullptr, *bad = nullptr;
   cudaStream_t st = nullptr;
   sw2g_status rc = SW2G_OK;
   auto run = [&]() -> sw2g_status {
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     CK(cudaMalloc((void**)&d, sizeof(double) * n));
     CK(cudaMalloc((void**)&bad, sizeof(unsigned long long)));
+    CK(cudaMalloc((void**)&y, sizeof(unsigned long long) * n));
     CK(cudaMemcpyAsync(d, divisors, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(y, recip.data(), sizeof(unsigned long long) * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st));
-    fp64_check_division(d, n, samples, seed, bad, st);
+    fp64_check_division(d, y, n, samples, seed, bad, st);
     CK(cudaGetLastError());
     unsigned long long h = 0;
     CK(cudaMemcpyAsync(&h, bad, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -1688,6 +1693,7 @@ extern "C" sw2g_status sw2g_selfcheck_division(const double* divisors, int n, lo
   };
   rc = run();
   if (d) cudaFree(d);
+  if (y) cudaFree(y);
   if (bad) cudaFree(bad);
   if (st) cudaStreamDestroy(st);
   return rc;

@@ -143,4 +143,39 @@ SIG_FN uint64_t sig_div(uint64_t a, uint64_t b) {
   return sig_pack(m, sig_exp(a) - sig_exp(b) + SIG_BIAS - (ge ? 0u : 1u << 20));
 }
 
+// How many of the operations above give another result than the product and
+// the quotient of a and b, with y = sig_recip of b's bits (none where an operand
+// or result is not a normal number).
+union SigDouble {
+  double d;
+  uint64_t u;
+};
+SIG_FN uint64_t sig_mag(double x) {
+  SigDouble v;
+  v.d = x;
+  return v.u & 0x7fffffffffffffffULL;
+}
+SIG_FN bool sig_normal(uint64_t a) { return (a >> 52) - 1 < 2046; }
+SIG_FN int sig_mismatches(double a, double b, uint64_t y) {
+  const uint64_t A = sig_mag(a), B = sig_mag(b), q = sig_mag(a / b), p = sig_mag(a * b);
+  int n = 0;
+  if (!sig_normal(A) || !sig_normal(B)) return 0;
+  if (sig_normal(q)) n += (sig_div(A, B) != q) + (sig_div_known(A, B, y) != q);
+  if (sig_normal(p)) {
+    n += sig_mul(A, B) != p;
+    if (sig_normal(p - SIG_ONE)) n += sig_mul(A, B, 0xfff00000u) != p - SIG_ONE;
+  }
+  if (sig_normal(q)) {
+    bool far = false;
+    const uint64_t m = sig_mul3(A, B, q, far);
+    n += !far && m != sig_mag(a * b * (a / b));
+  }
+  return n;
+}
+// Whether sig_rcp(f), 1 < f <= 2, is within 2^-24 of 1/f (the product has 48 bits, the difference fewer).
+SIG_FN bool sig_rcp_close(float f) {
+  const double e = (double)sig_rcp(f) * (double)f - 1.0;
+  return (e < 0 ? -e : e) <= 0x1p-24 * (double)f;
+}
+
 }  // namespace sw2g

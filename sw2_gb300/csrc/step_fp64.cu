@@ -1069,10 +1069,12 @@ __device__ __forceinline__ void adv_v_strip(const DevState& s, const F7& f, doub
 #undef UF
 #undef VF
 #undef HF
-// Self-check of div_rcp: for each divisor b, `samples` numerators a drawn
-// from a SplitMix64 stream (random significands over exponents 2^-950..2^60,
-// both signs, and numerators whose quotient lies within a few ulps of a
-// rounding midpoint), compared bit for bit with the IEEE quotient a/b.
+// Self-check of the step's products and quotients: for each divisor b (recip:
+// its sig_recip), `samples` numerators a drawn from a SplitMix64 stream (random
+// significands over exponents 2^-950..2^60, both signs, and numerators whose
+// quotient lies within a few ulps of a rounding midpoint), compared bit for
+// bit with IEEE: a/b by div_rcp, and the integer-pipe operations on a and b
+// (sig_mismatches); and the reciprocals that sig_div starts from, all 2^23.
 __device__ __forceinline__ unsigned long long splitmix(unsigned long long& x) {
   unsigned long long z = (x += 0x9E3779B97F4A7C15ULL);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
@@ -1080,8 +1082,8 @@ __device__ __forceinline__ unsigned long long splitmix(unsigned long long& x) {
   return z ^ (z >> 31);
 }
 
-__global__ void k_check_division(const double* div, int n, long long samples, unsigned long long seed,
-                                 unsigned long long* bad) {
+__global__ void k_check_division(const double* div, const unsigned long long* recip, int n, long long samples,
+                                 unsigned long long seed, unsigned long long* bad) {
   const long long total = (long long)n * samples;
   unsigned long long miss = 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -1102,6 +1104,7 @@ __global__ void k_check_division(const double* div, int n, long long samples, un
     }
     const double want = a / b, got = div_rcp(a, b, y);
     if (dbits(want) != dbits(got)) miss++;
+    miss += sig_mismatches(a, b, recip[t / samples]);
   }
   // every divisor against the numerators +-(2 - k ulp), k = 1..512: with the
   // divisor's significand also within a few ulps of 2 these are the pairs
@@ -1116,7 +1119,10 @@ __global__ void k_check_division(const double* div, int n, long long samples, un
     const double a = __longlong_as_double((long long)((0x3FFFFFFFFFFFFFFFULL - k) | (neg << 63)));
     const double want = a / b, got = div_rcp(a, b, y);
     if (dbits(want) != dbits(got)) miss++;
+    miss += sig_mismatches(a, b, recip[t >> 10]);
   }
+  for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < (1u << 23); u += gridDim.x * blockDim.x)
+    if (!sig_rcp_close(__uint_as_float(0x3f800001u + u))) miss++;
   if (miss) atomicAdd(bad, miss);
 }
 
@@ -2148,9 +2154,9 @@ void fp64_check_add(long long samples, unsigned long long seed, unsigned long lo
   k_check_add<<<152 * 8, 256, 0, st>>>(samples, seed, bad);
 }
 
-void fp64_check_division(const double* d_div, int n, long long samples, unsigned long long seed,
-                         unsigned long long* bad, cudaStream_t st) {
-  k_check_division<<<152 * 8, 256, 0, st>>>(d_div, n, samples, seed, bad);
+void fp64_check_division(const double* d_div, const unsigned long long* d_recip, int n, long long samples,
+                         unsigned long long seed, unsigned long long* bad, cudaStream_t st) {
+  k_check_division<<<152 * 8, 256, 0, st>>>(d_div, d_recip, n, samples, seed, bad);
 }
 
 void halo_wrap(double* x, int nx, int ny, cudaStream_t st) {

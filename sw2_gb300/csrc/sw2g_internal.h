@@ -186,11 +186,12 @@ void fp64_channel(double* u, double* v, double* wx, double* wy, int nx, int ny, 
 void fp64_range(const DevState& s, const double* const* fields, int n, int* bad, cudaStream_t st);
 // f[cells[k]] = values[k] (values NULL: 0.0) for k < n; the cells are distinct.
 void fp64_scatter_cells(double* f, const int* cells, const double* values, int n, cudaStream_t st);
-// Compares the step's division by a row metric (div_rcp) with IEEE division
-// on `samples` random numerators per divisor; returns the mismatch count in
-// *bad (device pointer) once the stream is done.
-void fp64_check_division(const double* d_div, int n, long long samples, unsigned long long seed,
-                         unsigned long long* bad, cudaStream_t st);
+// Compares the step's quotients (div_rcp, and on the integer pipe with
+// d_recip, each divisor's sig_recip) and integer-pipe products with IEEE
+// arithmetic on `samples` random numerators per divisor; returns the mismatch
+// count in *bad (device pointer) once the stream is done.
+void fp64_check_division(const double* d_div, const unsigned long long* d_recip, int n, long long samples,
+                         unsigned long long seed, unsigned long long* bad, cudaStream_t st);
 // Compares the step's integer-pipe additions (sadd, ssub) with the FP64
 // unit's on `samples` operand pairs; mismatch count in *bad (device pointer).
 void fp64_check_add(long long samples, unsigned long long seed, unsigned long long* bad, cudaStream_t st);

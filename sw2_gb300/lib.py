@@ -106,7 +106,7 @@ def load():
 
 
 def selfcheck_division(divisors, samples: int, seed: int = 1, device: int = 0) -> int:
-    """Mismatches of the step's metric division against IEEE division."""
+    """Mismatches of the step's quotients and integer-pipe products against IEEE arithmetic."""
     L = load()
     L.sw2g_selfcheck_division.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.c_int, ctypes.c_longlong,
                                           ctypes.c_ulonglong, ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]

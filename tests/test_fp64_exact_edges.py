@@ -115,6 +115,60 @@ def test_quotients_hold_with_a_reciprocal_one_ulp_off(tmp_path, ulps):
     assert host_run(tmp_path, DIV, 20_000_000) == ["0"]
 
 
+CHECK = r"""
+int main(int, char** argv) {  // the self-check's draws
+  long long n = 0, far = 0;
+  for (long long i = 0; i < atoll(argv[1]); i++) {
+    const double b = from(((uint64_t)(1003 + next() % 80) << 52) | frac());
+    double a;
+    if (next() % 2) a = from(((uint64_t)(73 + next() % 1010) << 52) | frac());
+    else a = b * (from(((uint64_t)(523 + next() % 500) << 52) | frac()) * (1 + std::ldexp((double)(next() % 8 + 1), -54)));
+    if (next() % 64 == 0) a = from(((uint64_t)(900 + next() % 100) << 52) | (frac() >> 26 << 26));  // products that end in a tie
+    n += sig_mismatches(a, i % 64 ? b : from(0x3ff0000000000000ULL | 1ULL << 51), sig_recip(bits(i % 64 ? b : 1.5)));
+  }
+  for (uint32_t u = 0; u < (1u << 23); u++) {
+    SigFloat f;
+    f.u = 0x3f800001u + u;
+    far += !sig_rcp_close(f.f);
+  }
+  printf("%d %d\n", n != 0, far != 0);
+}
+"""
+
+
+@GXX
+@pytest.mark.parametrize("right,wrong,told", [
+    ("", "", ["0", "0"]),
+    ("0x20000u - 520u", "0x20000u", ["1", "0"]),        # sig_div: digits that came out low
+    ("mid >= 0xff800000u", "false", ["1", "0"]),        # sig_div_known: an estimate that came out low
+    ("m &= ~1ULL;", ";", ["1", "0"]),                   # sig_mul: ties
+    ("- SIG_BIAS + ((sh", "- SIG_BIAS + (1u << 20) + ((sh", ["1", "0"]),
+    ("return 1.0f / f;", "return 1.0f / f - 3 * 0x1p-24f;", ["1", "1"]),
+])
+def test_self_check_tells_planted_mistakes(tmp_path, right, wrong, told):
+    """sw2g_selfcheck_division's comparison, with mistakes planted in a host copy."""
+    with open(os.path.join(ROOT, "sw2_gb300", "csrc", "sigmath.cuh")) as f:
+        text = f.read()
+    if right:
+        assert text.count(right) == 1
+        text = text.replace(right, wrong)
+    (tmp_path / "sigmath.cuh").write_text(text)
+    assert host_run(tmp_path, CHECK, 4_000_000) == told
+
+
+@pytest.mark.gpu
+def test_gpu_quotients_and_products_match_ieee():
+    """Divisors whose leading 24 bits round up to 2 or to the least above 1, and
+    those of every exponent the metric factors may have."""
+    rng = np.random.default_rng(17)
+    low = rng.integers(0, 1 << 29, 4000, dtype=np.uint64)
+    ones = np.uint64(0x3FF0000000000000) | np.uint64(((1 << 23) - 1) << 29) | low
+    none = np.uint64(0x3FF0000000000000) | low
+    d = np.concatenate([ones.view(np.float64), none.view(np.float64),
+                        np.ldexp(rng.uniform(1.0, 2.0, 8000), rng.integers(-20, 60, 8000))])
+    assert lib.selfcheck_division(d, samples=20_000, seed=14) == 0
+
+
 def same_steps(case, counts, flags=0, raw=False):
     s = lib.Solver(case.params, flags=flags)
     s.upload(*case.fields(), mode=lib.UPLOAD_RAW if raw else lib.UPLOAD_FRAME)
