@@ -623,7 +623,10 @@ sw2g_status sw2g_create(const sw2g_case* c, int precision, int device, sw2g_ctx*
   s.nu2 = c->hypernu[0];
   s.nu4 = -c->hypernu[1];  // init.c:120
   s.nu6 = c->hypernu[2];
-  s.sig_ok = rows_in_window(*c, x->rows) ? 1 : 0;
+  const SigRanges ranges = sig_ranges(*c, x->rows);
+  s.sig_ok = ranges.divisors;
+  s.lap_ok = ranges.laplacian;
+  s.nu_ok = ranges.nu;
   s.lape_eta = (c->flags & SW2G_FLAG_LAPE_ETA) ? 1 : 0;
   s.nu2dt = s.nu2 * s.Dt;
   s.nu4dt = s.nu4 * s.Dt;

@@ -43,13 +43,22 @@ double fcor(const Planet& p, double lat) { return 2.0 * p.Omega * std::sin(lat);
 // init.c:56-58 does), or already converted (SW2G_FLAG_RADIANS).
 double angle(const sw2g_case& c, double a) { return (c.flags & SW2G_FLAG_RADIANS) ? a : deg2rad(a); }
 
-// The divisors of the integer-pipe quotients and where their reciprocals go.
+// The divisors of the integer-pipe quotients, where their reciprocals go, and
+// the last row that a step divides by (from row 1), after ny. The row above ny
+// may lie beyond the pole, where rM is negative; DYNS = DYN(j) + DYN(j+1) of row
+// ny is then near zero, and the body of v tests it.
 struct SigDivisor {
-  int row, recip;
+  int row, recip, last;
 };
-constexpr SigDivisor kSigDivisors[] = {{R_DXE, R_YDXE}, {R_DXC, R_YDXC},   {R_DXV, R_YDXV},   {R_DYN, R_YDYN},
-                                       {R_DYC, R_YDYC}, {R_DYV, R_YDYV},   {R_DXE2, R_YDXE2}, {R_DYNS, R_YDYNS},
-                                       {R_RZC, R_YRZC}, {R_RZN, R_YRZN}};
+constexpr SigDivisor kSigDivisors[] = {{R_DXE, R_YDXE, 0},   {R_DXC, R_YDXC, 0}, {R_DXV, R_YDXV, 0}, {R_DYN, R_YDYN, 0},
+                                       {R_DYC, R_YDYC, 1},   {R_DYV, R_YDYV, 0}, {R_DXE2, R_YDXE2, 0},
+                                       {R_DYNS, R_YDYNS, -1}, {R_RZC, R_YRZC, 0}, {R_RZN, R_YRZN, 0}};
+// The factors of the Laplacians, and the rows they are read at: first to ny + last.
+struct LapFactor {
+  int row, first, last;
+};
+constexpr LapFactor kLapFactors[] = {{R_KX, 1, 0},   {R_KY, 1, 0},   {R_KC, 1, 0},   {R_IDXE, 1, 0}, {R_IDXC, 1, 0},
+                                     {R_IDXV, 1, 0}, {R_IDYN, 1, 0}, {R_IDYC, 1, 1}, {R_DXC, 1, 1},  {R_DXV, 0, 0}};
 uint64_t bits_of(double x) {
   uint64_t b;
   std::memcpy(&b, &x, sizeof b);
@@ -62,20 +71,17 @@ bool positive_in_window(uint64_t b) {  // 2^-20 <= x < 2^60
 
 }  // namespace
 
-bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows) {
+SigRanges sig_ranges(const sw2g_case& c, const std::vector<double>& rows) {
   const int H = c.ny + 4;
-  if (!positive_in_window(bits_of(c.Dt))) return false;
-  for (const auto& d : kSigDivisors)
-    for (int j = 0; j <= c.ny + 1; j++)  // the rows a step divides by
-      if (!positive_in_window(bits_of(rows[(size_t)d.row * H + (j + 1)]))) return false;
-  // the factors of the Laplacians and of their terms, where used: 2^-130 .. 2^250
+  auto R = [&](int t, int j) { return rows[(size_t)t * H + (j + 1)]; };
   auto mid = [](double x) { return std::fabs(x) >= 0x1p-130 && std::fabs(x) < 0x1p250; };
-  for (int t : {R_KX, R_KY, R_KC})
-    for (int j = 0; j <= c.ny + 1; j++)
-      if (!mid(rows[(size_t)t * H + (j + 1)])) return false;
-  for (double nu : c.hypernu)
-    if (nu != 0 && !mid(nu * c.Dt)) return false;
-  return true;
+  SigRanges r{positive_in_window(bits_of(c.Dt)), true, true};
+  for (const auto& d : kSigDivisors)
+    for (int j = 1; j <= c.ny + d.last; j++) r.divisors = r.divisors && positive_in_window(bits_of(R(d.row, j)));
+  for (const auto& f : kLapFactors)
+    for (int j = f.first; j <= c.ny + f.last; j++) r.laplacian = r.laplacian && mid(R(f.row, j));
+  for (double nu : c.hypernu) r.nu = r.nu && (nu == 0 || mid(nu * c.Dt));
+  return r;
 }
 
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my) {

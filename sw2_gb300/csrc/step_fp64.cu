@@ -433,8 +433,9 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 // that is not negative (first_term_plus_zero). So it is in a flow at rest and
 // for a tracer that is zero. Otherwise the cell is recomputed literally.
 // The Van Leer limiter in its reference form (0/0 at r = -1) keeps the
-// literal kernels, and so do cases whose Dt or metric factors lie outside
-// 2^-20 .. 2^60 (DevState::sig_ok).
+// literal kernels, and so do cases whose Dt or metric divisors lie outside
+// 2^-20 .. 2^60 (DevState::sig_ok). The face north of row ny serves no cell above:
+// its terms there are taken with row ny's metric.
 constexpr int FW = 31;      // cells per strip along x (32 faces)
 constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the launch's queue
 // Resident blocks per SM the register allocation must allow: 7 blocks (28
@@ -526,11 +527,11 @@ __device__ __forceinline__ double smul(double a, double b) {
   if (mid(a) && mid(b)) return from_bits(sig_mul(mag(a), mag(b)) | ((unsigned long long)(dbits(a) ^ dbits(b)) & kSign));
   return mul_fp64(a, b);
 }
-// s.sig_ok says that the row constants and hyperviscosity coefficients are of
-// magnitude 2^-130 .. 2^250; k: such a factor.
-__device__ __forceinline__ double rmul(const DevState& s, double k, double a) {
+// k: a factor of which `ok` (DevState::lap_ok, nu_ok) says that it is of
+// magnitude 2^-130 .. 2^250.
+__device__ __forceinline__ double rmul(bool ok, double k, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(k)) & kSign;
-  if (wider(a) && s.sig_ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
+  if (wider(a) && ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
   if (!nz(a)) return from_bits(sg);
   return mul_fp64(k, a);
 }
@@ -874,7 +875,7 @@ __device__ __forceinline__ void mass_strip(const DevState& s, const F7& f, doubl
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, METRIC(DYN, j), bad);
-    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, min(j + 1, ny)), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);  // calc.c:100 in its order: +w -e +s -n
     slow = __any_sync(FULL, bad) || slow;
@@ -926,7 +927,7 @@ __device__ __forceinline__ void tracer_strip(const DevState& s, const F7& f, dou
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, my, bad);
-    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, min(j + 1, ny)), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);
     slow = __any_sync(FULL, bad) || slow;
@@ -983,7 +984,7 @@ __device__ __forceinline__ void adv_u_strip(const DevState& s, const F7& f, doub
     const Vel v = vel_pair(va, vb, vn);
     const Face FY = y_face<SCH, true>(v, dm, d0, d1, u2, u3, dt, bad);
     const Side tn = side_of<true>(FY, my, bad);
-    const Side ns = side_of<true>(FY, METRIC(DYV, j + 1), bad);
+    const Side ns = side_of<true>(FY, METRIC(DYV, min(j + 1, ny)), bad);
     bool slow;
     const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, u2, slow);
     slow = __any_sync(FULL, bad) || slow;
@@ -1049,7 +1050,9 @@ __device__ __forceinline__ void adv_v_strip(const DevState& s, const F7& f, doub
     // sums of u symmetric in their operands
     const double ue = __shfl_sync(FULL, uw, (lane + 1) & 31);
     const double ux = ue - uw, vy = v3 - v1;
-    const double p2 = Dt * two_products(v2, ux, 0xfff00000u, mx, vy, 0, METRIC(DYNS, j));
+    const Metric ms = METRIC(DYNS, j);
+    slow = slow || ms.y == 0;  // row ny, where DYN(ny+1) lies beyond the pole
+    const double p2 = Dt * two_products(v2, ux, 0xfff00000u, mx, vy, 0, ms);
     if (own) {
       double r;
       if (slow) r = advv_cell_ool<SCH>(s, f, i, j);
@@ -1283,18 +1286,18 @@ struct LapEta {
     own = lane > 0 && c <= s.nx;
     e0 = e[IX(W, cc, j0)];
     xs = 0.0;
-    if (j0 > 1) xs = mdiv(s, rmul(s, RW(s, R_KY, j0 - 1), e0 - e[IX(W, cc, j0 - 1)]), METRIC(DYC, j0 - 1));
+    if (j0 > 1) xs = mdiv(s, rmul(s.lap_ok, RW(s, R_KY, j0 - 1), e0 - e[IX(W, cc, j0 - 1)]), METRIC(DYC, j0 - 1));
   }
   // the value at row j (warp-wide)
   __device__ __forceinline__ double next(const DevState& s, const double* e, int j) {
     const int W = s.W;
     touch(e + IX(W, cc, min(j + 2, s.ny + 1)));
     const double ee = e[IX(W, cc + 1, j)], en = e[IX(W, cc, j + 1)];
-    double psi = mdiv(s, rmul(s, RW(s, R_KX, j), ee - e0), METRIC(DXC, j));
+    double psi = mdiv(s, rmul(s.lap_ok, RW(s, R_KX, j), ee - e0), METRIC(DXC, j));
     if (c == 0) psi = 0.0;
     const double pw = __shfl_up_sync(FULL, psi, 1);
-    const double xi = mdiv(s, rmul(s, RW(s, R_KY, j), en - e0), METRIC(DYC, j));
-    const double v = rmul(s, RW(s, R_KC, j), mdiv(s, psi - pw, METRIC(DXE, j)) + mdiv(s, xi - xs, METRIC(DYN, j)));
+    const double xi = mdiv(s, rmul(s.lap_ok, RW(s, R_KY, j), en - e0), METRIC(DYC, j));
+    const double v = rmul(s.lap_ok, RW(s, R_KC, j), mdiv(s, psi - pw, METRIC(DXE, j)) + mdiv(s, xi - xs, METRIC(DYN, j)));
     e0 = en;
     xs = xi;
     return v;
@@ -1347,7 +1350,7 @@ __device__ __forceinline__ double hyper_terms(const DevState& s, double x, doubl
 #pragma unroll
     for (int t = 0; t < 3; t++) {
       const double v = V[t];
-      if ((NZ >> t) & 1) x = x + rmul(s, nd[t], v);
+      if ((NZ >> t) & 1) x = x + rmul(s.nu_ok, nd[t], v);
       else if (!zero_term_is_exact(x, v)) x = add_product(x, nd[t], v);
     }
     return x;
@@ -1453,13 +1456,13 @@ __device__ __forceinline__ void lapv_strip(const DevState& s, const double* uu, 
   const bool own = lane > 0 && lane <= LVW && c <= nx;
   // ze and di at row j of the column, the products of u (rows j, j+1) and v (rows j-1, j) given
   auto zeta = [&](int j, double v0, double ve, double pu, double pu1) {
-    return rmul(s, RW(s, R_IDXV, j), (ve - v0) - rmul(s, RW(s, R_IDYC, j + 1), pu1 - pu));
+    return rmul(s.lap_ok, RW(s, R_IDXV, j), (ve - v0) - rmul(s.lap_ok, RW(s, R_IDYC, j + 1), pu1 - pu));
   };
   auto divg = [&](int j, double u0, double uw, double qs, double qv) {
-    return rmul(s, RW(s, R_IDXE, j), (u0 - uw) + rmul(s, RW(s, R_IDYN, j), qv - qs));
+    return rmul(s.lap_ok, RW(s, R_IDXE, j), (u0 - uw) + rmul(s.lap_ok, RW(s, R_IDYN, j), qv - qs));
   };
-  auto PU = [&](int j, double u) { return rmul(s, RW(s, R_DXC, j), u); };
-  auto QV = [&](int j, double v) { return rmul(s, RW(s, R_DXV, j), v); };
+  auto PU = [&](int j, double u) { return rmul(s.lap_ok, RW(s, R_DXC, j), u); };
+  auto QV = [&](int j, double v) { return rmul(s.lap_ok, RW(s, R_DXV, j), v); };
   auto u_at = [&](int i, int j) { return uu[IX(W, i, j)]; };
   auto v_at = [&](int i, int j) { return vv[IX(W, i, j)]; };
   double u0 = u_at(sc, j0), v0 = v_at(sc, j0);
@@ -1493,8 +1496,8 @@ __device__ __forceinline__ void lapv_strip(const DevState& s, const double* uu, 
     }
     const double zw = __shfl_up_sync(FULL, z, 1), de = __shfl_down_sync(FULL, d, 1);
     // (-a)*x + b*y = b*y - a*x
-    const double xu = rmul(s, RW(s, R_IDXC, j), de - d) - rmul(s, RW(s, R_IDYN, j), z - zs);
-    const double xv = rmul(s, RW(s, R_IDXV, j), z - zw) + rmul(s, RW(s, R_IDYC, j + 1), dn - d);
+    const double xu = rmul(s.lap_ok, RW(s, R_IDXC, j), de - d) - rmul(s.lap_ok, RW(s, R_IDYN, j), z - zs);
+    const double xv = rmul(s.lap_ok, RW(s, R_IDXV, j), z - zw) + rmul(s.lap_ok, RW(s, R_IDYC, j + 1), dn - d);
     if (own) {
       if (images) {
         put_images<HK_LU>(s, lu, c, j, xu);

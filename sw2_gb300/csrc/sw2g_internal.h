@@ -54,7 +54,8 @@ struct DevState {
   double nu2dt, nu4dt, nu6dt;  // (nu)*(Dt) as the reference forms it (calc.c:346-348)
   int plain;           // windx, windy and hB are +0.0 in every padded cell
   int lape_eta;        // laplacian_eta of eta instead of u (SW2G_FLAG_LAPE_ETA)
-  int sig_ok;          // Dt and the metric factors lie in the range of the integer-pipe quotients
+  int sig_ok;          // Dt and the metric divisors lie in the range of the integer-pipe quotients,
+  int lap_ok, nu_ok;   // the Laplacians' factors and the nu*Dt in that of its products (SigRanges)
   int fk;              // rows per strip of the fast TVD bodies (set per launch)
   unsigned* strips;    // the fast bodies' strip queue: next strip, warps done (zero between launches)
   int polar;           // 0: band; +-1: polar cap, with the fields below
@@ -71,8 +72,13 @@ bool grid_ok(const sw2g_case* c);
 // Host geometry (geometry.cpp): fills rows[R_NUM*H]; returns the at-rest CFL
 // maxima used by compute_Dt when the flow is at rest (calc.c:715-725).
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my);
-// Whether Dt and every metric divisor of the rows lie in [2^-20, 2^60).
-bool rows_in_window(const sw2g_case& c, const std::vector<double>& rows);
+// Which constants lie in the ranges of the integer-pipe operations: Dt and the
+// metric divisors in 2^-20 .. 2^60 (and positive), the factors of the Laplacians
+// and each nonzero nu*Dt in 2^-130 .. 2^250.
+struct SigRanges {
+  bool divisors, laplacian, nu;
+};
+SigRanges sig_ranges(const sw2g_case& c, const std::vector<double>& rows);
 // The fields of a polar cap (P_NUM x (nx+4)(ny+4)) and the at-rest CFL maxima
 // computed with them.
 void polar_fields(const sw2g_case& c, std::vector<double>& f, double* rest_mx, double* rest_my);

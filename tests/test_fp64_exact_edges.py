@@ -228,3 +228,47 @@ def test_gpu_zero_sums_of_a_diverging_flow_are_plus_zero(sch, tau):
     S = (p.nx + 4) * (p.ny + 4)
     history = s.checkpoint()[-8 * S:][:S].reshape(p.ny + 4, p.nx + 4)  # of eta's tendency, the step's
     assert not np.any(history) and not np.any(np.signbit(history))
+
+
+def rough_case(nx, ny, lat, orders=(1, 1, 1), **kw):
+    """Rough velocities everywhere, wall rows included, and a tracer."""
+    rng = np.random.default_rng(nx + ny)
+    case = cases.make_case(nx=nx, ny=ny, sch=2, seed=3, jet="none", bumps=0, lat0=-lat, lat1=lat, tracer=True, cfl=0.05, **kw)
+    nu4 = case.params.hypernu[1]
+    case.params.hypernu = (orders[0] * 0.02 * nu4 ** 0.5, orders[1] * nu4, orders[2] * 0.05 * nu4 ** 1.5)
+    case.params.CFL = 1e30
+    for x in (case.u, case.v):
+        x[:] = 0.1 * rng.standard_normal(x.shape)
+        cases.halo_wrap(x)
+    return case
+
+
+def launches_of_a_step(case):
+    s = lib.Solver(case.params)
+    s.upload(*case.fields(), mode=lib.UPLOAD_RAW)
+    assert s.step(2) == lib.OK and s.step(1) == lib.OK
+    return s.last_launches()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lat,nx,ny,wall", [(89.8, 64, 33, 0.0), (89.0, 33, 89, 1.0), (70.0, 40, 5, 1.0), (80.0, 31, 7, 0.0)])
+def test_gpu_bands_next_to_a_pole_keep_the_merged_launch(lat, nx, ny, wall):
+    """The row above the wall lies beyond the pole, where the metric factor of y
+    turns negative and that of DYN(ny) + DYN(ny+1) is next to zero: only the wall
+    row of v divides by it."""
+    case = rough_case(nx, ny, lat)
+    assert case.params.lat1 + 1.5 * (2 * lat) / ny > 90.0
+    case.v[ny + 1] *= wall
+    same_steps(case, (1, 1, 1), raw=True)
+    assert launches_of_a_step(case) == launches_of_a_step(rough_case(nx, ny, 40.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nu", [1e-45, 1e-300])
+def test_gpu_coefficients_outside_the_integer_range_keep_the_merged_launch(nu):
+    """A hyperviscosity coefficient that the integer-pipe products do not take
+    concerns that product alone."""
+    case = rough_case(64, 33, 60.0, hyper=False)
+    case.params.hypernu = (nu, 0.0, 0.0)
+    same_steps(case, (1, 1, 1, 2), raw=True)
+    assert launches_of_a_step(case) == launches_of_a_step(rough_case(64, 33, 60.0, orders=(1, 0, 0)))
