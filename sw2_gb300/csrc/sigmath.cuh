@@ -61,13 +61,16 @@ SIG_FN uint64_t sig_mul(uint64_t a, uint64_t b, uint32_t k20 = 0) {
   return sig_pack(m, sig_exp(a) + sig_exp(b) + k20 - SIG_BIAS + ((sh - 1) << 20));
 }
 
-// |(a * b) * c|, rounded after each product. far is set where a, b or a
-// product is not a normal number: the result is then not the product.
-SIG_FN uint64_t sig_mul3(uint64_t a, uint64_t b, uint64_t c, bool& far) {
-  const uint32_t ea = (uint32_t)(a >> 52), eb = (uint32_t)(b >> 52), s = ea + eb, e = s + (uint32_t)(c >> 52);
-  far = far || (ea > eb ? ea : eb) > 2046u || (ea < eb ? ea : eb) == 0 || s - 1024u >= 2045u || e - 2050u >= 2030u;
-  return sig_mul(sig_mul(a, b), c);
+// |(a * b) * c|, rounded after each product, where sig_mul3_far does not say
+// that a, b (a zero too) or a product is not a normal number, or the result not in
+// 2^-921 .. 2^121. For c in 2^-902 .. 2^102 and |a * c| at most 2^101: with c's
+// range, a result in that window leaves no room for an a * b outside the normal
+// range, and with |a * c|'s none for a b below it. ha, hb, hc: upper words.
+SIG_FN bool sig_mul3_far(uint32_t ha, uint32_t hb, uint32_t hc) {
+  const uint32_t ea = ha >> 20, e = ea + (hb >> 20) + (hc >> 20);
+  return ea - 1 >= 2046u || e - 2148u >= 1042u;
 }
+SIG_FN uint64_t sig_mul3(uint64_t a, uint64_t b, uint64_t c) { return sig_mul(sig_mul(a, b), c); }
 
 // The last step of a quotient N / mb in [1, 2) (mb: 53 bits): t = floor(N/mb *
 // 2^53) or, where `unsure`, possibly one less than it; the quotient of two
@@ -164,11 +167,6 @@ SIG_FN int sig_mismatches(double a, double b, uint64_t y) {
   if (sig_normal(p)) {
     n += sig_mul(A, B) != p;
     if (sig_normal(p - SIG_ONE)) n += sig_mul(A, B, 0xfff00000u) != p - SIG_ONE;
-  }
-  if (sig_normal(q)) {
-    bool far = false;
-    const uint64_t m = sig_mul3(A, B, q, far);
-    n += !far && m != sig_mag(a * b * (a / b));
   }
   return n;
 }

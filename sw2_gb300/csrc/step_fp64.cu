@@ -664,19 +664,18 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, N2 
   return F;
 }
 
-// (hp*g)*d, rounded twice as written, d a zero or an in-range difference. On the
+// (hp*g)*d, rounded twice as written. On the
 // integer pipe: k_adv_u at 2048x1024 0.146 ms with both products on the FP64
 // unit, 0.136 with one of them, 0.133 with none (the mass body 0.118, 0.109,
 // 0.101); c*B, whose B may be anything, stays there.
 // bad is set where a factor or a product is not a normal number, g = 1 - c = 0
-// (a Courant number of exactly 1) among them.
+// (a Courant number of exactly 1) among them. d is in range, and |hp*d| at
+// most the larger of |d| and half the ratio's numerator, at most 2^101.
 __device__ __forceinline__ double slope_term(double hp, double g, double d, bool& bad) {
   const unsigned long long sg = (unsigned long long)(dbits(hp) ^ dbits(g) ^ dbits(d)) & kSign;
   const bool zero = !nz(hp) || !nz(d);
-  bool far = false;
-  const unsigned long long m = sig_mul3(mag(hp), mag(g), mag(d), far);
-  bad = bad || (!zero && far);
-  return zero ? 0.0 : from_bits(m | sg);
+  bad = bad || (!zero && sig_mul3_far(hi_mag(hp), hi_mag(g), hi_mag(d)));
+  return zero ? 0.0 : from_bits(sig_mul3(mag(hp), mag(g), mag(d)) | sg);
 }
 // C*B of one side with c = |C|: B2BP (pos) = q0 + psi*0.5*(1-c)*(q1-q0), or
 // B2BM = q1 - psi*0.5*(1-c)*(q1-q0) (C- = -c; q1 - X = q1 + (-X) exactly).

@@ -49,30 +49,34 @@ def bitwise(a, b):
 
 
 MUL3 = r"""
-// any exponents: where sig_mul3 does not say `far`, it is the rounded product;
-// and it does not say so for factors and products well inside the range
+// c in 2^-902 .. 2^102, |a*c| at most 2^101, b any number a Courant number may
+// leave (zeros and subnormals too): where sig_mul3_far does not say so, sig_mul3
+// is the rounded product; and it does not for factors and products well inside
 int main(int, char** argv) {
   long long wrong = 0, refused = 0, taken = 0;
   for (long long i = 0; i < atoll(argv[1]); i++) {
-    const int wide = next() % 2 ? 2046 : 300, lo = wide == 300 ? 873 : 1;
-    uint64_t x[3];
-    for (uint64_t& v : x) v = ((uint64_t)(lo + next() % wide) << 52) | frac();
+    const bool wide = next() % 2;
+    const int ec = wide ? 121 + next() % 1004 : 874 + next() % 186;
+    uint64_t c = ((uint64_t)ec << 52) | frac(), a = ((wide ? 1 + next() % 2046 : 874 + next() % 186) << 52) | frac();
+    uint64_t b = ((wide ? next() % 2047 : 874 + next() % 186) << 52) | frac();
     const int k = next() % 16;
-    if (k == 0) x[1] = 0;                                   // a Courant number of 1
-    if (k == 1) x[1] = bits(1.0 - from(bits(1.0) - 1));     // and next to it
-    if (k == 2) x[next() % 2] = frac();                     // subnormal
-    if (k == 3) x[0] = 0x7ff0000000000000ULL | (next() % 2);  // inf, NaN
-    bool far = false;
-    const uint64_t m = sig_mul3(x[0], x[1], x[2], far);
+    if (k == 0) b = 0;                                   // a Courant number of 1
+    if (k == 1) b = bits(1.0 - from(bits(1.0) - 1));     // and next to it
+    if (k == 2) a = frac();                              // subnormal
+    if (k == 3) a = 0x7ff0000000000000ULL | (next() % 2);  // inf, NaN
+    if (k == 4) a = ((uint64_t)(2147 - ec > 2046 ? 2046 : 2147 - ec) << 52) | frac(), b = next() % 2 ? 0 : frac();
+    if (k != 3 && (int)(a >> 52) + ec > 2147) continue;
+    const bool far = sig_mul3_far(a >> 32, b >> 32, c >> 32);
     if (!far) {
       taken++;
-      wrong += m != bits(from(x[0]) * from(x[1]) * from(x[2]));
+      wrong += sig_mul3(a, b, c) != bits(from(a) * from(b) * from(c));
     }
     bool inside = true;
-    for (uint64_t v : x) inside = inside && (v >> 52) >= 873 && (v >> 52) < 1173;
+    const uint64_t x[3] = {a, b, c};
+    for (uint64_t v : x) inside = inside && (v >> 52) >= 874 && (v >> 52) < 1060;
     refused += inside && far;
   }
-  printf("%lld %lld %d\n", wrong, refused, taken > 1000);
+  printf("%lld %lld %d\n", wrong, refused, taken > 100000);
 }
 """
 
