@@ -276,3 +276,44 @@ def test_gpu_coefficients_outside_the_integer_range_keep_the_merged_launch(nu):
     case.params.hypernu = (nu, 0.0, 0.0)
     same_steps(case, (1, 1, 1, 2), raw=True)
     assert launches_of_a_step(case) == launches_of_a_step(rough_case(64, 33, 60.0, orders=(1, 0, 0)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx", [4095, 4096, 4097, 8193])
+@pytest.mark.parametrize("field", ["u", "v"])
+def test_gpu_cfl_maximum_is_found_in_every_column(nx, field):
+    """A warp takes 4096 columns of the CFL maxima: the one fast cell of the
+    grid at their edges."""
+    for col in sorted({1, min(nx, 4096), min(nx, 4097), nx}):
+        case = cases.make_case(nx=nx, ny=6, sch=2, seed=3, jet="none", bumps=0, lat0=-30.0, lat1=20.0, hyper=False)
+        p = case.params
+        for x in (case.eta, case.u, case.v):
+            x[:] = 0.0
+        x = getattr(case, field)
+        x[4, col + 1] = 1e-3
+        cases.halo_wrap(x)
+        g = cases.Grid(p)
+        lat = g.latc(3)
+        d = (g.lon1 - g.lon0) / nx * g.rZ(lat) if field == "u" else (g.lat1 - g.lat0) / p.ny * g.rM(lat)
+        for slack, want in ((1.0001, lib.OK), (0.9999, lib.ERR_CFL)):
+            p.CFL = p.Dt * 1e-3 / d * slack
+            s = lib.Solver(p)
+            s.upload(*case.fields(), mode=lib.UPLOAD_RAW)
+            assert s.step(1) == want, (col, slack)
+
+
+@pytest.mark.gpu
+def test_gpu_wide_grid_takes_no_longer_than_a_square_one():
+    """As many cells in 16 rows: no kernel's strips grow with the row."""
+    ms = []
+    for nx, ny in ((1024, 1024), (65536, 16)):
+        case = cases.make_case(nx, ny, sch=2, seed=3, bumps=1, cfl=0.2)
+        s = lib.Solver(case.params)
+        s.upload(*case.fields())
+        assert s.step(3) == lib.OK
+        t = []
+        for _ in range(7):
+            assert s.step(5) == lib.OK
+            t.append(s.last_step_ms())
+        ms.append(min(t))
+    assert ms[1] < 1.5 * ms[0]
