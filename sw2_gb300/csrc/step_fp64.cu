@@ -515,8 +515,7 @@ __device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j
 
 // Products and quotients of any operands, on the integer pipe when the
 // operands are of magnitude 2^-255 .. 2^257 (the result is then normal), on
-// the FP64 unit, out of line, otherwise. c: a factor that is finite and not
-// zero (a row constant or a coefficient): a zero times it is that zero.
+// the FP64 unit, out of line, otherwise. A zero times a finite factor is a zero.
 __device__ __forceinline__ bool mid(double x) { return ((hi_word(x) - 0x30000000u) & 0x60000000u) == 0; }
 // 2^-700 (2^-850) <= |x| < 2^257: times a factor of 2^-255 (2^-130) or more
 // still normal, and over a metric factor
@@ -532,20 +531,20 @@ __device__ __forceinline__ double smul(double a, double b) {
 __device__ __forceinline__ double rmul(bool ok, double k, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(k)) & kSign;
   if (wider(a) && ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
-  if (!nz(a)) return from_bits(sg);
+  if (!nz(a) && ok) return from_bits(sg);
   return mul_fp64(k, a);
 }
 __device__ __forceinline__ double cmul(double c, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(c)) & kSign;
   if (wide(a) && mid(c)) return from_bits(sig_mul(mag(a), mag(c)) | sg);
-  if (!nz(a)) return from_bits(sg);
+  if (!nz(a) && hi_mag(c) < SIG_EXP) return from_bits(sg);
   return mul_fp64(c, a);
 }
 __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
-// a / x.b (x.b > 0): a zero gives itself.
+// a / x.b: with x.b > 0, as s.sig_ok says, a zero gives itself.
 __device__ __forceinline__ double mdiv(const DevState& s, double a, const Metric& x) {
   if (wider(a) && s.sig_ok) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
-  if (!nz(a)) return a;
+  if (!nz(a) && s.sig_ok) return a;
   return div_fp64(a, from_bits(x.b));
 }
 

@@ -317,3 +317,23 @@ def test_gpu_wide_grid_takes_no_longer_than_a_square_one():
             t.append(s.last_step_ms())
         ms.append(min(t))
     assert ms[1] < 1.5 * ms[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", [dict(hypernu=(np.inf, 0.0, 0.0)), dict(hypernu=(0.0, np.nan, 0.0)), dict(hypernu=(0.0, 0.0, np.inf)),
+                                    dict(gE=np.inf), dict(gE=np.nan)])
+def test_gpu_constants_that_are_not_finite_fail_as_in_the_oracle(change):
+    """A layer at rest: a zero times infinity or NaN is NaN, and the step's check finds it."""
+    case = cases.make_case(nx=40, ny=24, sch=2, seed=3, jet="none", bumps=0, hyper=False)
+    for x in (case.eta, case.u, case.v):
+        x[:] = 0.0
+    p = case.params
+    p.CFL = 1e30
+    for k, v in change.items():
+        setattr(p, k, v)
+    s = lib.Solver(p)
+    s.upload(*case.fields(), mode=lib.UPLOAD_RAW)
+    o = orc.Oracle(p)
+    o.load(case.fields(), raw=True)
+    rc, _ = o.step(1)
+    assert s.step(1) == {1: lib.ERR_CFL, 2: lib.ERR_NONFINITE}[rc]
