@@ -1645,21 +1645,31 @@ struct PdlLaunch {
 };
 
 // Height of a single member's strips: cols strip columns (of all kinds) on
-// `slots` resident warps. A strip costs its rows and `lead` rows more (its first
-// rows and carried faces); the queue evens out the warps' speeds, which costs
-// about half a strip's time at the end when a warp takes several, and `one`
-// when each takes one (a quarter, or half with strips of two kinds). At 4096x2048: kb_lap1 18 rows (one strip a warp) 0.057
-// ms and 5 rows 0.050; kb_main2 27 and 7 rows 0.179 and 0.168; kb_main1 44, 22
-// and 11 rows 0.246, 0.212 and 0.200. At 1501x755, where strips are short, the
-// tracer's 5 rows (one strip a warp) 0.029 and 2 rows 0.036, kb_main1's 10 rows
-// 0.067 and 5 rows 0.058.
-inline int strip_height(int ny, int cols, int slots, double lead, double one) {
+// `slots` resident warps. A strip costs its rows and a lead of rows more (its
+// first rows and carried faces). One kind (lead 0.7): the queue evens out the
+// warps' speeds, which costs about half a strip's time at the end when a warp
+// takes several, a quarter when each takes one. At 4096x2048 kb_lap1 with 18 rows
+// (one strip a warp) 0.057 ms and with 5 rows 0.050; kb_main2 with 27 and 7 rows
+// 0.179 and 0.168. Several kinds (kb_main1, lead 1.2), whose strips differ in
+// length: nine tenths of a strip's time at the end, and half of what is missing
+// to whole rounds. Over 24 grids from 200x100 to 3000x1500, 16x60000 and 4096x2048,
+// plain and with winds and a tracer, the height so found is 0.4 % slower than the
+// best on average and 4 % at most (with the rule of one kind, lead 1.3 and one half,
+// 3.5 and 15 %): 1100x550 with winds and a tracer 2, 3 and 5 rows 0.055, 0.045
+// and 0.051 ms; plain 2048x1024 3, 4 and 5 rows 0.065, 0.063 and 0.067; 64x16384
+// 2, 4 and 5 rows 0.077, 0.072 and 0.075; 4096x2048 44, 22 and 9 rows 0.246, 0.212 and 0.197.
+inline int strip_height(int ny, int cols, int slots, bool several) {
   int best = 1;
   double least = 0;
   for (int sr = 1; sr <= 64; sr++) {
     const double rounds = (double)cols * ((ny + sr - 1) / sr) / slots;
-    const double time = rounds + (rounds <= 1.0 ? one : 0.5);
-    const double cost = (sr + lead) * (time > 1.0 ? time : 1.0);
+    double cost = 0;
+    if (several) {
+      cost = (sr + 1.2) * (0.5 * (rounds + std::ceil(rounds)) + 0.9);
+    } else {
+      const double time = rounds + (rounds <= 1.0 ? 0.25 : 0.5);
+      cost = (sr + 0.7) * (time > 1.0 ? time : 1.0);
+    }
     if (sr == 1 || cost < least) {
       least = cost;
       best = sr;
@@ -1678,7 +1688,7 @@ void run_phase(const char* tag, int smem, const PhaseArgs<N>& a, int& nl, int ki
   const int cap = grid_cap<K>(smem);
   int nstrips = a.nstrips, sr = a.sr;
   if constexpr (N == 1) {
-    sr = strip_height(a.ny, a.nbx * kinds, cap * NWARP, kinds > 1 ? 1.3 : 0.7, kinds > 1 ? 0.5 : 0.25);
+    sr = strip_height(a.ny, a.nbx * kinds, cap * NWARP, kinds > 1);
     nstrips = a.nbx * ((a.ny + sr - 1) / sr);
   }
   const int per = nstrips;
