@@ -632,8 +632,8 @@ struct Face {
   bool pos, act, both;
 };
 // PAIR: w is a sum of two velocities, to be halved. n1: q0 - qm when v.pos,
-// q2 - q1 otherwise; n2(): the other of the two. bad is set where the skipped
-// side might not be finite.
+// q2 - q1 otherwise; n2(): the other of the two. bad is set where a skipped
+// side might not be finite (both are skipped without a velocity).
 template <int SCH, bool PAIR, typename N2>
 __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, N2 n2, double q0, double q1,
                                           unsigned long long dt, bool& bad) {
@@ -646,7 +646,10 @@ __device__ __forceinline__ Face make_face(const Vel& v, double d, double n1, N2 
   F.act = v.act;
   F.both = v.both;
   F.hp = half_psi<SCH>(n1, d);
-  if (hi_mag(d) < HI_POW2(-397) && nz(d)) bad = bad || hi_mag(n2()) >= hi_mag(d) + (490u << 20);
+  if (hi_mag(d) < HI_POW2(-397) && nz(d)) {
+    bad = bad || hi_mag(n2()) >= hi_mag(d) + (490u << 20);
+    if constexpr (SCH == 5 || SCH == 6) bad = bad || (!v.act && hi_mag(n1) >= hi_mag(d) + (490u << 20));
+  }
   F.p = sig_mul(mag(v.w), dt, K);
   F.hp2 = 0.0;
   F.p2 = 0;

@@ -337,3 +337,27 @@ def test_gpu_constants_that_are_not_finite_fail_as_in_the_oracle(change):
     o.load(case.fields(), raw=True)
     rc, _ = o.step(1)
     assert s.step(1) == {1: lib.ERR_CFL, 2: lib.ERR_NONFINITE}[rc]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sch", [5, 6])
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("side", [1, -1])
+def test_gpu_skipped_sides_that_are_not_finite_match_oracle(sch, axis, side):
+    """No velocity anywhere, and a difference so small beside its neighbour that
+    the square of the limiter's ratio overflows: zero times NaN is NaN."""
+    case = cases.make_case(nx=64, ny=33, sch=sch, seed=3, jet="none", bumps=0, hyper=False)
+    for x in (case.eta, case.u, case.v):
+        x[:] = 0.0
+    t = np.zeros(12)
+    t[3], t[5] = 1.0, 1e-200  # ratios of 1/1e-200 on one side of the face between cells 4 and 5
+    if side < 0:
+        t = t[::-1]
+    if axis:
+        case.tracer[15, 20:32] = t
+    else:
+        case.tracer[10:22, 25] = t
+    case.tracer[5, 50] = 1.0
+    cases.halo_wrap(case.tracer)
+    s = same_steps(case, (1,), raw=True)
+    assert np.any(np.isnan(s.download()["tracer"]))
