@@ -146,7 +146,10 @@ void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, 
   }
   for (int j = -1; j <= ny + 2; j++)
     for (const auto& d : kSigDivisors) {
-      const uint64_t b = bits_of(R(d.row, j)), y = positive_in_window(b) ? sig_recip(b) : 0;
+      // of the row above ny the magnitude: the terms that the face north of row
+      // ny would have there are formed and dropped
+      const uint64_t b = bits_of(R(d.row, j)) & (j > ny ? ~(1ULL << 63) : ~0ULL);
+      const uint64_t y = positive_in_window(b) ? sig_recip(b) : 0;
       std::memcpy(&R(d.recip, j), &y, sizeof y);
     }
   // compute_Dt fallback for a flow at rest (calc.c:715-725): depends on geometry only

@@ -122,18 +122,18 @@ SIG_FN uint32_t sig_mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64
 // |a / b|, by long division in three digits of about 20 bits. y is the
 // reciprocal of b's leading 24 bits rounded up (at most 2^-23 above b in
 // [1, 2)), less three ulps of 2^-24. With the approximation within one ulp it
-// is below 1/b, by a factor of at most 1 - 9*2^-24. So every digit comes out low
-// and every remainder is positive: below 1154, 651 and 368 units of the digit's
-// place (e -> e*2^20*9*2^-24 + 2, from 2*2^30*9*2^-24 + 2), the first below 2^64. The
-// sum of the digits is at most 368 units of 2^-70 below the quotient; the rounding
-// test allows 520.
+// is below 1/b, by a factor of at most 1 - 9*2^-24, or, where it falls below 1/2 (f =
+// 2), whose ulps count double here, 1 - 11*2^-24. So every digit comes out low and
+// every remainder is positive: below 1410, 971 and 670 units of the digit's place
+// (e -> e*2^20*11*2^-24 + 2, from 2*2^30*11*2^-24 + 2), the first below 2^64. The
+// sum of the digits is at most 670 units of 2^-70 below the quotient; the rounding
+// test allows 700.
 SIG_FN uint64_t sig_div(uint64_t a, uint64_t b) {
   const uint64_t ma = sig_of(a), mb = sig_of(b);
   SigFloat f;
   f.u = (0x3f800000u | ((uint32_t)(mb >> 29) & 0x7fffffu)) + 1u;
   f.f = sig_rcp(f.f);
-  f.u = f.u > 0x3f000000u ? f.u : 0x3f000000u;  // 1/f >= 1/2, where the approximation may be an ulp less (f = 2)
-  const uint32_t y = (f.u << 8 | 0x80000000u) - 0x300u;  // units of 2^-32
+  const uint32_t y = (f.u << 8) + (0x80000000u - 0x300u);  // units of 2^-32; a sum: it carries on below 1/2
   const bool ge = ma >= mb;
   const uint64_t N = ge ? ma : ma + ma;
   const uint32_t q1 = sig_mulhi32((uint32_t)(N >> 22), y);  // units of 2^-30
@@ -142,7 +142,7 @@ SIG_FN uint64_t sig_div(uint64_t a, uint64_t b) {
   const uint64_t r2 = (r1 << 20) - (uint64_t)q2 * mb;
   const uint32_t q3 = sig_mulhi32((uint32_t)(r2 >> 32), y);  // units of 2^-70
   const uint64_t t = ((uint64_t)q1 << 23) + ((uint64_t)q2 << 3) + (q3 >> 17);
-  const uint64_t m = sig_round_quotient(t, (q3 & 0x1ffffu) >= 0x20000u - 520u, N, mb);
+  const uint64_t m = sig_round_quotient(t, (q3 & 0x1ffffu) >= 0x20000u - 700u, N, mb);
   return sig_pack(m, sig_exp(a) - sig_exp(b) + SIG_BIAS - (ge ? 0u : 1u << 20));
 }
 

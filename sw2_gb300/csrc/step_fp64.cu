@@ -434,8 +434,7 @@ __device__ __noinline__ double advv_cell_ool(const DevState& s, const F7& f, int
 // for a tracer that is zero. Otherwise the cell is recomputed literally.
 // The Van Leer limiter in its reference form (0/0 at r = -1) keeps the
 // literal kernels, and so do cases whose Dt or metric divisors lie outside
-// 2^-20 .. 2^60 (DevState::sig_ok). The face north of row ny serves no cell above:
-// its terms there are taken with row ny's metric.
+// 2^-20 .. 2^60 (DevState::sig_ok).
 constexpr int FW = 31;      // cells per strip along x (32 faces)
 constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the launch's queue
 // Resident blocks per SM the register allocation must allow: 7 blocks (28
@@ -762,10 +761,9 @@ __device__ __forceinline__ double sum_faces(const Side& w, const Side& so, const
   }
   const double S = ((w.t - te) + so.t) - n.t;
   slow = false;
-  if (!nz(S)) {
-    slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1);
-    return 0.0;  // -0 here where the terms are -0, +0, -0 and +0; the literal sum, from its +0 on, stays +0
-  }
+  // a -0 (terms -0, +0, -0 and +0): the literal sum starts at +0 and stays there
+  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) &&
+                     (dbits(S) < 0 || !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1));
   return S;
 }
 
@@ -876,7 +874,7 @@ __device__ __forceinline__ void mass_strip(const DevState& s, const F7& f, doubl
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, METRIC(DYN, j), bad);
-    const Side ns = side_of<false>(FY, METRIC(DYN, min(j + 1, ny)), bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);  // calc.c:100 in its order: +w -e +s -n
     slow = __any_sync(FULL, bad) || slow;
@@ -928,7 +926,7 @@ __device__ __forceinline__ void tracer_strip(const DevState& s, const F7& f, dou
     const Vel b = vel_one(vn);
     const Face FY = y_face<SCH, false>(b, dm, d0, d1, h2, h3, dt, bad);
     const Side tn = side_of<false>(FY, my, bad);
-    const Side ns = side_of<false>(FY, METRIC(DYN, min(j + 1, ny)), bad);
+    const Side ns = side_of<false>(FY, METRIC(DYN, j + 1), bad);
     bool slow;
     const double S = sum_faces<false>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, h2, slow);
     slow = __any_sync(FULL, bad) || slow;
@@ -985,7 +983,7 @@ __device__ __forceinline__ void adv_u_strip(const DevState& s, const F7& f, doub
     const Vel v = vel_pair(va, vb, vn);
     const Face FY = y_face<SCH, true>(v, dm, d0, d1, u2, u3, dt, bad);
     const Side tn = side_of<true>(FY, my, bad);
-    const Side ns = side_of<true>(FY, METRIC(DYV, min(j + 1, ny)), bad);
+    const Side ns = side_of<true>(FY, METRIC(DYV, j + 1), bad);
     bool slow;
     const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, u2, slow);
     slow = __any_sync(FULL, bad) || slow;
