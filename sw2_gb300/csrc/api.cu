@@ -627,6 +627,7 @@ sw2g_status sw2g_create(const sw2g_case* c, int precision, int device, sw2g_ctx*
   s.sig_ok = ranges.divisors;
   s.lap_ok = ranges.laplacian;
   s.nu_ok = ranges.nu;
+  s.finite = ranges.finite;
   s.lape_eta = (c->flags & SW2G_FLAG_LAPE_ETA) ? 1 : 0;
   s.nu2dt = s.nu2 * s.Dt;
   s.nu4dt = s.nu4 * s.Dt;

@@ -75,12 +75,17 @@ SigRanges sig_ranges(const sw2g_case& c, const std::vector<double>& rows) {
   const int H = c.ny + 4;
   auto R = [&](int t, int j) { return rows[(size_t)t * H + (j + 1)]; };
   auto mid = [](double x) { return std::fabs(x) >= 0x1p-130 && std::fabs(x) < 0x1p250; };
-  SigRanges r{positive_in_window(bits_of(c.Dt)), true, true};
+  SigRanges r{positive_in_window(bits_of(c.Dt)), true, true, true};
   for (const auto& d : kSigDivisors)
     for (int j = 1; j <= c.ny + d.last; j++) r.divisors = r.divisors && positive_in_window(bits_of(R(d.row, j)));
   for (const auto& f : kLapFactors)
     for (int j = f.first; j <= c.ny + f.last; j++) r.laplacian = r.laplacian && mid(R(f.row, j));
-  for (double nu : c.hypernu) r.nu = r.nu && (nu == 0 || mid(nu * c.Dt));
+  for (double nu : c.hypernu) {
+    r.nu = r.nu && (nu == 0 || mid(nu * c.Dt));
+    r.finite = r.finite && std::isfinite(nu * c.Dt);
+  }
+  for (int t : {R_MGEDT, R_MGNDT, R_DXC, R_DYC})
+    for (int j = 1; j <= c.ny; j++) r.finite = r.finite && std::isfinite(R(t, j));
   return r;
 }
 

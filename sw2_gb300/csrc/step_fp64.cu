@@ -514,7 +514,9 @@ __device__ __forceinline__ Metric metric(const DevState& s, int t, int ty, int j
 
 // Products and quotients of any operands, on the integer pipe when the
 // operands are of magnitude 2^-255 .. 2^257 (the result is then normal), on
-// the FP64 unit, out of line, otherwise. A zero times a finite factor is a zero.
+// the FP64 unit, out of line, otherwise. A zero times a factor is a zero: the
+// factors are finite (DevState::finite; without it k_hyper_add and k_pres_sum
+// take plain FP64 in every step: asking here costs flows from rest 1.5 %).
 __device__ __forceinline__ bool mid(double x) { return ((hi_word(x) - 0x30000000u) & 0x60000000u) == 0; }
 // 2^-700 (2^-850) <= |x| < 2^257: times a factor of 2^-255 (2^-130) or more
 // still normal, and over a metric factor
@@ -530,20 +532,20 @@ __device__ __forceinline__ double smul(double a, double b) {
 __device__ __forceinline__ double rmul(bool ok, double k, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(k)) & kSign;
   if (wider(a) && ok) return from_bits(sig_mul(mag(a), mag(k)) | sg);
-  if (!nz(a) && ok) return from_bits(sg);
+  if (!nz(a)) return from_bits(sg);
   return mul_fp64(k, a);
 }
 __device__ __forceinline__ double cmul(double c, double a) {
   const unsigned long long sg = (unsigned long long)(dbits(a) ^ dbits(c)) & kSign;
   if (wide(a) && mid(c)) return from_bits(sig_mul(mag(a), mag(c)) | sg);
-  if (!nz(a) && hi_mag(c) < SIG_EXP) return from_bits(sg);
+  if (!nz(a)) return from_bits(sg);
   return mul_fp64(c, a);
 }
 __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
-// a / x.b: with x.b > 0, as s.sig_ok says, a zero gives itself.
+// a / x.b (x.b > 0): a zero gives itself.
 __device__ __forceinline__ double mdiv(const DevState& s, double a, const Metric& x) {
   if (wider(a) && s.sig_ok) return from_bits(sig_div_known(mag(a), x.b, x.y) | sign_of(a));
-  if (!nz(a) && s.sig_ok) return a;
+  if (!nz(a)) return a;
   return div_fp64(a, from_bits(x.b));
 }
 
@@ -761,9 +763,10 @@ __device__ __forceinline__ double sum_faces(const Side& w, const Side& so, const
   }
   const double S = ((w.t - te) + so.t) - n.t;
   slow = false;
-  // a -0 (terms -0, +0, -0 and +0): the literal sum starts at +0 and stays there
-  if (!nz(S)) slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) &&
-                     (dbits(S) < 0 || !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1));
+  if (!nz(S)) {
+    slow = !nz(w.t) && !nz(te) && !nz(so.t) && !nz(n.t) && !first_term_plus_zero(act, w.pos, w.t, qm, q0, q1);
+    return 0.0;  // -0 where the terms are -0, +0, -0 and +0; the literal sum starts at +0 and stays there
+  }
   return S;
 }
 
@@ -1368,6 +1371,10 @@ __global__ void k_hyper_add(DevState s, double* d, const double* l2, const doubl
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
+  if (!s.finite) {
+    d[q] = d[q] + s.nu2dt * l2[q] + s.nu4dt * l4[q] + s.nu6dt * l6[q];
+    return;
+  }
   d[q] = hyper_terms<NZ>(s, d[q], l2[q], l4[q], l6[q]);
 }
 
@@ -1428,6 +1435,15 @@ __global__ void k_pres_sum(DevState s, F7 f, const double* duadv, const double* 
   SW2G_PDL_ENTRY();
   INTERIOR_IJ
   const int q = IX(W, i, j);
+  if (!s.finite) {
+    const double mge = s.polar ? -PF(s, P_GE, q) * s.Dt : RW(s, R_MGEDT, j);
+    const double mgn = s.polar ? -PF(s, P_GN, q) * s.Dt : RW(s, R_MGNDT, j);
+    dun[q] = duadv[q] + mge * (f.eta[IX(W, i + 1, j)] - f.eta[q]) / RW(s, R_DXC, j);
+    dvn[q] = dvadv[q] + mgn * (f.eta[IX(W, i, j + 1)] - f.eta[q]) / RW(s, R_DYC, j + 1);
+    dun[q] -= f.u[q] * (s.polar ? PF(s, P_SU, q) : s.sigma) * s.Dt;
+    dvn[q] -= f.v[q] * (s.polar ? PF(s, P_SV, q) : s.sigma) * s.Dt;
+    return;
+  }
   dun[q] = u_tendency<UD>(s, f.eta, duadv[q], f.u[q], i, j);
   dvn[q] = v_tendency<UD>(s, f.eta, dvadv[q], f.v[q], i, j);
 }
@@ -2187,6 +2203,10 @@ namespace {
     nl++;                                         \
   } while (0)
 
+// Whether the tails of the tendencies run as one kernel each: from the third
+// step (AB3), unless a constant is not finite (which fails the first step).
+bool tails_fused(const DevState& s, int k) { return k >= 2 && s.finite; }
+
 // Head of a step: core.c:134-290, through the velocity halos.
 // fused_checks: the range checks are done by the kernels that write the new
 // values (a whole step, from the third step).
@@ -2198,6 +2218,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
               cudaStream_t st, Timers* tm, bool fused_checks, bool whole, StepHooks hk) {
   int* const fbad = fused_checks ? chk.bad + slot : nullptr;
   const dim3 g((s.nx + TX - 1) / TX, s.ny);
+  const bool fused = tails_fused(s, k);
   int nl = 0;
   auto F = [&]() { return F7{b.f[0], b.f[1], b.f[2], b.f[3], b.f[4], b.f[5], b.f[6]}; };
   const bool hyper = (s.nu2 != 0 || s.nu4 != 0 || s.nu6 != 0);
@@ -2224,7 +2245,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   const bool laplacians_first = hyper && !s.lape_eta && hk.v_in;
   // From the third step the eta kernel computes the last level itself, except
   // where that level's source is eta, which the kernel changes.
-  const bool last_in_eta = hyper && k >= 2 && !laplacians_first && !(s.lape_eta && nlap == 1);
+  const bool last_in_eta = hyper && fused && !laplacians_first && !(s.lape_eta && nlap == 1);
   if (laplacians_first) eta_laplacians(0, nlap);
   if (hk.v_in) cudaStreamWaitEvent(st, hk.v_in, 0);
 
@@ -2258,7 +2279,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   }
 
   if (tracer) {
-    if (k >= 2) {
+    if (fused) {
       LAUNCH("tracer_ab3", pdl_launch(k_tracer_ab3, g, dim3(TX), st, s, b.f[3], b.dtr[0], b.dtr[1], b.dtr[2], fbad));
       rotate3(b.dtr);
     } else {
@@ -2270,9 +2291,9 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   }
   if (hyper) {
     if (!laplacians_first) eta_laplacians(1, nle);
-    if (k < 2) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
+    if (!fused) LAUNCH("hyper_add", hyper_add(s, g, st, b.deta[0], b.Le[0], b.Le[1], b.Le[2]));
   }
-  if (k >= 2) {
+  if (fused) {
     // writes eta's halo images too
     LAUNCH("eta_ab3", fused_tail(s, g, st, F(), b, 0, fbad, last_in_eta ? lap_eta_source(nlap - 1) : nullptr));
     rotate3(b.deta);
@@ -2286,7 +2307,7 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
   if (hk.eta_out) cudaEventRecord(hk.eta_out, st);  // eta is final for this step
 
   // momentum (core.c:212-280), from the third step in the Coriolis kernels
-  if (k < 2) {
+  if (!fused) {
     auto pres_sum = s.polar == 0 && s.sigma == 0.0 ? k_pres_sum<true> : k_pres_sum<false>;
     LAUNCH("pres_sum", pdl_launch(pres_sum, dim3(g), dim3(TX), st, s, F(), b.duadv, b.dvadv, b.du[0], b.dv[0]));
   }
@@ -2298,12 +2319,12 @@ int step_head(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, St
     for (int q = 1; q < nlap; q++)
       LAUNCH("lapv", pdl_launch(k_lapv, m.grid, dim3(TX), st, s, b.L[2 * q - 2], b.L[2 * q - 1], b.L[2 * q],
                                 b.L[2 * q + 1], m.rows, q + 1 < nlap));
-    if (k < 2) {
+    if (!fused) {
       LAUNCH("hyper_add", hyper_add(s, g, st, b.du[0], b.L[0], b.L[2], b.L[4]));
       LAUNCH("hyper_add", hyper_add(s, g, st, b.dv[0], b.L[1], b.L[3], b.L[5]));
     }
   }
-  if (k >= 2) {
+  if (fused) {
     // AB3 of u and v folded into the Coriolis updates (core.c:271-285); the v
     // tendency does not depend on the new u
     LAUNCH("coriolis_u", fused_tail(s, g, st, F(), b, 1, fbad));
@@ -2357,7 +2378,7 @@ int step_tail(const DevState& s, Fp64Buffers& b, bool tracer, StepChecks chk, in
 int fp64_step(const DevState& s, Fp64Buffers& b, int sch, int k, bool tracer, StepChecks chk, int slot,
               cudaStream_t st, Timers* tm, int parts, StepHooks hk) {
   int nl = 0;
-  const bool fused_checks = (parts == STEP_FULL) && k >= 2;
+  const bool fused_checks = (parts == STEP_FULL) && tails_fused(s, k);
   const bool whole = (parts == STEP_FULL) && s.polar == 0;  // halos and do_channel in one launch
   if (parts & STEP_HEAD) nl += step_head(s, b, sch, k, tracer, chk, slot, st, tm, fused_checks, whole, hk);
   if (parts & STEP_TAIL) nl += step_tail(s, b, tracer, chk, slot, st, tm, fused_checks, whole);

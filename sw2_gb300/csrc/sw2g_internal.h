@@ -55,7 +55,8 @@ struct DevState {
   int plain;           // windx, windy and hB are +0.0 in every padded cell
   int lape_eta;        // laplacian_eta of eta instead of u (SW2G_FLAG_LAPE_ETA)
   int sig_ok;          // Dt and the metric divisors lie in the range of the integer-pipe quotients,
-  int lap_ok, nu_ok;   // the Laplacians' factors and the nu*Dt in that of its products (SigRanges)
+  int lap_ok, nu_ok;   // the Laplacians' factors and the nu*Dt in that of its products,
+  int finite;          // and gravity, the divisors and the nu*Dt are finite (SigRanges)
   int fk;              // rows per strip of the fast TVD bodies (set per launch)
   unsigned* strips;    // the fast bodies' strip queue: next strip, warps done (zero between launches)
   int polar;           // 0: band; +-1: polar cap, with the fields below
@@ -74,9 +75,10 @@ bool grid_ok(const sw2g_case* c);
 void build_rows(const sw2g_case& c, std::vector<double>& rows, double* rest_mx, double* rest_my);
 // Which constants lie in the ranges of the integer-pipe operations: Dt and the
 // metric divisors in 2^-20 .. 2^60 (and positive), the factors of the Laplacians
-// and each nonzero nu*Dt in 2^-130 .. 2^250.
+// and each nonzero nu*Dt in 2^-130 .. 2^250; and whether gravity, the metric
+// divisors and nu*Dt are finite.
 struct SigRanges {
-  bool divisors, laplacian, nu;
+  bool divisors, laplacian, nu, finite;
 };
 SigRanges sig_ranges(const sw2g_case& c, const std::vector<double>& rows);
 // The fields of a polar cap (P_NUM x (nx+4)(ny+4)) and the at-rest CFL maxima
