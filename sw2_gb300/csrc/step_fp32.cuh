@@ -768,9 +768,11 @@ __device__ __forceinline__ bool strip_lap(const MemberDesc& d, const View& vw, i
 // launch, which its warps take from the queue, the longer momentum strips
 // first. In one strip their windows, carried faces and rings took 168
 // registers and 19 KB of shared memory a warp, which left 12 warps per SM;
-// apart they take 96 registers and 11 KB, and 20 are resident, for u and v read
-// twice: 0.229 -> 0.199 ms at 4096x2048 (bound by instruction latency: issue on
-// two thirds of the cycles before).
+// apart the plain form's take 96 registers (spilling 28 to 180 bytes a thread) and
+// 11 KB, and 20 are resident, for u and v read twice: 0.229 -> 0.199 ms at
+// 4096x2048 (bound by instruction latency: issue on two thirds of the cycles
+// before). The EXTRA form's, which stage the winds and the bottom too, take 160 to
+// 168 registers and 18 KB: 12 warps per SM.
 //
 // Mass: rows j0-2 .. j1+2 (ring row t <-> j0-2+t) of the eta shadow, with
 // EXTRA of the bottom height (H = eta + depth - hB, sw.h:213); and rows j0-1 ..

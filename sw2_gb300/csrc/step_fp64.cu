@@ -177,7 +177,8 @@ __device__ __forceinline__ double sadd(double a, double b) {
   return __longlong_as_double((long long)((A & ~MAG) | ((unsigned long long)e << 52) | (r & FRAC)));
 }
 // a - b = a + (-b), exactly and for every operand (a NaN operand gives a
-// NaN either way; NaN bit patterns are not compared anywhere).
+// NaN either way; NaN bit patterns are not compared anywhere). The step's kernels
+// add only; the self-check takes the adder's other signs through it.
 __device__ __forceinline__ double ssub(double a, double b) {
   return sadd(a, __longlong_as_double(dbits(b) ^ (long long)0x8000000000000000ULL));
 }
@@ -442,7 +443,10 @@ constexpr int FWARPS = 4;   // warps per block; each warp takes strips from the 
 // 2048x1024 with 4, 5, 6, 7, 8 and 10 blocks: 0.138, 0.133, 0.128, 0.122,
 // 0.124 and 0.125 ms. In one launch with the other kinds, whole steps with 6, 7
 // and 8: four at 2048x1024 3.229, 3.212, 3.197 ms; four of a 500x500 cap 0.763,
-// 0.759, 0.771; two forced ones from rest at 1024x512 2.147, 2.000, 2.051.
+// 0.759, 0.771; two forced ones from rest at 1024x512 2.147, 2.000, 2.051. At 72
+// registers the launch's frame, which seven kinds of strips share, spills 120 to 124
+// bytes a thread for limiter 2, 152 to 236 for the others (limiter 8); k_lapv alone
+// takes 56 registers and spills none.
 #define FAST_MIN_BLOCKS 7
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -459,16 +463,13 @@ __device__ __forceinline__ bool nz(double x) { return (dbits(x) & 0x7fffffffffff
 __device__ __forceinline__ double mn(double a, double b) { return key(a) < key(b) ? a : b; }  // sw.h MIN
 __device__ __forceinline__ double mx(double a, double b) { return key(a) > key(b) ? a : b; }  // sw.h MAX
 
-// The limiters of calc.c:54-63 with the comparisons above.
+// The limiters of calc.c:54-63 that compare, with the comparisons above, but
+// for those whose formula half_psi writes out (2, 4, 5, 6 and the safe Van Leer).
 template <int SCH>
 __device__ __forceinline__ double limiter_fast(double r) {
   if constexpr (SCH == 0) return mx(0.0, mn(mn(HALF(1 + r), TWICE(r)), 2.0));
   else if constexpr (SCH == 1) return mx(mx(0.0, mn(TWICE(r), 1.0)), mx(0.0, mn(r, 2.0)));
-  else if constexpr (SCH == 2) return mn(r, 1.0);
-  else if constexpr (SCH == 4) { const double r2 = TWICE(r); return mx(0.0, mn(r2, mn((1 + r2) / 3.0, 2.0))); }
   else if constexpr (SCH == 7) return mx(0.0, mn(mn(2.0, TWICE(r)), mn(0.25 + 0.75 * r, 0.75 + QUARTER(r))));
-  else if constexpr (SCH == kVanLeerSafe)
-    return (dbits(r) == dbits(-1.0)) ? 0.0 : (r + fabs(r)) / (1.0 + r);
   else return limiter<SCH>(r);
 }
 
@@ -991,7 +992,7 @@ __device__ __forceinline__ void adv_u_strip(const DevState& s, const F7& f, doub
     const double S = sum_faces<true>(tw, ts, tn, lane, FX.act, xn.m2, xn.m1, u2, slow);
     slow = __any_sync(FULL, bad) || slow;
     // calc.c:198: u0*(uep-uwm)/(2 DXE) + u0*((vn0+vn1)/2 - (vs0+vs1)/2)/DYV; the
-    // halving commutes with the difference (its operands are zero or at least 2^-352)
+    // halving commutes with the difference (its operands are zero or at least 2^-902)
     const double ux = xn.p1 - xn.m1, vy = vn - vs;
     const double p2 = Dt * two_products(u2, ux, 0, METRIC(DXE2, j), vy, 0xfff00000u, my);
     if (own) {
@@ -2008,7 +2009,7 @@ __global__ void k_range(DevState s, RangeFields r, int* bad) {
 // out the warps' different speeds, and the end of the launch, with part of the
 // warps idle, costs about a strip's time (more in flows from rest, where the
 // cells that need the literal code lie together). So the height is the one
-// with the least (fk + 1) * max(1, strips per resident warp + 1.2). With 0.3,
+// with the least (fk + 1) * (strips per resident warp + 1.2). With 0.3,
 // 1.0 and 1.6 in place of 1.2: two forced steps from rest at 1024x512 2.41,
 // 2.03 and 1.93 ms; four steps of a 500x500 cap 0.830, 0.795 and 0.794; four
 // steps at 2048x1024 3.286, 3.290 and 3.318. One launch for the bodies in place
@@ -2019,8 +2020,7 @@ int choose_strip_rows(int columns, int ny, long long warps) {
   double least = 0;
   for (int fk = 1; fk <= 24; fk++) {
     const long long strips = (long long)columns * ((ny + fk - 1) / fk);
-    const double rounds = (double)strips / (double)warps + 1.2;
-    const double cost = (fk + 1) * (rounds > 1.0 ? rounds : 1.0);
+    const double cost = (fk + 1) * ((double)strips / (double)warps + 1.2);
     if (fk == 1 || cost < least) {
       least = cost;
       best = fk;
@@ -2064,7 +2064,7 @@ void launch_strips(cudaStream_t st, const DevState& s0, const F7& f, const Bodie
 template <int SCH>
 int launch_bodies(dim3 g, cudaStream_t st, const DevState& s, const F7& f, const Bodies& o) {
   if constexpr (SCH != 3) {
-    if (s.sig_ok) {  // Dt and the metric factors in the range of the integer-pipe quotients
+    if (s.sig_ok) {  // Dt and the metric divisors in the range of the integer-pipe quotients
       if (!s.plain) launch_strips<k_bodies<SCH, false, false>>(st, s, f, o);
       else if (!s.polar && s.sigma == 0.0) launch_strips<k_bodies<SCH, true, true>>(st, s, f, o);
       else launch_strips<k_bodies<SCH, true, false>>(st, s, f, o);
